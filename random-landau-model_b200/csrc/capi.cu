@@ -293,14 +293,24 @@ int rlmb_rlm_assemble(rlmb_context* ctx, const double* d_vmn, const double* d_co
             return RLMB_ERR_ARG;
     if (count == 0) return RLMB_OK;
     RLMB_CUDA_TRY(cudaSetDevice(ctx->device));
-    if (int rc = ensure_workspace(ctx, 2 * (size_t)count * sizeof(int))) return rc;
-    int* d_t = static_cast<int*>(ctx->ws);
+    std::vector<int> uniq(h_theta2, h_theta2 + count);   // the distinct theta_2, ascending
+    std::sort(uniq.begin(), uniq.end());
+    uniq.erase(std::unique(uniq.begin(), uniq.end()), uniq.end());
+    size_t bytes = 0;
+    need<int>(bytes, 2 * (size_t)count);
+    const size_t s_elems = rlm_assemble_ws_elems(n_phi, dim, 1, (int)uniq.size());
+    need<cplx>(bytes, s_elems);
+    if (int rc = ensure_workspace(ctx, bytes)) return rc;
+    Carver cv(ctx->ws);
+    int* d_t = cv.take<int>(2 * (size_t)count);
+    cplx* d_s = cv.take<cplx>(s_elems);
     RLMB_CUDA_TRY(cudaMemcpyAsync(d_t, h_theta1, count * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     RLMB_CUDA_TRY(cudaMemcpyAsync(d_t + count, h_theta2, count * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     return launch_rlm_assemble(ctx, reinterpret_cast<const cplx*>(d_vmn),
                                reinterpret_cast<const cplx*>(d_coeff_m_theta),
                                reinterpret_cast<const cplx*>(d_coeff_jm), d_t, d_t + count, count,
-                               count, n_phi, dim, off_head, reinterpret_cast<cplx*>(d_h));
+                               count, n_phi, dim, off_head, uniq.data(), (int)uniq.size(), d_s,
+                               reinterpret_cast<cplx*>(d_h));
 }
 
 int rlmb_hlm_basis(rlmb_context* ctx, int lx, int ly, int Q, int band, int n_mesh, int theta_1,
@@ -498,7 +508,10 @@ static int rlm_prepare(rlmb_context* ctx, int n_phi, double qc, double ic, int n
     p->d_out = cv.take<double>(2 * (size_t)n_phi * nb);
     p->d_info = cv.take<int>((size_t)kpts * nb);
     if (int rc = ensure_pinned(ctx, 2 * (size_t)kpts * nb * sizeof(int))) return rc;
-    if (int rc = ensure_workspace(ctx, rlm_potential_ws_elems(nimp, nb, dim) * sizeof(cplx))) return rc;
+    // (the V_mn partial sums and the assembly's theta_2 slabs, in turn)
+    if (int rc = ensure_workspace(ctx, std::max(rlm_potential_ws_elems(nimp, nb, dim),
+                                                rlm_assemble_ws_elems(n_phi, dim, nb, g + 1)) * sizeof(cplx)))
+        return rc;
     RLMB_CUDA_TRY(cudaMemcpyAsync(p->d_cmn, cmn.data(), cmn.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     RLMB_CUDA_TRY(cudaMemcpyAsync(p->d_cmt, cmt.data(), cmt.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     RLMB_CUDA_TRY(cudaMemcpyAsync(p->d_cjm, cjm.data(), cjm.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
@@ -523,6 +536,8 @@ static int rlm_prepare(rlmb_context* ctx, int n_phi, double qc, double ic, int n
 static int rlm_enqueue(rlmb_context* ctx, const RlmPlan& p, int sample0, const int* d_sample0, double* energies,
                        double* chern, bool dev_out, const char* wfs_dir) {
     const int n_phi = p.n_phi, nimp = p.nimp, nb = p.nb, kpts = p.kpts, g = p.g, dim = p.dim, o = p.o;
+    std::vector<int> all_t2(g + 1);
+    for (int t = 0; t <= g; ++t) all_t2[t] = t;
     for (int s0 = 0; s0 < p.n_samples; s0 += nb) {
         const int cnt = std::min(nb, p.n_samples - s0);
         double* dx = p.d_imp;
@@ -539,7 +554,7 @@ static int rlm_enqueue(rlmb_context* ctx, const RlmPlan& p, int sample0, const i
                                           p.d_vmn))
             return rc;
         if (int rc = launch_rlm_assemble(ctx, p.d_vmn, p.d_cmt, p.d_cjm, p.d_t, p.d_t + (size_t)nb * kpts, cnt * kpts,
-                                         kpts, n_phi, dim, o, p.d_H))
+                                         kpts, n_phi, dim, o, all_t2.data(), g + 1, static_cast<cplx*>(ctx->ws), p.d_H))
             return rc;
         if (int rc = heevd_batched_band(ctx, reinterpret_cast<double*>(p.d_H), p.d_W, n_phi, cnt * kpts, p.d_info, o))
             return rc;

@@ -1,7 +1,9 @@
 // Assembly and Chern-step kernels of the rlm and hlm twist-mesh pipelines (sm_100a, FP64).
 #include "model_kernels.cuh"
 #include "small_eig.cuh"
+#include "zgemm.cuh"
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 
@@ -100,59 +102,123 @@ size_t rlm_potential_ws_elems(int nimp, int nsamples, int dim) {
 //   F[j][k] = sum_m conj(c_t2[m]) c_jm[j][m] * sum_{n in {o+k-j, o+k-j-N}} V[m][n] c_t1[n]
 // stored row-major as the reference does: buf[j*N+k] = F[j][k] (k > j), conj(F[j][j]) on
 // the diagonal, buf[k*N+j] = conj(F[j][k]); zero outside the cyclic band.
-__device__ __forceinline__ cplx rlm_entry(const cplx* __restrict__ V, const cplx* __restrict__ c1,
-                                          const cplx* __restrict__ c2, const cplx* __restrict__ cj,
-                                          int n_phi, int dim, int o, int j, int delta) {
-    const bool ta = delta <= o, tb = n_phi - delta <= o;
-    const int na = o + delta, nb = o + delta - n_phi;
-    cplx f = mk(0, 0);
-    const cplx g1a = ta ? c1[na] : mk(0, 0);
-    const cplx g1b = tb ? c1[nb] : mk(0, 0);
-    for (int m = 0; m < dim; ++m) {
-        cplx t = mk(0, 0);
-        if (ta) cfma(t, V[m * dim + na], g1a);
-        if (tb) cfma(t, V[m * dim + nb], g1b);
-        const cplx p = cmulc(c2[m], cj[j * dim + m]);   // conj(c_t2[m]) * c_jm[j][m]
-        cfma(f, t, p);
-    }
-    return f;
-}
+//
+// The sum over m does not see theta_1: with
+//   S_t2[j][n] = sum_m conj(c_t2[m]) c_jm[j][m] V[m][n]
+// every entry is F[j][k] = sum_{n} S_t2[j][n] c_t1[n] (one or two terms).  S is one complex
+// N x dim by dim x dim product per theta_2 (the FP64 tensor-path GEMM engine), shared by all
+// theta_1, and the fill is bound by writing H.  Evaluating the m sum per entry and k-point
+// took 8.9 ms at n_phi = 512, g = 16, 2 samples (2.4 GB of H); this form takes 0.50 ms (4.8 TB/s of H).
+struct ThetaList {   // theta_2 indices of one group, ascending
+    static constexpr int MAX = 64;
+    int n;
+    int t2[MAX];
+};
 
+// A(j, m) = conj(c_t2[m]) c_jm[j][m], batch z = sample * list.n + slot
+struct OpThetaA {
+    static constexpr bool RFAST = false;
+    const cplx* cmt;
+    const cplx* cjm;
+    int dim;
+    ThetaList list;
+    __device__ __forceinline__ cplx elem(size_t z, int j, int m) const {
+        const int t2 = list.t2[z % list.n];
+        return cmulc(cmt[(size_t)t2 * dim + m], cjm[(size_t)j * dim + m]);
+    }
+};
+// B(m, n) = V[m][n] of the batch's sample
+struct OpVmnB {
+    static constexpr bool KFAST = false;
+    const cplx* vmn;
+    int dim, per;
+    __device__ __forceinline__ cplx elem(size_t z, int m, int n) const {
+        return vmn[((size_t)(z / per) * dim + m) * dim + n];
+    }
+};
+// S[z][j][n], n contiguous
+struct EpRowMajor {
+    cplx* s;
+    int rows, cols;
+    __device__ __forceinline__ bool skip(int, int, int) const { return false; }
+    __device__ __forceinline__ void store(size_t z, int j, int n, cplx acc) const {
+        s[(z * rows + j) * cols + n] = acc;
+    }
+};
+
+// One warp per row j of a k-point's buffer, lanes along k.  kp0: first k-point of the launch;
+// a k-point whose theta_2 is not in the list belongs to another launch.
 __global__ void __launch_bounds__(256)
-k_rlm_assemble(const cplx* __restrict__ vmn, const cplx* __restrict__ cmt, const cplx* __restrict__ cjm,
-               const int* __restrict__ t1s, const int* __restrict__ t2s, int n_phi, int dim, int o,
-               int samples_stride_kpts, cplx* __restrict__ H) {
-    const int kp = blockIdx.y;
-    const int sample = kp / samples_stride_kpts;
-    const cplx* V = vmn + (size_t)sample * dim * dim;
+k_rlm_assemble(const cplx* __restrict__ S, const cplx* __restrict__ cmt, const int* __restrict__ t1s,
+               const int* __restrict__ t2s, const __grid_constant__ ThetaList list, int n_phi, int dim, int o,
+               int kpts_per_sample, int kp0, cplx* __restrict__ H) {
+    const int kp = kp0 + blockIdx.y;
+    const int t2 = t2s[kp];
+    int lo = 0, hi = list.n - 1;   // the slot of t2
+    while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        if (list.t2[mid] < t2) lo = mid + 1;
+        else hi = mid;
+    }
+    if (list.t2[lo] != t2) return;
+    const int j = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (j >= n_phi) return;
+    const int sample = blockIdx.y / kpts_per_sample;
+    const cplx* s = S + ((size_t)sample * list.n + lo) * n_phi * dim;
     const cplx* c1 = cmt + (size_t)t1s[kp] * dim;
-    const cplx* c2 = cmt + (size_t)t2s[kp] * dim;
-    cplx* h = H + (size_t)kp * n_phi * n_phi;
-    const size_t nn = (size_t)n_phi * n_phi;
-    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < nn;
-         idx += (size_t)gridDim.x * blockDim.x) {
-        const int j = (int)(idx / n_phi), k = (int)(idx % n_phi);   // buf[j*N + k]
-        const int lo = min(j, k), hi = max(j, k);
-        const int delta = hi - lo;
-        cplx val = mk(0, 0);
-        if (delta <= o || n_phi - delta <= o) {
-            const cplx f = rlm_entry(V, c1, c2, cjm, n_phi, dim, o, lo, delta);
-            val = (k > j) ? f : cconj(f);
-        }
-        h[idx] = val;
+    cplx* h = H + ((size_t)kp * n_phi + j) * n_phi;
+    for (int k = threadIdx.x & 31; k < n_phi; k += 32) {
+        const int row = min(j, k), delta = max(j, k) - row;
+        const cplx* sr = s + (size_t)row * dim;
+        cplx f = mk(0, 0);
+        if (delta <= o) cfma(f, sr[o + delta], c1[o + delta]);
+        if (n_phi - delta <= o) cfma(f, sr[o + delta - n_phi], c1[o + delta - n_phi]);
+        h[k] = k > j ? f : cconj(f);
     }
 }
 
+// theta_2 slabs of S held at once: at most 64 per sample and 256 MB in all, at least one.
+static size_t rlm_slab_cap(int n_phi, int dim) {
+    const size_t slab = (size_t)n_phi * dim * sizeof(cplx);
+    return std::max<size_t>(1, ((size_t)256 << 20) / slab);
+}
+size_t rlm_assemble_ws_elems(int n_phi, int dim, int nsamples, int n_t2) {
+    const size_t want = (size_t)nsamples * std::min(n_t2, (int)ThetaList::MAX);
+    return std::min(want, rlm_slab_cap(n_phi, dim)) * n_phi * dim;
+}
+
+// k-points kp = 0 .. count-1 (kpts_per_sample consecutive ones per sample, angles d_t1 / d_t2);
+// uniq_t2: the n_t2 distinct theta_2 indices among them, ascending (host); ws:
+// rlm_assemble_ws_elems(n_phi, dim, samples, n_t2) elements.
 int launch_rlm_assemble(rlmb_context* ctx, const cplx* vmn, const cplx* cmt, const cplx* cjm,
                         const int* d_t1, const int* d_t2, int count, int kpts_per_sample,
-                        int n_phi, int dim, int o, cplx* H) {
-    const size_t nn = (size_t)n_phi * n_phi;
-    const int bx = (int)std::min<size_t>((nn + 255) / 256, 1024);
-    dim3 g(bx, count);
-    prof_begin(ctx, "k_rlm_assemble");
-    k_rlm_assemble<<<g, 256, 0, ctx->stream>>>(vmn, cmt, cjm, d_t1, d_t2, n_phi, dim, o,
-                                               kpts_per_sample, H);
-    RLMB_LAUNCHED(ctx);
+                        int n_phi, int dim, int o, const int* uniq_t2, int n_t2, cplx* ws, cplx* H) {
+    const int nsamples = (count + kpts_per_sample - 1) / kpts_per_sample;
+    const size_t cap = rlm_slab_cap(n_phi, dim);
+    const int group = (int)std::min<size_t>(std::min(n_t2, (int)ThetaList::MAX), cap);
+    // samples per launch: their slabs within the cap, both grids within 65535 in y / z
+    const int per = (int)std::max<size_t>(1, std::min<size_t>({(size_t)nsamples, cap / group, (size_t)65535 / group,
+                                                               (size_t)65535 / kpts_per_sample}));
+    for (int s0 = 0; s0 < nsamples; s0 += per) {
+        const int ns = std::min(per, nsamples - s0);
+        const int kp0 = s0 * kpts_per_sample, kps = std::min(ns * kpts_per_sample, count - kp0);
+        for (int u = 0; u < n_t2; u += group) {
+            ThetaList list;
+            list.n = std::min(group, n_t2 - u);
+            for (int i = 0; i < ThetaList::MAX; ++i) list.t2[i] = i < list.n ? uniq_t2[u + i] : 0;
+            prof_begin(ctx, "k_rlm_assemble");
+            RLMB_CUDA_TRY((launch_zgemm<cplx, 64>(ctx->stream, OpThetaA{cmt, cjm, dim, list},
+                                                  OpVmnB{vmn + (size_t)s0 * dim * dim, dim, list.n},
+                                                  EpRowMajor{ws, n_phi, dim}, n_phi, dim, dim, ns * list.n)));
+            RLMB_LAUNCHED(ctx);
+            for (int q = 0; q < kps; q += 65535) {
+                prof_begin(ctx, "k_rlm_assemble");
+                k_rlm_assemble<<<dim3((n_phi + 7) / 8, std::min(65535, kps - q)), 256, 0, ctx->stream>>>(
+                    ws, cmt, d_t1, d_t2, list, n_phi, dim, o, kpts_per_sample, kp0 + q, H);
+                RLMB_LAUNCHED(ctx);
+            }
+        }
+    }
     return RLMB_OK;
 }
 
@@ -205,7 +271,7 @@ int launch_rlm_links(rlmb_context* ctx, const cplx* X, int n_phi, int g, int nsa
 // slots' sums are added by shuffles and through shared memory in a fixed order.  The work is
 // one atan2 per plaquette and state, so what matters is that a small number of states on a
 // fine mesh still fills the GPU's warps: with one thread per state the rlm n_phi = 16, g = 64,
-// 2-sample mesh took 2,960 us (32 threads walking 4,096 plaquettes each), with this split 14 us.
+// 2-sample mesh took 2,960 us (32 threads walking 4,096 plaquettes each), with this split 33 us.
 template <int TX, int TY>
 __global__ void __launch_bounds__(TX * TY)
 k_plaquettes(const cplx* __restrict__ U1, const cplx* __restrict__ U2, const double* __restrict__ W, int n_phi,

@@ -12,7 +12,8 @@ int launch_rlm_potential(rlmb_context* ctx, const double* x, const double* y, co
 size_t rlm_potential_ws_elems(int nimp, int nsamples, int dim);
 int launch_rlm_assemble(rlmb_context* ctx, const cplx* vmn, const cplx* cmt, const cplx* cjm,
                         const int* d_t1, const int* d_t2, int count, int kpts_per_sample,
-                        int n_phi, int dim, int o, cplx* H);
+                        int n_phi, int dim, int o, const int* uniq_t2, int n_t2, cplx* ws, cplx* H);
+size_t rlm_assemble_ws_elems(int n_phi, int dim, int nsamples, int n_t2);
 int launch_rlm_links(rlmb_context* ctx, const cplx* X, int n_phi, int g, int nsamples, cplx* U1, cplx* U2);
 int launch_plaquettes(rlmb_context* ctx, const cplx* U1, const cplx* U2, const double* W, int n_phi,
                       int g, int nsamples, int hlm, double* energies, double* chern);

@@ -41,3 +41,24 @@ def test_hlm_mesh_edges(lx, ly, g, samples):
     for k in range(samples):
         _close(e[k], c[k], ohlm.run_sample(p, pots[k]))
     ctx.close()
+
+
+@pytest.mark.parametrize("n_phi,g", [(8, 70), (70, 130), (65, 3)])
+def test_assemble_theta_groups(n_phi, g):
+    """More distinct theta_2 than one launch's list holds, unsorted and repeated; every entry
+    within 1e-13 of the largest one (sums of at most dim^2 = 1225 terms, n eps)."""
+    import torch
+
+    import rlmb
+    ctx = rlmb.Context(0)
+    p = orlm.RlmParams(n_phi, 1.0, 16.0, g, 1, 3)
+    cmn, cmt, cjm = orlm.prepare_coeff(p)
+    rng = np.random.default_rng(5)
+    v = rng.standard_normal(p.dim ** 2) + 1j * rng.standard_normal(p.dim ** 2)
+    t2 = np.concatenate([rng.permutation(g + 1), rng.integers(0, g + 1, 5)])
+    t1 = rng.integers(0, g + 1, len(t2))
+    got = ctx.rlm_assemble(*(torch.from_numpy(a).cuda() for a in (v, cmt, cjm)), n_phi, p.off_head, g, t1, t2)
+    for i in range(0, len(t2), max(1, len(t2) // 40)):
+        ref = orlm.assemble(p, v, cmt, cjm, int(t1[i]), int(t2[i])).reshape(n_phi, n_phi)
+        assert np.abs(got[i].cpu().numpy() - ref).max() <= 1e-13 * np.abs(ref).max()
+    ctx.close()
