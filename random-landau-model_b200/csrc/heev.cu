@@ -26,8 +26,9 @@
 //   small orders   up to order 20 (autotuned up to 80) the whole eigensolve is batched
 //                  two-sided Jacobi instead (jacobi.cuh).
 //
-// Waits are __syncthreads inside one CTA, except the panel queue's per-column counts
-// (k_hetrd_panel_q), whose spins are bounded in time and abort the chunk when they run out.
+// Waits are __syncthreads inside one CTA and the hardware barriers of a cluster
+// (k_hetrd_panel_c), except the panel queue's per-column counts (k_hetrd_panel_q), whose spins
+// are bounded in time and abort the chunk when they run out.
 #include "common.cuh"
 #include "jacobi.cuh"
 #include "tridiag_dc.cuh"
@@ -1682,6 +1683,469 @@ k_hetrd_panel_q(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, doubl
     }
 }
 
+// ---- the panel by a cluster of CTAs per matrix
+// barrier of the cluster (or of the CTA, P = 1): orders global and (distributed) shared memory
+__device__ __forceinline__ void panel_sync(int P) {
+    if (P == 1) {
+        __syncthreads();
+    } else {
+        asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    }
+}
+// the address of this CTA's shared variable p in CTA `rank` of the cluster
+template <class T>
+__device__ __forceinline__ T* panel_peer(T* p, int rank, int P) {
+    if (P == 1) return p;
+    T* q;
+    asm("mapa.u64 %0, %1, %2;" : "=l"(q) : "l"(p), "r"(rank));
+    return q;
+}
+
+// p += A v for the Hermitian leading m x m block stored in the upper triangle of a
+// (column-major, leading dimension ld; read only), dealt over the GW = P * warps warps of a
+// cluster (this warp: gw), each CTA summing into its own p (shared).  A unit is a segment of
+// seg 32-row blocks of a strip of HU_W columns: segment g meets the strips from 32 g seg / HU_W
+// on, and the units are counted off segment by segment, so that every warp gets the same
+// number within one.  A block is taken in four quarters of 4 columns, lane (lr = lane % 8,
+// lc = lane / 8) holding rows lr + 8 i (i < 4) and column lc of each: the cross-lane sums are
+// then over 4 lanes per row (three exchanges and one shared add per 512 entries) and over 8
+// lanes per column, once per unit.  The entries come through shared memory by cp.async, every
+// lane copying what it will read itself (no synchronisation): four quarters per warp, one
+// being multiplied while the next three are on their way, whatever the unit they belong to.
+static constexpr int HU_W = 16;
+static constexpr int HU_RING = 4 * 32 * 4;   // entries of a warp's ring: quarters x lanes x columns
+struct HemvPos {
+    int u, g, c0, r0, r1;   // unit counted from segment g on, its strip, block and last row
+    bool ok;
+    // the first unit at or after u counted from segment g on
+    __device__ __forceinline__ void unit(int m, int seg) {
+        const int nstrips = (m + HU_W - 1) / HU_W;
+        for (;; ++g) {
+            const int s0 = g * seg * (32 / HU_W), cnt = nstrips - s0;
+            if (cnt <= 0) {
+                ok = false;
+                return;
+            }
+            if (u < cnt) {
+                c0 = (s0 + u) * HU_W;
+                r0 = g * seg * 32;
+                r1 = min(min(c0 + HU_W, m), (g + 1) * seg * 32);   // rows on or above the diagonal
+                ok = true;
+                return;
+            }
+            u -= cnt;
+        }
+    }
+};
+template <class C>
+__device__ __forceinline__ void hemv_fetch(const C* __restrict__ a, int ld, int m, const HemvPos& t, int q, C* ring) {
+    const int lane = threadIdx.x & 31;
+    const int r = t.r0 + (lane & 7), c = t.c0 + 4 * q + (lane >> 3);
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(ring + q * 128 + lane);
+    const C* src = a + (size_t)c * ld + r;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int n = c < m && r + 8 * i <= c ? (int)sizeof(C) : 0;   // outside: zeros
+        const C* s = n ? src + 8 * i : a;
+        if constexpr (sizeof(C) == 16)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst + i * 32 * 16), "l"(s), "r"(n) : "memory");
+        else
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst + i * 32 * 8), "l"(s), "r"(n) : "memory");
+    }
+}
+// The first block's four quarters on their way (one group each).
+template <class C>
+__device__ __forceinline__ HemvPos hemv_begin(const C* __restrict__ a, int ld, int m, int gw, int seg, C* ring) {
+    HemvPos t;
+    t.u = gw;
+    t.g = 0;
+    t.c0 = t.r0 = t.r1 = 0;
+    t.unit(m, seg);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (t.ok) hemv_fetch(a, ld, m, t, q, ring);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    return t;
+}
+// The product from position t (hemv_begin) on; returns this lane's share of v^H A v.
+template <class C, class R>
+__device__ __forceinline__ R hemv_units(const C* __restrict__ a, int ld, int m, const C* __restrict__ v, C* p,
+                                        HemvPos t, int GW, int seg, C* ring) {
+    const int lane = threadIdx.x & 31, lr = lane & 7, lc = lane >> 3;
+    R quad = 0;
+    C es[4], vc[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) es[j] = vc[j] = cz<C>();
+    bool first = true;   // block of its unit
+#pragma unroll 1
+    while (t.ok) {
+        if (first)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                vc[j] = v[min(t.c0 + lc + 4 * j, m - 1)];   // (beyond the matrix the entries are 0)
+                es[j] = cz<C>();
+            }
+        HemvPos nx = t;
+        nx.r0 += 32;
+        const bool last = nx.r0 >= t.r1;
+        if (last) {
+            nx.u += GW;
+            nx.unit(m, seg);
+        }
+        const bool inside = t.c0 + HU_W <= m && t.r0 + 32 <= t.c0;
+        C rs[4], vr[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            rs[i] = cz<C>();
+            vr[i] = v[min(t.r0 + lr + 8 * i, m - 1)];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            asm volatile("cp.async.wait_group 3;\n" ::: "memory");
+            C x[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = ring[q * 128 + i * 32 + lane];
+            if (!inside) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (t.r0 + lr + 8 * i == t.c0 + lc + 4 * q) {   // the diagonal: real, counted once
+                        const C d = cscale(vc[q], x[i].x);
+                        rs[i] = cadd(rs[i], d);
+                        quad -= vr[i].x * d.x + vr[i].y * d.y;
+                        x[i] = cz<C>();
+                    }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                cfma(rs[i], x[i], vc[q]);
+                cfmac(es[q], x[i], vr[i]);
+            }
+            if (nx.ok) hemv_fetch(a, ld, m, nx, q, ring);
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+        }
+        {   // row sums over the four lanes of a row: lane ends with row r0 + lane
+            const bool u1 = (lane & 16) != 0, u0 = (lane & 8) != 0;
+            C y[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const C send = u1 ? rs[i] : rs[i + 2], keep = u1 ? rs[i + 2] : rs[i];
+                y[i] = cadd(keep, shfl_xor(send, 16));
+            }
+            const C send = u0 ? y[0] : y[1], keep = u0 ? y[1] : y[0];
+            const C s = cadd(keep, shfl_xor(send, 8));
+            const int r = t.r0 + lane;
+            if (r < min(t.c0 + HU_W, m)) {
+                const C vl = v[r];
+                quad += 2 * (vl.x * s.x + vl.y * s.y);
+                smem_atomic_add(&p[r], s);
+            }
+        }
+        if (last) {   // column sums over the eight lanes of a column: lane ends with column lc + 4 (lr / 2)
+            const bool u2 = (lane & 4) != 0, u1 = (lane & 2) != 0;
+            C y[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const C send = u2 ? es[j] : es[j + 2], keep = u2 ? es[j + 2] : es[j];
+                y[j] = cadd(keep, shfl_xor(send, 4));
+            }
+            const C send = u1 ? y[0] : y[1], keep = u1 ? y[1] : y[0];
+            C e = cadd(keep, shfl_xor(send, 2));
+            e = cadd(e, shfl_xor(e, 1));
+            const int c = t.c0 + lc + 4 * (lr >> 1);
+            if ((lr & 1) == 0 && c < m) smem_atomic_add(&p[c], e);
+        }
+        first = last;
+        t = nx;
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    return quad;
+}
+
+static constexpr int PC_MAX = 16;   // CTAs per cluster
+template <int NT, class R>
+__host__ __device__ constexpr size_t panel_c_smem(int m, int P) {
+    typedef typename Cx<R>::T C;
+    return (2 * (size_t)m + (NT / 32) * HU_RING + (size_t)P * 2 * HP_W_MAX + 4 * HP_W_MAX + 4) * sizeof(C) +
+           2 * (size_t)P * (NT / 32) * sizeof(R);
+}
+
+// The panel of one matrix by a cluster of P CTAs (blockIdx.x = matrix * P + rank): the leading
+// block's product is dealt over all the cluster's warps, the rows of the column vectors over
+// its CTAs in blocks of 8 (a warp takes 8 rows, its four 8-lane groups every fourth pair).  Per
+// column two cluster barriers:
+//   rows   w of the previous column, and with it the next column brought up to date, in one
+//          pass over the panel pairs; every CTA receives the column and its norm's parts
+//   -- barrier --   reflector (each CTA redundantly), A v and the pairs' products with v
+//   -- barrier --   sums of the CTAs' parts over distributed shared memory
+// x^H v for w = x - tau/2 (x^H v) v comes from v^H A v and the pairs' products, so that it
+// needs no barrier of its own.
+// Bound: the stream of the leading block (25 matrices of order 2500, clusters of 5: 229 ms for
+// 1.04 TB, 4.5 TB/s; of order 3000 in single precision 224 ms, 4.0 TB/s); 135 ms of the 229
+// remain with the loads taken out.  One CTA per matrix, 25 SMs at work, took 923 and 957 ms.
+template <int NT, class R>
+__global__ void __launch_bounds__(NT, NT > 256 ? 1 : 2)
+k_hetrd_panel_c(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, double* __restrict__ E,
+                typename Cx<R>::T* __restrict__ TAU, typename Cx<R>::T* __restrict__ PV,
+                typename Cx<R>::T* __restrict__ PW, int n, int m, int pw, int P) {
+    typedef typename Cx<R>::T C;
+    constexpr int NW = NT / 32;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C* ring = reinterpret_cast<C*>(smem_raw) + (threadIdx.x >> 5) * HU_RING;   // this warp's staging
+    C* v = reinterpret_cast<C*>(smem_raw) + NW * HU_RING;   // [m] column / reflector
+    C* pn = v + m;                                // [m] this CTA's part of A v
+    C* coefp = pn + m;                            // [P][2 * HP_W_MAX] the CTAs' parts of w_q^H v, v_q^H v
+    C* coef = coefp + (size_t)P * 2 * HP_W_MAX;   // [2 * HP_W_MAX] their sums
+    C* rowc = coef + 2 * HP_W_MAX;                // [2 * HP_W_MAX] V_q, W_q at the next column's index
+    C* scal_s = rowc + 2 * HP_W_MAX;              // [0..1] alpha by parity, [2] al, [3] w at the next column's index
+    R* quadp = reinterpret_cast<R*>(scal_s + 4);  // [P * NW] parts of v^H A v
+    R* normp = quadp + (size_t)P * NW;            // [P * NW] parts of the column's norm
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const size_t mat = blockIdx.x / P;
+    const int rank = (int)(blockIdx.x % P);
+    C* a = A + mat * (size_t)n * n;
+    double* dd = D + mat * n;
+    double* ee = E + mat * n;
+    C* tt = TAU + mat * n;
+    C* V = PV + mat * (size_t)pw * n;
+    C* W = PW + mat * (size_t)pw * n;
+    const int rl = lane & 7, ql = lane >> 3;   // row of the block of 8, pair group
+    if (m == n && rank == 0 && tid == 0) {
+        ee[n - 1] = 0.0;
+        tt[n - 1] = cz<C>();
+    }
+    C tau = cz<C>();
+    bool act = false;
+    HemvPos pos{};
+    int seg = 1;
+    for (int j = -1; j < pw; ++j) {
+        const int c = m - 1 - j;   // column of step j; the pass below finishes step j and starts step j + 1
+        if (j >= 0) {
+            panel_sync(P);
+            // reflector of step c-1 from the column's norm and alpha = column[c-1]
+            R xn2 = 0;
+            for (int i = lane; i < P * NW; i += 32) xn2 += normp[i];
+            xn2 = warp_sum(xn2);
+            R beta;
+            C scal;
+            reflector(scal_s[j & 1], xn2, beta, tau, scal);
+            act = !(tau.x == 0 && tau.y == 0);
+            for (int r = tid; r < c; r += NT) {
+                C x = r == c - 1 ? cm<C>(1, 0) : act ? cmul(scal, v[r]) : v[r];
+                v[r] = x;
+                pn[r] = cz<C>();
+                if ((r >> 3) % P == rank) {
+                    a[(size_t)c * n + r] = r == c - 1 ? cm<C>(beta, 0) : x;
+                    V[(size_t)j * n + r] = x;
+                }
+            }
+            if (rank == 0 && tid == 0) {
+                ee[c - 1] = beta;
+                tt[c - 1] = tau;
+            }
+            // the pairs at row c - 1, for the next column
+            C vq = cz<C>(), wq = cz<C>();
+            if (warp == 0 && lane < j) {
+                vq = __ldcg(V + (size_t)lane * n + c - 1);
+                wq = __ldcg(W + (size_t)lane * n + c - 1);
+            }
+            __syncthreads();
+            R quad = 0;
+            if (act) quad = hemv_units<C, R>(a, n, c, v, pn, pos, P * NW, seg, ring);
+            else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            quad = warp_sum(quad);
+            if (lane < P) panel_peer(quadp, lane, P)[rank * NW + warp] = quad;
+            // this CTA's rows of w_q^H v (even slots) and v_q^H v (odd slots)
+            for (int t2 = warp; t2 < 2 * j; t2 += NW) {
+                const C* y = ((t2 & 1) ? V : W) + (size_t)(t2 >> 1) * n;
+                C sd = cz<C>();
+                for (int i = lane;; i += 32) {
+                    const int r = ((i >> 3) * P + rank) * 8 + (i & 7);
+                    if (r >= c) break;
+                    cfmac(sd, y[r], v[r]);
+                }
+                sd = warp_sum(sd);
+                if (lane < P) panel_peer(coefp, lane, P)[rank * 2 * HP_W_MAX + t2] = sd;
+            }
+            panel_sync(P);
+            if (warp == 0) {
+                C ca = cz<C>(), cb = cz<C>(), y = cz<C>();
+                R q2 = 0;
+                for (int i = lane; i < P * NW; i += 32) q2 += quadp[i];
+                if (lane < j) {
+                    for (int k = 0; k < P; ++k) {
+                        ca = cadd(ca, coefp[k * 2 * HP_W_MAX + 2 * lane]);
+                        cb = cadd(cb, coefp[k * 2 * HP_W_MAX + 2 * lane + 1]);
+                    }
+                    coef[2 * lane] = ca;
+                    coef[2 * lane + 1] = cb;
+                    rowc[2 * lane] = vq;
+                    rowc[2 * lane + 1] = wq;
+                    q2 -= 2 * (ca.x * cb.x + ca.y * cb.y);
+                    cfma(y, vq, ca);
+                    cfma(y, wq, cb);
+                    y = cscale(y, (R)-1);
+                }
+                if (lane < P) y = cadd(y, panel_peer(pn, lane, P)[c - 1]);
+                y = warp_sum(y);
+                q2 = warp_sum(q2);
+                if (lane == 0) {
+                    // x = tau y, x^H v = conj(tau) (v^H y), al = -tau/2 x^H v = -|tau|^2/2 v^H y
+                    const R al = (R)-0.5 * cabs2(tau) * q2;
+                    C w = cmul(tau, y);
+                    w.x += al;   // v[c-1] = 1
+                    scal_s[2] = cm<C>(al, 0);
+                    scal_s[3] = act ? w : cz<C>();
+                }
+            }
+            __syncthreads();
+        }
+        // the next product's first entries on their way (the leading block does not change)
+        const bool next = j + 1 < pw;
+        if (next) {
+            const int mc = c - 1, ns = (mc + HU_W - 1) / HU_W;
+            const int blocks = ns * (ns + 2) / 4;   // 32-row blocks over all strips
+            seg = min(max(blocks / (4 * P * NW), 1), 32);
+            pos = hemv_begin(a, n, mc, warp * P + rank, seg, ring);
+        }
+        // rows: w_j, and the next column (index c - 1) brought up to date with the pairs 0 .. j
+        const int cn = c - 1;
+        const R al = j >= 0 ? scal_s[2].x : (R)0;
+        const C wcn = j >= 0 ? scal_s[3] : cz<C>();
+        R part = 0;
+        const int top = j >= 0 ? cn : m - 1;   // (step -1: the first column as stored)
+        const int col = j >= 0 ? cn : m - 1;
+        for (int b = warp * P + rank; b * 8 <= top; b += NW * P) {
+            const int r = b * 8 + rl;
+            const bool in = r <= top;
+            C x = cz<C>(), y = cz<C>(), s2 = cz<C>();
+            if (in) {
+                if (next && ql == 0) x = a[(size_t)col * n + r];
+                if (j >= 0) {
+                    for (int k = ql; k < P; k += 4) y = cadd(y, panel_peer(pn, k, P)[r]);
+                    C s1 = cz<C>();
+#pragma unroll 2
+                    for (int q = ql; q < j; q += 4) {
+                        const C vr = V[(size_t)q * n + r], wr = W[(size_t)q * n + r];
+                        cfma(s1, vr, coef[2 * q]);
+                        cfma(s1, wr, coef[2 * q + 1]);
+                        cfma(s2, vr, cconj(rowc[2 * q + 1]));
+                        cfma(s2, wr, cconj(rowc[2 * q]));
+                    }
+                    y = csub(y, s1);
+                }
+            }
+            if (j >= 0) {
+                x = csub(x, s2);
+                y = cadd(y, shfl_xor(y, 8));
+                y = cadd(y, shfl_xor(y, 16));
+                x = cadd(x, shfl_xor(x, 8));
+                x = cadd(x, shfl_xor(x, 16));
+                if (in) {
+                    const C vr = V[(size_t)j * n + r];
+                    C w = cmul(tau, y);
+                    w.x += al * vr.x;
+                    w.y += al * vr.y;
+                    if (!act) w = cz<C>();
+                    if (ql == 0) W[(size_t)j * n + r] = w;
+                    C u = cmul(vr, cconj(wcn));
+                    u = cadd(u, w);   // conj(v[cn]) = 1
+                    x = csub(x, u);
+                }
+            } else {
+                x = cm<C>(__shfl_sync(0xffffffffu, x.x, rl), __shfl_sync(0xffffffffu, x.y, rl));
+            }
+            if (next && in) {
+                if (r == col) x.y = 0;
+                for (int k = ql; k < P; k += 4) {
+                    panel_peer(v, k, P)[r] = x;
+                    if (r == col - 1) panel_peer(scal_s, k, P)[(j + 1) & 1] = x;
+                }
+                if (ql == 0) {
+                    if (r == col) dd[col] = x.x;
+                    if (r < col - 1) part += cabs2(x);
+                }
+            }
+        }
+        if (next) {
+            part = warp_sum(part);
+            if (lane < P) panel_peer(normp, lane, P)[rank * NW + warp] = part;
+        }
+    }
+    panel_sync(P);   // no CTA leaves while a peer may still read its shared memory
+}
+
+template <int NT, class R>
+static cudaLaunchConfig_t panel_c_config(cudaLaunchAttribute* at, cudaStream_t st, int m, int nb, int P) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(nb * P);
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = panel_c_smem<NT, R>(m, P);
+    cfg.stream = st;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = P;
+    at->val.clusterDim.y = 1;
+    at->val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+template <int NT, class R>
+static cudaError_t panel_c_attrs(int m, int P) {
+    auto kern = k_hetrd_panel_c<NT, R>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)panel_c_smem<NT, R>(m, P));
+    if (e == cudaSuccess && P > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e;
+}
+template <int NT, class R>
+static cudaError_t launch_panel_c(cudaStream_t st, typename Cx<R>::T* A, double* D, double* E, typename Cx<R>::T* TAU,
+                                  typename Cx<R>::T* PV, typename Cx<R>::T* PW, int n, int m, int pw, int nb, int P) {
+    const cudaError_t e = panel_c_attrs<NT, R>(m, P);
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = panel_c_config<NT, R>(at, st, m, nb, P);
+    return cudaLaunchKernelEx(&cfg, k_hetrd_panel_c<NT, R>, A, D, E, TAU, PV, PW, n, m, pw, P);
+}
+
+// Shape of the cluster panel for a chunk of nb matrices, P = 0 where one CTA per matrix (or the
+// panel queue) is the better one.  The clusters of one launch should all run at once: of the
+// shapes whose nb clusters fit the device together the one with the most threads per matrix is
+// taken (measured best at orders 300 to 1000 with 1 to 81 matrices, wider CTAs winning ties),
+// if that is at least 1.5 (below order 512: 2) times the 512 threads of one CTA per matrix:
+// panels of order 300, double precision, 18 matrices 3.46 -> 2.63 ms, 36 3.47 -> 2.86, but 81
+// 3.49 -> 3.71; of order 512 10.9 -> 5.9, 11.3 -> 6.9, 13.1 -> 10.9; of order 2500, 25 matrices,
+// 923 -> 229.
+struct PanelShape {
+    int nt, P;
+};
+template <int NT, class R>
+static void panel_shape_try(int m, int nb, PanelShape* best) {
+    for (int P = PC_MAX; P >= 2; --P) {
+        if (NT * P <= best->nt * best->P) return;
+        if (panel_c_smem<NT, R>(m, P) > 227 * 1024) continue;
+        int active = 0;
+        cudaLaunchAttribute at[1];
+        const cudaLaunchConfig_t cfg = panel_c_config<NT, R>(at, 0, m, nb, P);
+        if (panel_c_attrs<NT, R>(m, P) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&active, k_hetrd_panel_c<NT, R>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            continue;
+        }
+        if (active >= nb) *best = PanelShape{NT, P};
+    }
+}
+template <class R>
+static PanelShape panel_shape(int m, int nb) {
+    PanelShape s{0, 0};
+    if (nb > 148) return s;
+    panel_shape_try<512, R>(m, nb, &s);
+    panel_shape_try<384, R>(m, nb, &s);
+    panel_shape_try<256, R>(m, nb, &s);
+    if (s.nt * s.P < (m >= 512 ? 768 : 1024)) s.P = 0;
+    return s;
+}
+
 // [V | W] (r, k) and [W | V]^H (k, c) of a panel: the operands of A -= V W^H + W V^H.
 template <class C, int w>
 struct OpPanelA {
@@ -2443,9 +2907,20 @@ static int tridiagonalise(rlmb_context* ctx, cudaStream_t st, const HeevPlan& p,
         const int grid = std::min(nb, queue ? qper * sms : sms);
         // the queue's counters, and its abort flag, which k_panel_abort_info reads in every case
         if (cudaMemsetAsync(Q, 0, (8 + (size_t)nb) * sizeof(int), st) != cudaSuccess) return RLMB_ERR_CUDA;
+        // chunks of few matrices: a cluster of CTAs per matrix (k_hetrd_panel_c)
+        PanelShape shape{};
+        if (p.panel_nt == 0) shape = panel_shape<R>(n, nb);
         for (int k = 0; k < p.npanels; ++k) {
             RLMB_CHUNK_PROF("k_hetrd_panel");
-            if (queue && qnt == 256)
+            if (shape.P > 0) {
+                if (shape.nt < 512 && k > 0) {   // (the vectors have shrunk: a wider CTA may fit by now)
+                    const PanelShape wider = panel_shape<R>(m, nb);
+                    if (wider.P > 0) shape = wider;
+                }
+                const auto launch = shape.nt == 512 ? launch_panel_c<512, R>
+                                  : shape.nt == 384 ? launch_panel_c<384, R> : launch_panel_c<256, R>;
+                if (launch(st, A, D, E, TAU, PV, PWb, n, m, pw, nb, shape.P) != cudaSuccess) return RLMB_ERR_CUDA;
+            } else if (queue && qnt == 256)
                 k_hetrd_panel_q<256, R><<<grid, 256, smem, st>>>(A, D, E, TAU, PV, PWb, n, m, pw, nb, Q,
                                                                  (long long)k * ((long long)nb * pw + grid),
                                                                  k * pw, info);
@@ -2858,7 +3333,7 @@ void rlmb::tune_free(rlmb_context* ctx) {
     ctx->tune = nullptr;
 }
 
-static std::vector<HeevTune> tune_candidates(int n, bool mixed) {
+static std::vector<HeevTune> tune_candidates(int n, bool mixed, int nb) {
     std::vector<HeevTune> out;
     if (n <= JAC_MAX_N) {
         HeevTune t;
@@ -2868,8 +3343,10 @@ static std::vector<HeevTune> tune_candidates(int n, bool mixed) {
     for (int blocked = 0; blocked <= 1; ++blocked) {
         if (blocked && n < 128) continue;
         for (int gemm = 0; gemm <= 1; ++gemm)
-            for (int nt : {256, 512}) {
-                if (!blocked && nt == 256) continue;   // no panels: one entry
+            for (int nt : {0, 256, 512}) {
+                if (!blocked && nt != 512) continue;   // no panels: one entry
+                // the built-in panels where they are clusters (few matrices)
+                if (nt == 0 && (mixed ? panel_shape<float>(n, nb) : panel_shape<double>(n, nb)).P == 0) continue;
                 for (int xt : {64, 128})
                     for (int bs : {64, 128}) {
                         if ((!gemm || mixed) && xt == 128) continue;
@@ -2901,7 +3378,7 @@ static int autotune(rlmb_context* ctx, int n, bool mixed, int refine_steps, int 
     const size_t nn = (size_t)n * n;
     const size_t cap = std::min<size_t>((size_t)2 * sms, ((size_t)2 << 30) / (nn * sizeof(cplx)));
     const int tb = (int)std::max<size_t>(1, std::min<size_t>((size_t)batch, cap));
-    const std::vector<HeevTune> cands = tune_candidates(n, mixed);
+    const std::vector<HeevTune> cands = tune_candidates(n, mixed, tb);
     size_t per = 0;
     for (const HeevTune& t : cands) {
         const HeevPlan pl = heev_plan(n, mixed, refine_steps, band, t);
