@@ -1398,7 +1398,7 @@ static constexpr int HP_W_WIDE_MIN = 1024;
 static constexpr int HT_TAIL = 64;   // order below which the unblocked kernel finishes
 static constexpr int HT_BLOCKED_MIN = 256;   // orders from which the blocked reduction runs
 static constexpr int DC_DEFAULT_MIN = 600;   // orders from which divide and conquer is the built-in tridiagonal solver (measured: even with bisection at 512, 1.4x at 1024, 2.3x at 3000)
-static constexpr int JAC_DEFAULT_MAX = 20;    // orders up to which k_jacobi is the built-in solver (measured: 2.1x the Householder path at 16, even at 24)
+static constexpr int JAC_DEFAULT_MAX = 20;    // orders up to which k_jacobi is the built-in solver (measured: 2.4x the Householder path at 16, 2.1x at 20, 1.2x at 24, even at 28)
 static constexpr int QUEUE_NT_DEFAULT = 512;   // panel queue CTAs: 512 threads, one per SM
 static constexpr int TUNE_MIN_N = 16;         // orders the autotuner tunes: TUNE_MIN_N .. TUNE_MAX_N
 static constexpr int TUNE_MAX_N = 1024;
@@ -3213,7 +3213,7 @@ static int heev_chunk(rlmb_context* ctx, cudaStream_t st, const HeevPlan& p, cpl
         if (cudaFuncSetAttribute(k_jacobi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem_jac) != cudaSuccess)
             return RLMB_ERR_CUDA;
         RLMB_CHUNK_PROF("k_jacobi");
-        k_jacobi<<<nb, jacobi_threads(n), p.smem_jac, st>>>(A, W, info, n);
+        k_jacobi<<<nb, jacobi_threads(n, nb), p.smem_jac, st>>>(A, W, info, n);
         RLMB_CHUNK_LAUNCHED();
         return RLMB_OK;
     }

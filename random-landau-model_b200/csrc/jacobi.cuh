@@ -10,15 +10,21 @@
 // of one round touch disjoint index pairs and run in parallel):
 //   for each sweep, until the off-diagonal mass is below 1e-32 of the total mass:
 //     for each of the m-1 rounds (m = n rounded up to even; index n is a bye for odd n):
-//       1. thread k computes the rotation of pair k from A_pp, A_qq and A_pq = r e (|e| = 1):
-//          tau = (A_qq - A_pp) / 2r, t = sgn(tau) / (|tau| + sqrt(1 + tau^2)),
-//          c = 1/sqrt(1 + t^2), s = t c, J = [[c, s e], [-s conj(e), c]] on (p, q);
-//          then J^H A J has (p, q) entry 0 and diagonal A_pp - t r, A_qq + t r;
-//       2. column phase, thread = (row, pair group):    A <- A J,   V <- V J;
-//       3. row phase,    thread = (column, pair group): A <- J^H A, with the (p,p), (q,q),
-//          (p,q), (q,p) entries set to their exact values.
-// Each phase is a __syncthreads apart; there are no other waits.  Within a phase the pairs are
-// disjoint, so the threads of a phase never touch the same element.
+//       1. thread k computes the rotation of pair k from A_pp, A_qq and b = A_pq: with
+//          h = A_qq - A_pp and u = 2 sgn(h) / (|h| + sqrt(h^2 + 4 |b|^2)) the tangent is
+//          t = u |b|, c = 1/sqrt(1 + t^2), J = [[c, c u b], [-c u conj(b), c]] on (p, q);
+//          then J^H A J has (p, q) entry 0 and diagonal A_pp - u |b|^2, A_qq + u |b|^2;
+//       2. A <- J^H A J by 2 x 2 blocks: a thread takes the block of two pairs, applies both
+//          rotations and writes it back (only the upper triangle is kept: an entry that lies
+//          below the diagonal is read and written as its conjugate); V <- V J, a thread per
+//          (row, pair).
+// Two __syncthreads per round; there are no other waits.  The blocks of a round are disjoint,
+// so no two threads touch the same element.  The round is a chain of latencies (the three
+// dependent square roots and divisions of the rotation, the shared-memory round trips), so it
+// is kept short: with separate column and row phases over A and a rotation through |b|, tau
+// and t the order-16 kernel took 202 us on 81 matrices and 1,143 us on 8,450; now 133 and 875.
+// On many matrices the bound is the shared-memory pipe (by count of the accesses about 200
+// wavefronts of the 265 cycles a round takes per matrix and SM, a third of them V's).
 //
 // Shared memory: A with an odd leading dimension (the row phase's stride-ld accesses of 16
 // bytes then hit distinct banks), V with leading dimension n, the round's rotations, the
@@ -27,47 +33,52 @@
 #pragma once
 #include "common.cuh"
 
+#include <algorithm>
+
 namespace rlmb {
 
 static constexpr int JAC_MAX_N = 80;
 static constexpr int JAC_MAX_SWEEPS = 30;
 
 struct JacRot {
-    double c, ap, aq;   // cosine, new diagonal entries (p,p) and (q,q)
+    double c;           // cosine
     cplx se;            // s e
-    int p, q;           // q < 0: no rotation this round (bye, or A_pq already zero)
+    int p, q;           // p < q; q = n: the bye of an odd order
+    int on;             // 0: no rotation this round (bye, or A_pq already zero)
 };
 
-// Thread layout: thread = (row or column r, pair group g), r = tid % n, g = tid / n; group g
-// takes pairs g, g + G, g + 2G, ...  The CTA gets W warps, enough that the matrices resident
-// per SM (as many as fit in its 228 KB of shared memory) bring about 20 warps, and G fills
-// those warps' lanes: at small orders many one-warp CTAs share an SM, from order ~60 on the
-// matrix alone fills the SM's shared memory and its own 8 warps must hide the latency.
-__host__ __device__ inline int jacobi_groups(int n);
+// Warps per matrix: enough that the matrices resident per SM (as many as fit in its 228 KB of
+// shared memory, or the batch's share of them) bring about 20 warps, and no more than give
+// every thread a task; from order ~60 on a matrix alone fills the SM's shared memory and its
+// own 8 warps must hide the latency.
 __host__ __device__ inline size_t jacobi_smem(int n);
-__host__ __device__ inline int jacobi_warps(int n) {
+inline int jacobi_threads(int n, int nb) {
+    const int np = (n + (n & 1)) / 2;
     int per_sm = (int)((size_t)233472 / (jacobi_smem(n) + 1024));
-    per_sm = per_sm < 1 ? 1 : per_sm > 32 ? 32 : per_sm;
-    const int w = (20 + per_sm - 1) / per_sm;
-    return w > 8 ? 8 : w;
-}
-__host__ __device__ inline int jacobi_groups(int n) {
-    const int np = (n + (n & 1)) / 2;
-    int g = 32 * jacobi_warps(n) / (n > 0 ? n : 1);
-    g = g < np ? g : np;
-    return g > 0 ? g : 1;
-}
-__host__ __device__ inline int jacobi_threads(int n) {
-    const int np = (n + (n & 1)) / 2;
-    int t = n * jacobi_groups(n);
-    t = t > np ? t : np;   // step 1 needs a thread per pair
-    return ((t + 31) / 32) * 32;
+    per_sm = std::min(std::min(std::max(per_sm, 1), 32), (nb + 147) / 148);
+    const int tasks = np * (np - 1) / 2 + n * np;
+    int w = std::min((20 + per_sm - 1) / per_sm, 8);
+    w = std::max(std::min(w, tasks / 32), 1);
+    return 32 * std::max(w, (std::max(np, n) + 31) / 32);   // step 1 needs a thread per pair
 }
 __host__ __device__ inline int jacobi_ld(int n) { return n | 1; }
 __host__ __device__ inline size_t jacobi_smem(int n) {
     const int m = n + (n & 1);
     return (size_t)sizeof(cplx) * ((size_t)n * jacobi_ld(n) + (size_t)n * n) + sizeof(JacRot) * (size_t)(m / 2) +
            sizeof(double) * (2 * 32 + 2 * (size_t)n) + sizeof(int) * (size_t)n;
+}
+
+// Pair k of round rd of the tournament of m players, p < q.
+__device__ __forceinline__ void jac_pair(int k, int rd, int m, int& p, int& q) {
+    int a = m - 1, b = rd;
+    if (k > 0) {
+        a = rd + k;
+        if (a >= m - 1) a -= m - 1;
+        b = rd - k;
+        if (b < 0) b += m - 1;
+    }
+    p = a < b ? a : b;
+    q = a < b ? b : a;
 }
 
 // (x_p, x_q) <- (c x_p - conj(se) x_q, se x_p + c x_q): columns p, q of A J or V J
@@ -94,7 +105,6 @@ __global__ void __launch_bounds__(256) k_jacobi(cplx* __restrict__ Ag, double* _
     const int ld = jacobi_ld(n);
     const int m = n + (n & 1);
     const int np = m / 2;
-    const int G = jacobi_groups(n);
     cplx* A = reinterpret_cast<cplx*>(jac_smem);
     cplx* V = A + (size_t)n * ld;
     JacRot* rot = reinterpret_cast<JacRot*>(V + (size_t)n * n);
@@ -103,19 +113,19 @@ __global__ void __launch_bounds__(256) k_jacobi(cplx* __restrict__ Ag, double* _
     int* rank = reinterpret_cast<int*>(lam + 2 * n);
     const int tid = threadIdx.x;
     const int nt = blockDim.x;
-    const int r = tid % n;             // row (column phase) or column (row phase)
-    const int g = tid / n;             // pair group; g >= G: idle in the phases
+    const int G = nt / n;              // (threads of a whole column: loads, stores, masses)
+    const int r = tid % n, g = tid / n;
     const bool act = g < G;
+    const int nblk = np * (np - 1) / 2, nv = n * np;
     const size_t mat = blockIdx.x;
     cplx* Am = Ag + mat * (size_t)n * n;
 
-    // load: the upper triangle of column c is rows 0..c; the lower triangle is its conjugate
+    // load: the upper triangle of column c is rows 0..c (the lower one is not kept)
     for (int c = g; act && c < n; c += G) {
         if (r <= c) {
             cplx v = Am[(size_t)c * n + r];
             if (c == r) v.y = 0.0;
             A[(size_t)c * ld + r] = v;
-            A[(size_t)r * ld + c] = cconj(v);
         }
         V[(size_t)c * n + r] = mk(c == r ? 1.0 : 0.0, 0.0);
     }
@@ -126,9 +136,9 @@ __global__ void __launch_bounds__(256) k_jacobi(cplx* __restrict__ Ag, double* _
         // off-diagonal and diagonal mass
         double off = 0.0, dia = 0.0;
         for (int c = g; act && c < n; c += G) {
-            const double a2 = cabs2(A[(size_t)c * ld + r]);
+            const double a2 = r <= c ? cabs2(A[(size_t)c * ld + r]) : 0.0;
             if (c == r) dia += a2;
-            else off += a2;
+            else off += 2.0 * a2;
         }
         off = warp_sum(off);
         dia = warp_sum(dia);
@@ -153,127 +163,79 @@ __global__ void __launch_bounds__(256) k_jacobi(cplx* __restrict__ Ag, double* _
             // 1. rotations of the round, thread k for pair k
             if (tid < np) {
                 int p, q;
-                if (tid == 0) {
-                    p = m - 1;
-                    q = rd;
-                } else {
-                    p = (rd + tid) % (m - 1);
-                    q = (rd - tid + m - 1) % (m - 1);
-                }
-                if (p > q) {
-                    const int s = p;
-                    p = q;
-                    q = s;
-                }
+                jac_pair(tid, rd, m, p, q);
                 JacRot R;
                 R.p = p;
-                R.q = -1;
+                R.q = q;
+                R.on = 0;
                 R.c = 1.0;
                 R.se = mk(0.0, 0.0);
-                R.ap = R.aq = 0.0;
                 if (q < n) {
                     const cplx b = A[(size_t)q * ld + p];
-                    const double rr = sqrt(cabs2(b));
-                    if (rr >= 1e-300) {
+                    const double b2 = cabs2(b);
+                    if (b2 > 0.0) {
                         const double a = A[(size_t)p * ld + p].x, d = A[(size_t)q * ld + q].x;
-                        const double tau = (d - a) / (2.0 * rr);
-                        const double at = fabs(tau);
-                        const double tt = at > 1e150 ? 0.5 / at : 1.0 / (at + sqrt(1.0 + tau * tau));
-                        const double tn = tau >= 0.0 ? tt : -tt;
-                        const double c = 1.0 / sqrt(1.0 + tn * tn);
-                        const double s = tn * c;
-                        R.q = q;
+                        const double h = d - a;
+                        const double u = copysign(2.0, h) / (fabs(h) + sqrt(fma(4.0, b2, h * h)));
+                        const double c = rsqrt(fma(u * b2, u, 1.0));
+                        R.on = 1;
                         R.c = c;
-                        R.se = mk(s * b.x / rr, s * b.y / rr);
-                        R.ap = a - tn * rr;
-                        R.aq = d + tn * rr;
+                        R.se = cscale(b, u * c);
+                        A[(size_t)p * ld + p] = mk(a - u * b2, 0.0);
+                        A[(size_t)q * ld + q] = mk(d + u * b2, 0.0);
+                        A[(size_t)q * ld + p] = mk(0.0, 0.0);
                     }
                 }
                 rot[tid] = R;
             }
             __syncthreads();
-            // 2. columns: A <- A J, V <- V J (r = row); two pairs in flight per thread
-            if (act) {
-                for (int k = g; k < np; k += 2 * G) {
+            // 2. the blocks of two pairs (k, l), k < l, then V
+            for (int t = tid; t < nblk + nv; t += nt) {
+                if (t < nblk) {
+                    int l = (int)((1.0f + sqrtf(8.0f * t + 1.0f)) * 0.5f);
+                    if (l * (l - 1) / 2 > t) --l;
+                    else if (l * (l + 1) / 2 <= t) ++l;
+                    const JacRot K = rot[t - l * (l - 1) / 2], L = rot[l];
+                    if (!K.on && !L.on) continue;
+                    const int kq = K.q, lq = L.q;
+                    const bool ok = kq < n, ol = lq < n;   // (an odd order's bye has no second index)
+                    const int kr = ok ? kq : K.p, lr = ol ? lq : L.p;
+                    const bool f0 = K.p > L.p, f1 = kr > L.p, f2 = K.p > lr, f3 = kr > lr;   // kept as the conjugate
+                    cplx* a0 = A + (f0 ? K.p * ld + L.p : L.p * ld + K.p);
+                    cplx* a1 = A + (f1 ? kr * ld + L.p : L.p * ld + kr);
+                    cplx* a2 = A + (f2 ? K.p * ld + lr : lr * ld + K.p);
+                    cplx* a3 = A + (f3 ? kr * ld + lr : lr * ld + kr);
+                    cplx pp = *a0, qp = *a1, pq = *a2, qq = *a3;
+                    if (f0) pp.y = -pp.y;
+                    if (f1) qp.y = -qp.y;
+                    if (f2) pq.y = -pq.y;
+                    if (f3) qq.y = -qq.y;
+                    if (L.on) {
+                        jac_rot_cols(pp, pq, L.c, L.se);
+                        jac_rot_cols(qp, qq, L.c, L.se);
+                    }
+                    if (K.on) {
+                        jac_rot_rows(pp, qp, K.c, K.se);
+                        jac_rot_rows(pq, qq, K.c, K.se);
+                    }
+                    if (f0) pp.y = -pp.y;
+                    if (f1) qp.y = -qp.y;
+                    if (f2) pq.y = -pq.y;
+                    if (f3) qq.y = -qq.y;
+                    *a0 = pp;
+                    if (ok) *a1 = qp;
+                    if (ol) *a2 = pq;
+                    if (ok && ol) *a3 = qq;
+                } else {
+                    const int k = (t - nblk) / n, row = (t - nblk) - k * n;
                     const JacRot R0 = rot[k];
-                    const bool two = k + G < np;
-                    const JacRot R1 = two ? rot[k + G] : R0;
-                    const bool d0 = R0.q >= 0, d1 = two && R1.q >= 0;
-                    cplx a0p, a0q, v0p, v0q, a1p, a1q, v1p, v1q;
-                    if (d0) {
-                        a0p = A[(size_t)R0.p * ld + r];
-                        a0q = A[(size_t)R0.q * ld + r];
-                        v0p = V[(size_t)R0.p * n + r];
-                        v0q = V[(size_t)R0.q * n + r];
-                    }
-                    if (d1) {
-                        a1p = A[(size_t)R1.p * ld + r];
-                        a1q = A[(size_t)R1.q * ld + r];
-                        v1p = V[(size_t)R1.p * n + r];
-                        v1q = V[(size_t)R1.q * n + r];
-                    }
-                    if (d0) {
-                        jac_rot_cols(a0p, a0q, R0.c, R0.se);
-                        jac_rot_cols(v0p, v0q, R0.c, R0.se);
-                        A[(size_t)R0.p * ld + r] = a0p;
-                        A[(size_t)R0.q * ld + r] = a0q;
-                        V[(size_t)R0.p * n + r] = v0p;
-                        V[(size_t)R0.q * n + r] = v0q;
-                    }
-                    if (d1) {
-                        jac_rot_cols(a1p, a1q, R1.c, R1.se);
-                        jac_rot_cols(v1p, v1q, R1.c, R1.se);
-                        A[(size_t)R1.p * ld + r] = a1p;
-                        A[(size_t)R1.q * ld + r] = a1q;
-                        V[(size_t)R1.p * n + r] = v1p;
-                        V[(size_t)R1.q * n + r] = v1q;
-                    }
-                }
-            }
-            __syncthreads();
-            // 3. rows: A <- J^H A (r = column); the pair's own 2x2 block gets its exact values
-            if (act) {
-                cplx* col = A + (size_t)r * ld;
-                for (int k = g; k < np; k += 2 * G) {
-                    const JacRot R0 = rot[k];
-                    const bool two = k + G < np;
-                    const JacRot R1 = two ? rot[k + G] : R0;
-                    const bool d0 = R0.q >= 0, d1 = two && R1.q >= 0;
-                    cplx y0p, y0q, y1p, y1q;
-                    if (d0) {
-                        y0p = col[R0.p];
-                        y0q = col[R0.q];
-                    }
-                    if (d1) {
-                        y1p = col[R1.p];
-                        y1q = col[R1.q];
-                    }
-                    if (d0) {
-                        if (r == R0.p) {
-                            y0p = mk(R0.ap, 0.0);
-                            y0q = mk(0.0, 0.0);
-                        } else if (r == R0.q) {
-                            y0p = mk(0.0, 0.0);
-                            y0q = mk(R0.aq, 0.0);
-                        } else {
-                            jac_rot_rows(y0p, y0q, R0.c, R0.se);
-                        }
-                        col[R0.p] = y0p;
-                        col[R0.q] = y0q;
-                    }
-                    if (d1) {
-                        if (r == R1.p) {
-                            y1p = mk(R1.ap, 0.0);
-                            y1q = mk(0.0, 0.0);
-                        } else if (r == R1.q) {
-                            y1p = mk(0.0, 0.0);
-                            y1q = mk(R1.aq, 0.0);
-                        } else {
-                            jac_rot_rows(y1p, y1q, R1.c, R1.se);
-                        }
-                        col[R1.p] = y1p;
-                        col[R1.q] = y1q;
-                    }
+                    if (!R0.on) continue;
+                    cplx* vp = V + (size_t)R0.p * n + row;
+                    cplx* vq = V + (size_t)R0.q * n + row;
+                    cplx xp = *vp, xq = *vq;
+                    jac_rot_cols(xp, xq, R0.c, R0.se);
+                    *vp = xp;
+                    *vq = xq;
                 }
             }
             __syncthreads();
