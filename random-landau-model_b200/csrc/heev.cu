@@ -77,35 +77,6 @@ __device__ __forceinline__ C block_sum_c(C v, R* red) {
     return s;
 }
 
-// Transpose-reduce for a 16-column group: lane l holds v[j] (the contribution of row l
-// to column j); on return lane l (and l^16) holds the sum over all 32 lanes of v[l & 15].
-template <class C>
-__device__ __forceinline__ C transpose_reduce16(C (&v)[16]) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) v[j] = cadd(v[j], shfl_xor(v[j], 16));
-#pragma unroll
-    for (int s = 8; s >= 1; s >>= 1) {
-        const bool up = (lane & s) != 0;
-#pragma unroll
-        for (int j = 0; j < s; ++j) {
-            C send = up ? v[j] : v[j + s];
-            C keep = up ? v[j + s] : v[j];
-            v[j] = cadd(keep, shfl_xor(send, s));
-        }
-    }
-    return v[0];
-}
-
-__device__ __forceinline__ void tile_of(int t, int& R, int& C) {
-    // t-th tile (row block R <= column block C) in column-major order of the upper triangle
-    int c = (int)((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
-    while ((c + 1) * (c + 2) / 2 <= t) ++c;
-    while (c * (c + 1) / 2 > t) --c;
-    C = c;
-    R = t - c * (c + 1) / 2;
-}
-
 template <class C>
 __device__ __forceinline__ void smem_atomic_add(C* p, C v) {
     atomicAdd(&p->x, v.x);
@@ -127,69 +98,116 @@ struct SharedStore {
     __device__ __forceinline__ C* at(int r, int c) const { return s + (c * (c + 1) / 2 + r); }
 };
 
-// One pass over the upper triangle of the leading m x m block, 32x32 tiles dealt to
-// warps: applies the rank-2 update A -= v w^H + w v^H of the previous reflector (if upd)
-// and accumulates pn += A' vn for the next one (if acc), reading and writing every
-// stored element once.  All loads of a 16-column half tile are issued before its stores.
-template <int NT, class C, class S>
-__device__ __forceinline__ void fused_pass(S st, int m, const C* __restrict__ v,
-                                           const C* __restrict__ w, bool upd,
-                                           const C* __restrict__ vn, bool acc, C* pn) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    constexpr int NW = NT / 32;
-    const int nb = (m + 31) / 32;
-    const int nitems = nb * (nb + 1);   // two 16-column halves per 32x32 tile
-    for (int it = warp; it < nitems; it += NW) {
-        int R, Cb;
-        tile_of(it >> 1, R, Cb);
-        const int c0 = Cb * 32 + 16 * (it & 1);
-        if (c0 >= m) continue;
-        const int r = R * 32 + lane;
-        const bool rin = r < m;
-        const C vr = rin ? v[r] : cz<C>();
-        const C wr = rin ? w[r] : cz<C>();
-        const C vnr = rin ? vn[r] : cz<C>();
-        C rowacc = cz<C>();
-        C e[16];
+// One 16 x 16 tile (rows from r0, columns from c0) of the upper triangle of the leading m x m
+// block: applies the rank-2 update A -= v w^H + w v^H of the previous reflector (UPD) and forms
+// the tile's part of A' vn.  Lane (lr = lane % 8, lc = lane / 8) holds rows lr + 8 i (i < 2) and
+// columns lc + 4 j (j < 4), so that the cross-lane sums are over 4 lanes per row and 8 per
+// column.  rowsum: on lanes with bit 3 clear, row r0 + lr + 8 (lane / 16); colsum: on even
+// lanes, column c0 + lc + 4 (lr / 2).  The vectors are readable up to the next multiple of 16.
+template <bool INSIDE, bool UPD, class C, class R, class S>
+__device__ __forceinline__ void hetrd_tile(const S& st, int m, int r0, int c0, const C* __restrict__ v,
+                                           const C* __restrict__ w, const C* __restrict__ vn, C& rowsum, C& colsum,
+                                           R& quad) {
+    const int lane = threadIdx.x & 31, lr = lane & 7, lc = lane >> 3;
+    C vr[2], wr[2], vnr[2], rs[2], es[4];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const int cc = c0 + j;
-            e[j] = (rin && cc < m && r <= cc) ? *st.at(r, cc) : cz<C>();
+    for (int i = 0; i < 2; ++i) {
+        const int r = r0 + lr + 8 * i;
+        if (UPD) {
+            vr[i] = v[r];
+            wr[i] = w[r];
+        }
+        vnr[i] = vn[r];
+        rs[i] = cz<C>();
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int c = c0 + lc + 4 * j;
+        C x[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int r = r0 + lr + 8 * i;
+            x[i] = INSIDE || (c < m && r <= c) ? *st.at(r, c) : cz<C>();
+        }
+        const C vnc = vn[c];
+        es[j] = cz<C>();
+        C vc, wc;
+        if (UPD) {
+            vc = cconj(v[c]);
+            wc = cconj(w[c]);
         }
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const int cc = c0 + j;
-            const bool valid = rin && cc < m && r <= cc;
-            C x = e[j];
-            if (upd) {
-                const C vc = cc < m ? v[cc] : cz<C>();
-                const C wc = cc < m ? w[cc] : cz<C>();
-                C u = cmul(vr, cconj(wc));
-                cfma(u, wr, cconj(vc));
-                x = csub(x, u);
-                if (r == cc) x.y = 0;
-                if (valid) *st.at(r, cc) = x;
+        for (int i = 0; i < 2; ++i) {
+            const int r = r0 + lr + 8 * i;
+            const bool in = INSIDE || (c < m && r <= c);
+            if (UPD) {
+                C u = cmul(vr[i], wc);
+                cfma(u, wr[i], vc);
+                x[i] = csub(x[i], u);
+                if (!INSIDE && r == c) x[i].y = 0;
+                if (in) *st.at(r, c) = x[i];
+                else x[i] = cz<C>();
             }
-            if (acc) {
-                const C vnc = cc < m ? vn[cc] : cz<C>();
-                if (!valid) {
-                    e[j] = cz<C>();
-                } else if (r == cc) {
-                    rowacc = cadd(rowacc, cscale(vnc, x.x));
-                    e[j] = cz<C>();
-                } else {
-                    cfma(rowacc, x, vnc);
-                    e[j] = cmulc(x, vnr);   // column partial: conj(A'[r][cc]) vn[r]
-                }
+            if (!INSIDE && r == c) {   // the diagonal: real, counted once
+                const C d = cscale(vnc, x[i].x);
+                rs[i] = cadd(rs[i], d);
+                quad -= vnr[i].x * d.x + vnr[i].y * d.y;
+                x[i] = cz<C>();
             }
-        }
-        if (acc) {
-            const C cs = transpose_reduce16(e);
-            const int cl = c0 + (lane & 15);
-            if (lane < 16 && cl < m) smem_atomic_add(&pn[cl], cs);
-            if (rin) smem_atomic_add(&pn[r], rowacc);
+            cfma(rs[i], x[i], vnc);
+            cfmac(es[j], x[i], vnr[i]);
         }
     }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) quad += 2 * (vnr[i].x * rs[i].x + vnr[i].y * rs[i].y);
+    const bool b4 = (lane & 16) != 0;
+    rowsum = cadd(b4 ? rs[1] : rs[0], shfl_xor(b4 ? rs[0] : rs[1], 16));
+    rowsum = cadd(rowsum, shfl_xor(rowsum, 8));
+    const bool b2 = (lane & 4) != 0, b1 = (lane & 2) != 0;
+    C y[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) y[j] = cadd(b2 ? es[j + 2] : es[j], shfl_xor(b2 ? es[j] : es[j + 2], 4));
+    colsum = cadd(b1 ? y[1] : y[0], shfl_xor(b1 ? y[0] : y[1], 2));
+    colsum = cadd(colsum, shfl_xor(colsum, 1));
+}
+
+// The pass over all tiles of the leading m x m block, dealt to the CTA's warps.  PARTS: tile
+// t's sums go to its own slots part[32 t ..] (16 rows, then 16 columns; hetrd_sum adds them up),
+// else into pn by shared-memory atomics.  Returns this lane's share of vn^H A' vn.
+template <int NT, bool PARTS, bool UPD, class C, class R, class S>
+__device__ __forceinline__ R hetrd_pass(S st, int m, const C* __restrict__ v, const C* __restrict__ w,
+                                        const C* __restrict__ vn, C* pn) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lr = lane & 7, lc = lane >> 3;
+    const int nb = (m + 15) / 16, nt = nb * (nb + 1) / 2;
+    R quad = 0;
+    for (int t = warp; t < nt; t += NT / 32) {
+        // t-th tile (row block rb <= column block cb), column blocks in turn
+        int cb = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
+        if ((cb + 1) * (cb + 2) / 2 <= t) ++cb;
+        else if (cb * (cb + 1) / 2 > t) --cb;
+        const int rb = t - cb * (cb + 1) / 2, r0 = 16 * rb, c0 = 16 * cb;
+        C rowsum, colsum;
+        if (rb < cb && c0 + 16 <= m) hetrd_tile<true, UPD, C, R>(st, m, r0, c0, v, w, vn, rowsum, colsum, quad);
+        else hetrd_tile<false, UPD, C, R>(st, m, r0, c0, v, w, vn, rowsum, colsum, quad);
+        if (PARTS) {
+            if (!(lane & 8)) pn[32 * t + lr + 8 * (lane >> 4)] = rowsum;
+            if (!(lane & 1)) pn[32 * t + 16 + lc + 4 * (lr >> 1)] = colsum;
+        } else {
+            const int r = r0 + lr + 8 * (lane >> 4), c = c0 + lc + 4 * (lr >> 1);
+            if (!(lane & 8) && r < m) smem_atomic_add(&pn[r], rowsum);
+            if (!(lane & 1) && c < m) smem_atomic_add(&pn[c], colsum);
+        }
+    }
+    return quad;
+}
+// (A' vn)[r] of the leading m x m block from the tiles' parts.
+template <class C>
+__device__ __forceinline__ C hetrd_sum(const C* __restrict__ part, int m, int r) {
+    const int nb = (m + 15) / 16, b = r >> 4, o = r & 15;
+    C s = cz<C>();
+    for (int cb = b; cb < nb; ++cb) s = cadd(s, part[32 * (cb * (cb + 1) / 2 + b) + o]);
+    for (int rb = 0; rb <= b; ++rb) s = cadd(s, part[32 * (b * (b + 1) / 2 + rb) + 16 + o]);
+    return s;
 }
 
 // Householder reflector of zlarfg for (alpha, x) with ||x||^2 = xnorm2: returns beta, tau
@@ -219,152 +237,128 @@ __device__ __forceinline__ void reflector(const C alpha, R xnorm2, R& beta, C& t
 // 1 and not stored), D/E the tridiagonal (double) and TAU the reflector scalars.  The
 // leading block moves into shared memory once its packed upper triangle fits in
 // `tri_cap` elements.
-template <int NT, class R>
-__global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 4)
+// Three barriers per column: w of the last reflector, the next column brought up to date and
+// its norm; the new reflector; the pass.  x^H v in w = x - tau/2 (x^H v) v is tau v^H A v, which
+// the pass sums on the way.  Small blocks (PARTS, m <= HT_PARTS_MAX) keep the pass's sums per
+// tile, so that it needs neither atomics nor a cleared accumulator.
+// Bound: instruction issue (several CTAs per SM hide the chains of the reflector).  With one
+// row and 16 columns per lane, shared double atomics and eight barriers per column 4,624 matrices
+// of order 64 took 4.03 ms, 2,304 of order 32 0.69 ms and 128 of order 129 0.93 ms; now 1.99,
+// 0.29 and 0.52.
+static constexpr int HT_PARTS_MAX = 144;
+__host__ __device__ constexpr int hetrd_pad(int m) { return (m + 15) / 16 * 16; }
+__host__ __device__ constexpr int hetrd_pn(int m) {   // elements of pn
+    return m <= HT_PARTS_MAX ? 16 * (hetrd_pad(m) / 16) * (hetrd_pad(m) / 16 + 1) : hetrd_pad(m);
+}
+template <int NT, class R, bool PARTS>
+__global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 512 / NT)
 k_hetrd(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, double* __restrict__ E,
         typename Cx<R>::T* __restrict__ TAU, int n, int m, int tri_cap) {
     typedef typename Cx<R>::T C;
+    constexpr int NW = NT / 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    C* v = reinterpret_cast<C*>(smem_raw);   // [m] current reflector
-    C* w = v + m;                             // [m] its w vector
-    C* vn = w + m;                            // [m] next reflector / column buffer
-    C* pn = vn + m;                           // [m] A' vn accumulator
-    R* red = reinterpret_cast<R*>(pn + m);    // [2*warps]
-    C* tri = reinterpret_cast<C*>(red + 2 * (NT / 32));   // packed triangle
-    const int tid = threadIdx.x;
+    const int mp = hetrd_pad(m);
+    C* v = reinterpret_cast<C*>(smem_raw);   // [mp] reflector of step i
+    C* vn = v + mp;                           // [mp] the next one / column buffer
+    C* w = vn + mp;                           // [mp] w of step i
+    C* pn = w + mp;                           // [hetrd_pn(m)] A' v
+    C* alpha = pn + hetrd_pn(m);              // [1]
+    R* normp = reinterpret_cast<R*>(alpha + 1);   // [NW] parts of the column's norm
+    R* quadp = normp + NW;                    // [NW] parts of v^H A' v
+    C* tri = reinterpret_cast<C*>(smem_raw) + ((3 * mp + hetrd_pn(m) + 1) + (2 * NW * (int)sizeof(R) + (int)sizeof(C) - 1) / (int)sizeof(C));
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const size_t mat = blockIdx.x;
     GlobalStore<C> gs{A + mat * (size_t)n * n, n};
     SharedStore<C> ss{tri};
     double* dd = D + mat * n;
     double* ee = E + mat * n;
     C* tt = TAU + mat * n;
-    if (m == 1) {
-        if (tid == 0) {
-            dd[0] = gs.at(0, 0)->x;
-            if (m == n) {
-                ee[0] = 0.0;
-                tt[0] = cz<C>();
-            }
-        }
-        return;
+    for (int r = tid; r < 3 * mp + hetrd_pn(m); r += NT) v[r] = cz<C>();
+    if (lane == 0) quadp[warp] = 0;
+    if (tid == 0 && m == n) {
+        ee[n - 1] = 0.0;
+        tt[n - 1] = cz<C>();
     }
+    __syncthreads();
     bool resident = false;
-    // -- prologue: reflector of step m-2 from column m-1, then p = A v over [0..m-2]^2
-    {
-        const int i = m - 2;
-        R part = 0;
-        for (int r = tid; r <= i + 1; r += NT) {
-            const C x = *gs.at(r, i + 1);
-            vn[r] = x;
-            if (r < i) part += cabs2(x);
-        }
-        const R xn2 = block_sum<NT>(part, red);
-        R beta;
-        C tau, scal;
-        reflector(vn[i], xn2, beta, tau, scal);
-        const bool act = !(tau.x == 0 && tau.y == 0);
-        __syncthreads();
-        for (int r = tid; r < i; r += NT) {
-            const C x = act ? cmul(scal, vn[r]) : vn[r];
-            v[r] = x;
-            *gs.at(r, i + 1) = x;
-        }
-        for (int r = tid; r < m; r += NT) {
-            w[r] = cz<C>();
-            pn[r] = cz<C>();
-        }
-        if (tid == 0) {
-            v[i] = cm<C>(1, 0);
-            dd[m - 1] = vn[m - 1].x;
-            *gs.at(i, i + 1) = cm<C>(beta, 0);
-            ee[i] = beta;
-            tt[i] = tau;
-        }
-        __syncthreads();
-        fused_pass<NT>(gs, i + 1, v, w, false, v, act, pn);
-        __syncthreads();
-        C dpart = cz<C>();
-        for (int r = tid; r <= i; r += NT) {
-            const C x = cmul(tau, pn[r]);
-            pn[r] = x;
-            cfmac(dpart, x, v[r]);
-        }
-        const C xv = block_sum_c<NT>(dpart, red);
-        const C al = cscale(cmul(tau, xv), (R)-0.5);
-        for (int r = tid; r <= i; r += NT) w[r] = cadd(pn[r], cmul(al, v[r]));
-        __syncthreads();
-    }
-    // -- main loop: v, w belong to step i (column i+1 done); finish column i, build the
-    //    reflector of step i-1 from it, then one fused pass over [0..i-1]^2
-    for (int i = m - 2; i >= 1; --i) {
+    C tau = cz<C>();
+    bool act = false;
+    // column i: rows 0..i of the leading block; step i's reflector (v) came from column i + 1
+    for (int i = m - 1; i >= 0; --i) {
         if (!resident && (i + 1) * (i + 2) / 2 <= tri_cap) {
             // move the leading (i+1)x(i+1) upper triangle into shared memory
-            for (int c = 0; c <= i; ++c)
-                for (int r = tid; r <= c; r += NT) *ss.at(r, c) = *gs.at(r, c);
+            for (int c = warp; c <= i; c += NW)
+                for (int r = lane; r <= c; r += 32) *ss.at(r, c) = *gs.at(r, c);
             resident = true;
             __syncthreads();
         }
-        // (1) updated column i, rows 0..i
+        // (1) w of step i, and column i brought up to date with it
+        R q2 = 0;
+#pragma unroll
+        for (int k = 0; k < NW; ++k) q2 += quadp[k];
+        const R al = (R)-0.5 * cabs2(tau) * q2;   // x^H v = conj(tau) v^H A v, al = -tau/2 x^H v
+        C wi = cmul(tau, PARTS ? hetrd_sum(pn, i + 1, i) : pn[i]);
+        wi.x += al;                               // (v[i] = 1)
+        if (!act) wi = cz<C>();
         R part = 0;
-        const C wi = w[i], vi = v[i];
         for (int r = tid; r <= i; r += NT) {
-            C x = resident ? *ss.at(r, i) : *gs.at(r, i);
-            C u = cmul(v[r], cconj(wi));
-            cfma(u, w[r], cconj(vi));
-            x = csub(x, u);
+            C wr = cz<C>(), x = resident ? *ss.at(r, i) : *gs.at(r, i);
+            if (act) {
+                const C vr = v[r];
+                wr = cmul(tau, PARTS ? hetrd_sum(pn, i + 1, r) : pn[r]);
+                wr.x += al * vr.x;
+                wr.y += al * vr.y;
+                C u = cmul(vr, cconj(wi));
+                x = csub(x, cadd(u, wr));
+            }
+            w[r] = wr;
             vn[r] = x;
             if (r < i - 1) part += cabs2(x);
-            pn[r] = cz<C>();
+            if (r == i - 1) *alpha = x;
+            if (r == i) dd[i] = x.x;
         }
-        const R xn2 = block_sum<NT>(part, red);
-        // (2) reflector of step i-1: alpha = A'[i-1][i], x = A'[0..i-2][i]
-        R beta;
-        C tau, scal;
-        reflector(vn[i - 1], xn2, beta, tau, scal);
-        const bool act = !(tau.x == 0 && tau.y == 0);
+        if (i == 0) break;
+        part = warp_sum(part);
+        if (lane == 0) normp[warp] = part;
         __syncthreads();
-        if (tid == 0) dd[i] = vn[i].x;
-        for (int r = tid; r < i - 1; r += NT) {
-            const C x = act ? cmul(scal, vn[r]) : vn[r];
-            vn[r] = x;
-            *gs.at(r, i) = x;   // reflector storage stays in global memory
+        // (2) reflector of step i-1: alpha = A'[i-1][i], x = A'[0..i-2][i]
+        R xn2 = 0, beta;
+#pragma unroll
+        for (int k = 0; k < NW; ++k) xn2 += normp[k];
+        C scal;
+        const bool upd = act;
+        reflector(*alpha, xn2, beta, tau, scal);
+        act = !(tau.x == 0 && tau.y == 0);
+        for (int r = tid; r < i; r += NT) {
+            if (!PARTS) pn[r] = cz<C>();
+            if (r == i - 1) {
+                vn[r] = cm<C>(1, 0);
+                *gs.at(r, i) = cm<C>(beta, 0);
+            } else {
+                const C x = act ? cmul(scal, vn[r]) : vn[r];
+                vn[r] = x;
+                *gs.at(r, i) = x;   // reflector storage stays in global memory
+            }
         }
         if (tid == 0) {
-            vn[i - 1] = cm<C>(1, 0);
-            *gs.at(i - 1, i) = cm<C>(beta, 0);
             ee[i - 1] = beta;
             tt[i - 1] = tau;
         }
         __syncthreads();
-        // (3) fused pass: update [0..i-1]^2 with (v, w), accumulate pn = A' vn
-        if (resident) fused_pass<NT>(ss, i, v, w, true, vn, act, pn);
-        else fused_pass<NT>(gs, i, v, w, true, vn, act, pn);
+        // (3) update [0..i-1]^2 with (v, w), accumulate pn = A' vn
+        R quad;
+        if (upd)
+            quad = resident ? hetrd_pass<NT, PARTS, true, C, R>(ss, i, v, w, vn, pn)
+                            : hetrd_pass<NT, PARTS, true, C, R>(gs, i, v, w, vn, pn);
+        else
+            quad = resident ? hetrd_pass<NT, PARTS, false, C, R>(ss, i, v, w, vn, pn)
+                            : hetrd_pass<NT, PARTS, false, C, R>(gs, i, v, w, vn, pn);
+        quad = warp_sum(quad);
+        if (lane == 0) quadp[warp] = quad;
         __syncthreads();
-        // (4) w' = tau pn - tau/2 (x^H vn) vn; v <- vn
-        C dpart = cz<C>();
-        for (int r = tid; r < i; r += NT) {
-            const C x = cmul(tau, pn[r]);
-            pn[r] = x;
-            cfmac(dpart, x, vn[r]);
-        }
-        const C xv = block_sum_c<NT>(dpart, red);
-        const C al = cscale(cmul(tau, xv), (R)-0.5);
-        for (int r = tid; r < i; r += NT) {
-            w[r] = act ? cadd(pn[r], cmul(al, vn[r])) : cz<C>();
-            v[r] = vn[r];
-        }
-        __syncthreads();
-    }
-    // -- step 0's update reaches only A[0][0]
-    if (tid == 0) {
-        C x = resident ? *ss.at(0, 0) : *gs.at(0, 0);
-        C u = cmul(v[0], cconj(w[0]));
-        cfma(u, w[0], cconj(v[0]));
-        dd[0] = x.x - u.x;
-        if (m == n) {
-            ee[n - 1] = 0.0;
-            tt[n - 1] = cz<C>();
-        }
+        C* t = v;
+        v = vn;
+        vn = t;
     }
 }
 
@@ -2679,40 +2673,43 @@ __global__ void k_to_single(const cplx* __restrict__ A, cplxf* __restrict__ B, s
         B[i] = from_c64<cplxf>(A[i]);
 }
 
-// Launch shape of k_hetrd: small matrices keep their whole triangle in shared memory with
-// 128 threads and several CTAs per SM; larger ones run 512 threads, one CTA per SM, with
-// as much of the leading triangle resident as ~220 KB allows.
+// Launch shape of k_hetrd: NT threads, as much of the leading triangle resident as fits (all
+// of it up to order ~155 in double precision).  Threads: the tiles of a pass are few (10 at
+// order 64), so 64 threads up to order 48 and 128 up to 100 with several CTAs per SM, 512 above
+// (one CTA per SM); chunks of fewer matrices than SMs take 512 from order 65 on and 256 below.
 struct HetrdCfg {
     int nt;
     int tri_cap;
     size_t smem;
 };
 template <class R>
-static HetrdCfg hetrd_config(int n) {
+static HetrdCfg hetrd_config(int m, int nb) {
     const size_t ce = 2 * sizeof(R);   // complex element
-    const size_t tri_full = (size_t)n * (n + 1) / 2;
-    const size_t vec128 = 4 * (size_t)n * ce + 2 * (128 / 32) * sizeof(R);
-    if (vec128 + tri_full * ce <= 110 * 1024) return {128, (int)tri_full, vec128 + tri_full * ce};
-    const size_t vec512 = 4 * (size_t)n * ce + 2 * (512 / 32) * sizeof(R);
+    const int nt = nb <= 148 ? (m > 64 ? 512 : 256) : m <= 48 ? 64 : m <= 100 ? 128 : 512;
+    const size_t vec = (3 * (size_t)hetrd_pad(m) + hetrd_pn(m) + 2) * ce + 2 * (nt / 32) * sizeof(R);
     const size_t budget = 220 * 1024;
-    size_t cap = budget > vec512 ? (budget - vec512) / ce : 0;
-    cap = std::min(cap, tri_full);
-    return {512, (int)cap, vec512 + cap * ce};
+    size_t cap = budget > vec ? (budget - vec) / ce : 0;
+    cap = std::min(cap, (size_t)m * (m + 1) / 2);
+    return {nt, (int)cap, vec + cap * ce};
+}
+template <int NT, class R, bool PARTS>
+static cudaError_t launch_hetrd_t(const HetrdCfg& c, cudaStream_t st, int nb, typename Cx<R>::T* A, double* D,
+                                  double* E, typename Cx<R>::T* TAU, int n, int m) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_hetrd<NT, R, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem);
+    if (e != cudaSuccess) return e;
+    k_hetrd<NT, R, PARTS><<<nb, NT, c.smem, st>>>(A, D, E, TAU, n, m, c.tri_cap);
+    return cudaGetLastError();
 }
 template <class R>
-static cudaError_t launch_hetrd(const HetrdCfg& c, cudaStream_t st, int nb, typename Cx<R>::T* A, double* D,
-                                double* E, typename Cx<R>::T* TAU, int n, int m) {
+static cudaError_t launch_hetrd(cudaStream_t st, int nb, typename Cx<R>::T* A, double* D, double* E,
+                                typename Cx<R>::T* TAU, int n, int m) {
+    const HetrdCfg c = hetrd_config<R>(m, nb);
     if (c.smem > 227 * 1024) return cudaErrorInvalidValue;
-    if (c.nt == 128) {
-        cudaError_t e = cudaFuncSetAttribute(k_hetrd<128, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem);
-        if (e != cudaSuccess) return e;
-        k_hetrd<128, R><<<nb, 128, c.smem, st>>>(A, D, E, TAU, n, m, c.tri_cap);
-    } else {
-        cudaError_t e = cudaFuncSetAttribute(k_hetrd<512, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem);
-        if (e != cudaSuccess) return e;
-        k_hetrd<512, R><<<nb, 512, c.smem, st>>>(A, D, E, TAU, n, m, c.tri_cap);
-    }
-    return cudaGetLastError();
+    if (m > HT_PARTS_MAX) return launch_hetrd_t<512, R, false>(c, st, nb, A, D, E, TAU, n, m);
+    const auto launch = c.nt == 64 ? launch_hetrd_t<64, R, true> : c.nt == 128 ? launch_hetrd_t<128, R, true>
+                      : c.nt == 256 ? launch_hetrd_t<256, R, true> : launch_hetrd_t<512, R, true>;
+    return launch(c, st, nb, A, D, E, TAU, n, m);
 }
 
 // Launch choices of one eigensolve configuration that the autotuner may set (0 / -1: the
@@ -2743,7 +2740,6 @@ struct HeevPlan {
     int refine_steps;    // mixed mode: 1 or 2
     bool rq;             // mixed mode, one step: then the eigenvalues as Rayleigh quotients (H kept until then)
     int band;            // >= 0: every matrix is a cyclic band of this half-bandwidth (rlm), else -1
-    HetrdCfg hc;
     size_t smem_tri;
     bool small_bt;       // k_ormtr (register-resident Z chunk) or the blocked GEMM path
     int ch, dbuf;
@@ -2783,7 +2779,6 @@ static HeevPlan heev_plan(int n, bool mixed, int refine_steps = 2, int band = -1
     const bool blocked = tune.blocked < 0 ? n >= HT_BLOCKED_MIN : (tune.blocked > 0 && n > HT_TAIL + p.pw);
     p.npanels = blocked ? (n - HT_TAIL + p.pw - 1) / p.pw : 0;
     p.m_tail = n - p.npanels * p.pw;
-    p.hc = mixed ? hetrd_config<float>(p.m_tail) : hetrd_config<double>(p.m_tail);
     p.smem_tri = 4 * (size_t)n * sizeof(double) + n * sizeof(int);
     p.nblk16 = (n - 1 + ORM_NB - 1) / ORM_NB;
     p.bt_nb = tune.bt_nb ? tune.bt_nb : n >= BT128_MIN ? 2 * BT_NB : BT_NB;
@@ -2945,7 +2940,7 @@ static int tridiagonalise(rlmb_context* ctx, cudaStream_t st, const HeevPlan& p,
         }
     }
     RLMB_CHUNK_PROF("k_hetrd");
-    if (launch_hetrd<R>(p.hc, st, nb, A, D, E, TAU, n, m) != cudaSuccess) return RLMB_ERR_CUDA;
+    if (launch_hetrd<R>(st, nb, A, D, E, TAU, n, m) != cudaSuccess) return RLMB_ERR_CUDA;
     RLMB_CHUNK_LAUNCHED();
     return RLMB_OK;
 }
@@ -3217,7 +3212,7 @@ static int heev_chunk(rlmb_context* ctx, cudaStream_t st, const HeevPlan& p, cpl
         RLMB_CHUNK_LAUNCHED();
         return RLMB_OK;
     }
-    if (p.hc.smem > 227 * 1024 || p.smem_tri > 227 * 1024) return RLMB_ERR_ARG;
+    if (p.smem_tri > 227 * 1024) return RLMB_ERR_ARG;
     if (cudaFuncSetAttribute(k_tridiag<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem_tri) != cudaSuccess ||
         cudaFuncSetAttribute(k_tridiag<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem_tri) != cudaSuccess)
         return RLMB_ERR_CUDA;
