@@ -99,6 +99,45 @@ static int hlm_tables(rlmb_context* ctx, int lx, int ly, int Q, int band, int g,
     return RLMB_OK;
 }
 
+// Coefficient tables of an rlm mesh geometry on the device (coeff_mn, coeff_m_theta, coeff_jm,
+// disorder independent), cached in the context like the hlm ones: the host's sines and cosines
+// take 17 ms at n_phi = 3000.  Synchronises the stream when it builds them.
+static int rlm_tables(rlmb_context* ctx, int n_phi, int o, int g, double L1, double L2, cplx** cmn, cplx** cmt,
+                      cplx** cjm) {
+    const int dim = 2 * o + 1;
+    const size_t n1 = (size_t)dim * dim, n2 = (size_t)(g + 1) * dim, n3 = (size_t)n_phi * dim;
+    const double key[5] = {(double)n_phi, (double)o, (double)g, L1, L2};
+    if (!ctx->rlm_tables || std::memcmp(key, ctx->rlm_key, sizeof(key)) != 0) {
+        if (ctx->frozen) return RLMB_ERR_ALLOC;
+        std::vector<double> h(2 * (n1 + n2 + n3));
+        if (int rc = rlmb_rlm_coeff_tables(n_phi, o, dim, g, L1, L2, h.data(), h.data() + 2 * n1,
+                                           h.data() + 2 * (n1 + n2)))
+            return rc;
+        if (ctx->rlm_tables) {
+            RLMB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+            RLMB_CUDA_TRY(cudaFree(ctx->rlm_tables));
+            ctx->rlm_tables = nullptr;
+        }
+        if (cudaMalloc(&ctx->rlm_tables, h.size() * sizeof(double)) != cudaSuccess) {
+            cudaGetLastError();
+            ctx->rlm_tables = nullptr;
+            return RLMB_ERR_ALLOC;
+        }
+        if (cudaMemcpyAsync(ctx->rlm_tables, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream) !=
+                cudaSuccess ||
+            cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+            cudaFree(ctx->rlm_tables);
+            ctx->rlm_tables = nullptr;
+            return RLMB_ERR_CUDA;
+        }
+        std::memcpy(ctx->rlm_key, key, sizeof(key));
+    }
+    *cmn = static_cast<cplx*>(ctx->rlm_tables);
+    *cmt = *cmn + n1;
+    *cjm = *cmt + n2;
+    return RLMB_OK;
+}
+
 // Eigensolve failures of a pipeline call are tallied on the device (no host round trip per
 // batch) and read once, when the call ends.
 __global__ void k_count_nonzero(const int* __restrict__ info, int count, int* __restrict__ fail) {
@@ -124,12 +163,17 @@ static int tally_failures(rlmb_context* ctx, const int* d_info, int count) {
     RLMB_LAUNCHED(ctx);
     return RLMB_OK;
 }
+// Small host-bound results travel through the context's pinned buffer (a copy into pageable
+// memory would block on the spot): the failure count in its first 256 bytes, results after it.
+static constexpr size_t PINNED_HEAD = 256;
+static constexpr size_t PINNED_RESULTS_MAX = (size_t)64 << 20;
 // Synchronises the context stream and returns the call's status: the failure count, if any.
 static int finish_call(rlmb_context* ctx) {
-    int h = 0;
-    RLMB_CUDA_TRY(cudaMemcpyAsync(&h, ctx->fail, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    if (int rc = ensure_pinned(ctx, PINNED_HEAD)) return rc;
+    int* h = static_cast<int*>(ctx->pinned);
+    RLMB_CUDA_TRY(cudaMemcpyAsync(h, ctx->fail, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     RLMB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    return h > 0 ? h : RLMB_OK;
+    return *h > 0 ? *h : RLMB_OK;
 }
 
 static bool hlm_args_ok(int lx, int ly, int Q, int band, int g) {
@@ -140,14 +184,14 @@ static bool hlm_args_ok(int lx, int ly, int Q, int band, int g) {
 // Device memory budget for one batch of mesh data: a third of the free memory, counting the
 // context's own pipeline buffer (reused by the batch) as free so that repeated calls batch
 // alike, at most 40 GB.
+static constexpr size_t MESH_BUDGET_MAX = (size_t)40 << 30;
 static size_t mesh_budget_bytes(const rlmb_context* ctx) {
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
         cudaGetLastError();
         return (size_t)8 << 30;
     }
-    const size_t cap = (size_t)40 << 30;
-    return std::min(cap, (free_b + ctx->pipe_bytes) / 3);
+    return std::min(MESH_BUDGET_MAX, (free_b + ctx->pipe_bytes) / 3);
 }
 
 // Samples per batch: at most `fit`, and the batches of one call equal in size (a short last
@@ -197,6 +241,7 @@ int rlmb_destroy(rlmb_context* ctx) {
     if (ctx->fail) cudaFree(ctx->fail);
     if (ctx->mt_state) cudaFree(ctx->mt_state);
     if (ctx->hlm_tables) cudaFree(ctx->hlm_tables);
+    if (ctx->rlm_tables) cudaFree(ctx->rlm_tables);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
     delete ctx;
     return RLMB_OK;
@@ -354,7 +399,7 @@ int rlmb_hlm_project(rlmb_context* ctx, int lx, int ly, int Q, int band, int n_m
     RLMB_CUDA_TRY(cudaMemcpyAsync(d_t, tl.data(), count * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     RLMB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));   // tl is a host temporary
     if (int rc = launch_hlm_vtilde(ctx, d_potential, lx, ly, Q, 1, vt)) return rc;
-    return launch_hlm_project(ctx, hb, vt, d_t, lx, ly, Q, count, 1, reinterpret_cast<cplx*>(d_h));
+    return launch_hlm_project(ctx, hb, vt, d_t, n_mesh, lx, ly, Q, count, 1, reinterpret_cast<cplx*>(d_h));
 }
 
 int rlmb_fhs_line(rlmb_context* ctx, const double* d_prev, const double* d_cur, int n_phi,
@@ -443,18 +488,18 @@ int rlmb_rlm_mesh_export(rlmb_context* ctx, int n_phi, double qc, double ic, int
 }
 
 // One prepared rlm pipeline geometry: sizes, the batch of samples, and the regions of the
-// context's pipeline buffer (coefficient tables and theta lists uploaded once).
+// context's pipeline buffer, and its cached coefficient tables.
 struct RlmPlan {
     int n_phi, nimp, o, dim, g, kpts, nb, n_samples;
     double L1, L2;
     unsigned long seed;
     cplx *d_cmn, *d_cmt, *d_cjm, *d_vmn, *d_H, *d_U;
     double *d_imp, *d_W, *d_out;
-    int *d_t, *d_info;
+    int* d_info;
 };
 
 // Sizes (with the reference's C truncations, rlm/main_rlm_cpu.cpp:29-33), buffers and the
-// disorder-independent tables of an rlm mesh call; synchronises the context stream.
+// disorder-independent tables of an rlm mesh call.
 static int rlm_prepare(rlmb_context* ctx, int n_phi, double qc, double ic, int n_mesh, unsigned long seed,
                        int n_samples, RlmPlan* p) {
     const double L1 = std::sqrt(n_phi * qc), L2 = std::sqrt(n_phi * qc);
@@ -464,25 +509,23 @@ static int rlm_prepare(rlmb_context* ctx, int n_phi, double qc, double ic, int n
     const int nimp = (int)nimp_l, o = (int)o_l, dim = 2 * o + 1;
     const int g = n_mesh, kpts = (g + 1) * (g + 1);
     const size_t nn = (size_t)n_phi * n_phi;
-    std::vector<double> cmn(2 * (size_t)dim * dim), cmt(2 * (size_t)(g + 1) * dim), cjm(2 * (size_t)n_phi * dim);
-    if (int rc = rlmb_rlm_coeff_tables(n_phi, o, dim, g, L1, L2, cmn.data(), cmt.data(), cjm.data())) return rc;
-    // batch of samples that fits the budget
+    // batch of samples that fits the budget: all of them, without asking for the free memory,
+    // where the pipeline buffer holds them already
     const size_t per_sample = kpts * (nn * sizeof(cplx) + (size_t)n_phi * (sizeof(double) + 2 * sizeof(cplx))) +
                               (size_t)dim * dim * sizeof(cplx) + 3 * (size_t)nimp * sizeof(double);
-    const int nb = balanced_batch(n_samples, mesh_budget_bytes(ctx) / per_sample);
-    size_t bytes = 0;
-    need<cplx>(bytes, cmn.size() / 2);
-    need<cplx>(bytes, cmt.size() / 2);
-    need<cplx>(bytes, cjm.size() / 2);
-    need<double>(bytes, 3 * (size_t)nimp * nb);
-    need<cplx>(bytes, (size_t)dim * dim * nb);
-    need<int>(bytes, 2 * (size_t)kpts * nb);
-    need<cplx>(bytes, nn * kpts * nb);
-    need<double>(bytes, (size_t)n_phi * kpts * nb);
-    need<cplx>(bytes, 2 * (size_t)n_phi * kpts * nb);
-    need<double>(bytes, 2 * (size_t)n_phi * nb);
-    need<int>(bytes, (size_t)kpts * nb);
-    if (int rc = ensure_pipe(ctx, bytes)) return rc;
+    auto pipe_bytes = [&](size_t nb) {
+        size_t bytes = 0;
+        need<double>(bytes, 3 * (size_t)nimp * nb);
+        need<cplx>(bytes, (size_t)dim * dim * nb);
+        need<cplx>(bytes, nn * kpts * nb);
+        need<double>(bytes, (size_t)n_phi * kpts * nb);
+        need<cplx>(bytes, 2 * (size_t)n_phi * kpts * nb);
+        need<double>(bytes, 2 * (size_t)n_phi * nb);
+        return need<int>(bytes, (size_t)kpts * nb);
+    };
+    const bool held = n_samples * per_sample <= MESH_BUDGET_MAX && pipe_bytes(n_samples) <= ctx->pipe_bytes;
+    const int nb = held ? n_samples : balanced_batch(n_samples, mesh_budget_bytes(ctx) / per_sample);
+    if (int rc = ensure_pipe(ctx, pipe_bytes(nb))) return rc;
     Carver cv(ctx->pipe);
     *p = RlmPlan{};
     p->n_phi = n_phi;
@@ -496,45 +539,28 @@ static int rlm_prepare(rlmb_context* ctx, int n_phi, double qc, double ic, int n
     p->L1 = L1;
     p->L2 = L2;
     p->seed = seed;
-    p->d_cmn = cv.take<cplx>(cmn.size() / 2);
-    p->d_cmt = cv.take<cplx>(cmt.size() / 2);
-    p->d_cjm = cv.take<cplx>(cjm.size() / 2);
     p->d_imp = cv.take<double>(3 * (size_t)nimp * nb);
     p->d_vmn = cv.take<cplx>((size_t)dim * dim * nb);
-    p->d_t = cv.take<int>(2 * (size_t)kpts * nb);
     p->d_H = cv.take<cplx>(nn * kpts * nb);
     p->d_W = cv.take<double>((size_t)n_phi * kpts * nb);
     p->d_U = cv.take<cplx>(2 * (size_t)n_phi * kpts * nb);
     p->d_out = cv.take<double>(2 * (size_t)n_phi * nb);
     p->d_info = cv.take<int>((size_t)kpts * nb);
-    if (int rc = ensure_pinned(ctx, 2 * (size_t)kpts * nb * sizeof(int))) return rc;
     // (the V_mn partial sums and the assembly's theta_2 slabs, in turn)
     if (int rc = ensure_workspace(ctx, std::max(rlm_potential_ws_elems(nimp, nb, dim),
                                                 rlm_assemble_ws_elems(n_phi, dim, nb, g + 1)) * sizeof(cplx)))
         return rc;
-    RLMB_CUDA_TRY(cudaMemcpyAsync(p->d_cmn, cmn.data(), cmn.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    RLMB_CUDA_TRY(cudaMemcpyAsync(p->d_cmt, cmt.data(), cmt.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    RLMB_CUDA_TRY(cudaMemcpyAsync(p->d_cjm, cjm.data(), cjm.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    int* pt = static_cast<int*>(ctx->pinned);
-    for (int s = 0; s < nb; ++s)
-        for (int t = 0; t < kpts; ++t) {
-            pt[s * kpts + t] = t / (g + 1);
-            pt[(size_t)nb * kpts + s * kpts + t] = t % (g + 1);
-        }
-    RLMB_CUDA_TRY(cudaMemcpyAsync(p->d_t, pt, 2 * (size_t)kpts * nb * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
-    // the host tables are call-local and the pinned staging is reused by the next call: both
-    // copies must have completed before this function returns
-    RLMB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    return RLMB_OK;
+    return rlm_tables(ctx, n_phi, o, g, L1, L2, &p->d_cmn, &p->d_cmt, &p->d_cjm);
 }
 
 // The stream-ordered work of an rlm mesh call on a prepared plan: samples sample0 ..
 // sample0 + n_samples - 1 (plus *d_sample0 when given: the first sample index is then read
 // from device memory, for a captured graph), energies / chern n_samples * n_phi values each,
-// in device memory if dev_out, else in host memory.  No host round trips: eigensolve
-// failures are tallied on the device.
+// in device memory if dev_out, else in host memory: in `staged` (pinned; per batch its energies,
+// then its Chern numbers) if given.  No host round trips: eigensolve failures are tallied on
+// the device.
 static int rlm_enqueue(rlmb_context* ctx, const RlmPlan& p, int sample0, const int* d_sample0, double* energies,
-                       double* chern, bool dev_out, const char* wfs_dir) {
+                       double* chern, bool dev_out, const char* wfs_dir, double* staged) {
     const int n_phi = p.n_phi, nimp = p.nimp, nb = p.nb, kpts = p.kpts, g = p.g, dim = p.dim, o = p.o;
     std::vector<int> all_t2(g + 1);
     for (int t = 0; t <= g; ++t) all_t2[t] = t;
@@ -553,7 +579,7 @@ static int rlm_enqueue(rlmb_context* ctx, const RlmPlan& p, int sample0, const i
         if (int rc = launch_rlm_potential(ctx, dx, dy, ds, nimp, cnt, p.d_cmn, dim, o, static_cast<cplx*>(ctx->ws),
                                           p.d_vmn))
             return rc;
-        if (int rc = launch_rlm_assemble(ctx, p.d_vmn, p.d_cmt, p.d_cjm, p.d_t, p.d_t + (size_t)nb * kpts, cnt * kpts,
+        if (int rc = launch_rlm_assemble(ctx, p.d_vmn, p.d_cmt, p.d_cjm, nullptr, nullptr, cnt * kpts,
                                          kpts, n_phi, dim, o, all_t2.data(), g + 1, static_cast<cplx*>(ctx->ws), p.d_H))
             return rc;
         if (int rc = heevd_batched_band(ctx, reinterpret_cast<double*>(p.d_H), p.d_W, n_phi, cnt * kpts, p.d_info, o))
@@ -568,10 +594,16 @@ static int rlm_enqueue(rlmb_context* ctx, const RlmPlan& p, int sample0, const i
         double* out_c = dev_out ? chern + (size_t)s0 * n_phi : p.d_out + (size_t)n_phi * nb;
         if (int rc = launch_plaquettes(ctx, d_U1, d_U2, p.d_W, n_phi, g, cnt, 0, out_e, out_c)) return rc;
         if (!dev_out) {
-            RLMB_CUDA_TRY(cudaMemcpyAsync(energies + (size_t)s0 * n_phi, p.d_out, (size_t)cnt * n_phi * sizeof(double),
-                                          cudaMemcpyDeviceToHost, ctx->stream));
-            RLMB_CUDA_TRY(cudaMemcpyAsync(chern + (size_t)s0 * n_phi, p.d_out + (size_t)n_phi * nb,
-                                          (size_t)cnt * n_phi * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+            // (to the pinned staging of the whole call, or straight to the caller's memory)
+            double* he = staged ? staged + 2 * (size_t)s0 * n_phi : energies + (size_t)s0 * n_phi;
+            double* hc = staged ? he + (size_t)cnt * n_phi : chern + (size_t)s0 * n_phi;
+            const size_t bytes = (size_t)cnt * n_phi * sizeof(double);
+            if (staged && cnt == nb) {
+                RLMB_CUDA_TRY(cudaMemcpyAsync(he, p.d_out, 2 * bytes, cudaMemcpyDeviceToHost, ctx->stream));
+            } else {
+                RLMB_CUDA_TRY(cudaMemcpyAsync(he, p.d_out, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+                RLMB_CUDA_TRY(cudaMemcpyAsync(hc, p.d_out + (size_t)n_phi * nb, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+            }
         }
     }
     return RLMB_OK;
@@ -591,8 +623,21 @@ static int rlm_mesh(rlmb_context* ctx, int n_phi, double qc, double ic, int n_me
     RlmPlan p;
     if (int rc = rlm_prepare(ctx, n_phi, qc, ic, n_mesh, seed, n_samples, &p)) return rc;
     if (int rc = reset_failures(ctx)) return rc;
-    if (int rc = rlm_enqueue(ctx, p, sample0, nullptr, energies, chern, dev_out, wfs_dir)) return rc;
-    return finish_call(ctx);
+    const size_t results = 2 * (size_t)n_phi * n_samples;
+    double* staged = nullptr;
+    if (!dev_out && !wfs_dir && results * sizeof(double) <= PINNED_RESULTS_MAX) {   // (an export uses the pinned buffer)
+        if (int rc = ensure_pinned(ctx, PINNED_HEAD + results * sizeof(double))) return rc;
+        staged = reinterpret_cast<double*>(static_cast<char*>(ctx->pinned) + PINNED_HEAD);
+    }
+    if (int rc = rlm_enqueue(ctx, p, sample0, nullptr, energies, chern, dev_out, wfs_dir, staged)) return rc;
+    const int rc = finish_call(ctx);
+    if (rc >= 0 && staged)
+        for (int s0 = 0; s0 < n_samples; s0 += p.nb) {
+            const size_t cnt = (size_t)std::min(p.nb, n_samples - s0) * n_phi, at = (size_t)s0 * n_phi;
+            std::memcpy(energies + at, staged + 2 * at, cnt * sizeof(double));
+            std::memcpy(chern + at, staged + 2 * at + cnt, cnt * sizeof(double));
+        }
+    return rc;
 }
 
 // ----------------------------------------------- rlm orders captured in one CUDA graph
@@ -699,7 +744,7 @@ int rlmb_rlm_fss_graph_create(int device, const int* n_phi, int count, double qc
         if ((rc = rlm_prepare(o.ctx, n_phi[i], qc, ic, n_mesh, seed, n_samples, &o.plan))) return fail(rc);
         if ((rc = reset_failures(o.ctx))) return fail(rc);
         if ((rc = rlm_enqueue(o.ctx, o.plan, 0, f->d_sample0, o.d_e, o.d_e + (size_t)n_samples * n_phi[i], true,
-                              nullptr)))
+                              nullptr, nullptr)))
             return fail(rc);
         if ((rc = finish_call(o.ctx)) < 0) return fail(rc);
     }
@@ -715,7 +760,7 @@ int rlmb_rlm_fss_graph_create(int device, const int* n_phi, int count, double qc
         o.ctx->frozen = 1;
         if (cudaMemsetAsync(o.ctx->fail, 0, sizeof(int), o.ctx->stream) != cudaSuccess) rc = RLMB_ERR_CUDA;
         if (rc == RLMB_OK)
-            rc = rlm_enqueue(o.ctx, o.plan, 0, f->d_sample0, o.d_e, o.d_e + (size_t)n_samples * n_phi[i], true, nullptr);
+            rc = rlm_enqueue(o.ctx, o.plan, 0, f->d_sample0, o.d_e, o.d_e + (size_t)n_samples * n_phi[i], true, nullptr, nullptr);
         o.ctx->frozen = 0;
         if (rc == RLMB_OK && (cudaEventRecord(o.done, o.ctx->stream) != cudaSuccess ||
                               cudaStreamWaitEvent(f->origin, o.done, 0) != cudaSuccess))
@@ -769,9 +814,9 @@ int rlmb_rlm_fss_graph_destroy(rlmb_fss_graph* f) {
 }
 
 // --------------------------------------------------------------------- hlm pipeline
-int rlmb_hlm_mesh_solve_device(rlmb_context* ctx, int lx, int ly, int Q, int band, int n_mesh,
-                               const double* d_potentials, int n_samples, double* d_energies,
-                               double* d_chern) {
+// The stream-ordered work of an hlm mesh call (set-up included).
+static int hlm_enqueue(rlmb_context* ctx, int lx, int ly, int Q, int band, int n_mesh, const double* d_potentials,
+                       int n_samples, double* d_energies, double* d_chern) {
     if (!ctx || !hlm_args_ok(lx, ly, Q, band, n_mesh) || n_samples < 0 ||
         (n_samples > 0 && (!d_potentials || !d_energies || !d_chern)))
         return RLMB_ERR_ARG;
@@ -784,17 +829,20 @@ int rlmb_hlm_mesh_solve_device(rlmb_context* ctx, int lx, int ly, int Q, int ban
     if (int rc = hlm_tables(ctx, lx, ly, Q, band, g, &hb)) return rc;
     const size_t per_sample = kpts * (nn * sizeof(cplx) + (size_t)N * (sizeof(double) + 2 * sizeof(cplx))) +
                               (size_t)ns * sizeof(cplx);
-    const int nb = balanced_batch(n_samples, mesh_budget_bytes(ctx) / per_sample);
-    size_t bytes = 0;
-    need<int>(bytes, kpts);
-    need<cplx>(bytes, (size_t)ns * nb);
-    need<cplx>(bytes, nn * kpts * nb);
-    need<double>(bytes, (size_t)N * kpts * nb);
-    need<cplx>(bytes, 2 * (size_t)N * kpts * nb);
-    need<int>(bytes, (size_t)kpts * nb);
-    if (int rc = ensure_pipe(ctx, bytes)) return rc;
+    auto pipe_bytes = [&](size_t nb) {
+        size_t bytes = 0;
+        need<cplx>(bytes, (size_t)ns * nb);
+        need<cplx>(bytes, nn * kpts * nb);
+        need<double>(bytes, (size_t)N * kpts * nb);
+        need<cplx>(bytes, (size_t)N * kpts * nb);
+        need<cplx>(bytes, (size_t)N * kpts * nb);
+        return need<int>(bytes, (size_t)kpts * nb);
+    };
+    // (the free memory is asked for only where the pipeline buffer does not hold all samples)
+    const bool held = n_samples * per_sample <= MESH_BUDGET_MAX && pipe_bytes(n_samples) <= ctx->pipe_bytes;
+    const int nb = held ? n_samples : balanced_batch(n_samples, mesh_budget_bytes(ctx) / per_sample);
+    if (int rc = ensure_pipe(ctx, pipe_bytes(nb))) return rc;
     Carver cv(ctx->pipe);
-    int* d_t = cv.take<int>(kpts);
     cplx* d_vt = cv.take<cplx>((size_t)ns * nb);
     cplx* d_H = cv.take<cplx>(nn * kpts * nb);
     double* d_W = cv.take<double>((size_t)N * kpts * nb);
@@ -802,17 +850,10 @@ int rlmb_hlm_mesh_solve_device(rlmb_context* ctx, int lx, int ly, int Q, int ban
     cplx* d_U2 = cv.take<cplx>((size_t)N * kpts * nb);
     int* d_info = cv.take<int>((size_t)kpts * nb);
     if (int rc = reset_failures(ctx)) return rc;
-    {
-        std::vector<int> tl(kpts);
-        for (int t1 = 0; t1 <= g; ++t1)
-            for (int t2 = 0; t2 < g; ++t2) tl[t1 * g + t2] = t1 * (g + 1) + t2;
-        RLMB_CUDA_TRY(cudaMemcpyAsync(d_t, tl.data(), kpts * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
-        RLMB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    }
     for (int s0 = 0; s0 < n_samples; s0 += nb) {
         const int cnt = std::min(nb, n_samples - s0);
         if (int rc = launch_hlm_vtilde(ctx, d_potentials + (size_t)s0 * ns, lx, ly, Q, cnt, d_vt)) return rc;
-        if (int rc = launch_hlm_project(ctx, hb, d_vt, d_t, lx, ly, Q, kpts, cnt, d_H)) return rc;
+        if (int rc = launch_hlm_project(ctx, hb, d_vt, nullptr, g, lx, ly, Q, kpts, cnt, d_H)) return rc;
         if (int rc = rlmb_heevd_batched(ctx, reinterpret_cast<double*>(d_H), d_W, N, cnt * kpts, d_info))
             return rc;
         if (int rc = tally_failures(ctx, d_info, cnt * kpts)) return rc;
@@ -821,7 +862,14 @@ int rlmb_hlm_mesh_solve_device(rlmb_context* ctx, int lx, int ly, int Q, int ban
                                        d_chern + (size_t)s0 * N))
             return rc;
     }
-    return finish_call(ctx);
+    return RLMB_OK;
+}
+
+int rlmb_hlm_mesh_solve_device(rlmb_context* ctx, int lx, int ly, int Q, int band, int n_mesh,
+                               const double* d_potentials, int n_samples, double* d_energies,
+                               double* d_chern) {
+    if (int rc = hlm_enqueue(ctx, lx, ly, Q, band, n_mesh, d_potentials, n_samples, d_energies, d_chern)) return rc;
+    return n_samples == 0 ? RLMB_OK : finish_call(ctx);
 }
 
 int rlmb_hlm_mesh_solve(rlmb_context* ctx, int lx, int ly, int Q, int band, int n_mesh,
@@ -839,13 +887,23 @@ int rlmb_hlm_mesh_solve(rlmb_context* ctx, int lx, int ly, int Q, int band, int 
     double* d_c = d_e + (size_t)N * n_samples;
     RLMB_CUDA_TRY(cudaMemcpyAsync(d_pot, h_potentials, (size_t)ns * n_samples * sizeof(double), cudaMemcpyHostToDevice,
                                   ctx->stream));
-    const int rc = rlmb_hlm_mesh_solve_device(ctx, lx, ly, Q, band, n_mesh, d_pot, n_samples, d_e, d_c);
-    if (rc < 0) return rc;
-    RLMB_CUDA_TRY(cudaMemcpyAsync(h_energies, d_e, (size_t)N * n_samples * sizeof(double), cudaMemcpyDeviceToHost,
-                                  ctx->stream));
-    RLMB_CUDA_TRY(cudaMemcpyAsync(h_chern, d_c, (size_t)N * n_samples * sizeof(double), cudaMemcpyDeviceToHost,
-                                  ctx->stream));
-    RLMB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    if (int rc = hlm_enqueue(ctx, lx, ly, Q, band, n_mesh, d_pot, n_samples, d_e, d_c)) return rc;
+    const size_t cnt = (size_t)N * n_samples, bytes = cnt * sizeof(double);
+    const bool staged = 2 * bytes <= PINNED_RESULTS_MAX;
+    if (staged) {   // energies and Chern numbers lie back to back
+        if (int rc = ensure_pinned(ctx, PINNED_HEAD + 2 * bytes)) return rc;
+        RLMB_CUDA_TRY(cudaMemcpyAsync(static_cast<char*>(ctx->pinned) + PINNED_HEAD, d_e, 2 * bytes,
+                                      cudaMemcpyDeviceToHost, ctx->stream));
+    } else {
+        RLMB_CUDA_TRY(cudaMemcpyAsync(h_energies, d_e, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        RLMB_CUDA_TRY(cudaMemcpyAsync(h_chern, d_c, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    }
+    const int rc = finish_call(ctx);
+    if (rc >= 0 && staged) {
+        const double* r = reinterpret_cast<const double*>(static_cast<char*>(ctx->pinned) + PINNED_HEAD);
+        std::memcpy(h_energies, r, bytes);
+        std::memcpy(h_chern, r + cnt, bytes);
+    }
     return rc;
 }
 

@@ -137,6 +137,9 @@ struct rlmb_context {
     unsigned long mt_seed;
     int mt_nimp;
     long long mt_next;
+    // cached rlm coefficient tables (device) of one mesh geometry: n_phi, o, g, L1, L2
+    double rlm_key[5];
+    void* rlm_tables;
     // cached hlm tables (Bloch vectors and link overlaps of one mesh geometry)
     int hlm_key[6];
     void* hlm_tables;

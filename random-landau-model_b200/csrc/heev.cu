@@ -3456,32 +3456,39 @@ int rlmb::heevd_batched_band(rlmb_context* ctx, double* d_a, double* d_w, int n,
     const HeevPlan plan = heev_plan(n, mixed, heev_steps(ctx), band, tune);
     const size_t per = plan.per;
     // workspace: 8 GB, or for large orders enough for two resident matrices per SM (one
-    // CTA each in k_tridiag), capped at 60 % of the free memory
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-        cudaGetLastError();
-        free_b = (size_t)8 << 30;
-    }
+    // CTA each in k_tridiag); where the workspace has to grow for that, capped at 60 % of the
+    // free memory
     const size_t per2 = plan.per2;
-    size_t budget = std::max<size_t>((size_t)8 << 30, 2 * 148 * (per + per2));
-    budget = std::min<size_t>(budget, free_b / 10 * 6 + ctx->ws_bytes);
-    budget = std::max<size_t>(budget, per + per2);
+    size_t budget = std::max<size_t>(std::max<size_t>((size_t)8 << 30, 2 * 148 * (per + per2)), per + per2);
     if (ctx->frozen) budget = std::max<size_t>(per + per2, ctx->ws_bytes);   // capture: the workspace as sized before
-    // the refinement regions take up to an eighth of the budget (its GEMMs fill the GPU from a
-    // few matrices on); the chunk -- all of whose matrices the one-CTA-per-matrix reduction and
-    // tridiagonal kernels run at once -- takes the rest
-    size_t nb2 = per2 ? std::max<size_t>(1, std::min<size_t>((size_t)batch, budget / 8 / per2)) : 0;
-    size_t chunk = std::max<size_t>(1, std::min<size_t>((budget - nb2 * per2) / per, (size_t)batch));
-    chunk = std::min<size_t>(chunk, 65535);   // grid y / z extent of the per-matrix launches
-    if (!plan.small_bt) chunk = std::min<size_t>(chunk, 65535 / std::max(plan.nblkbt, 1));   // (matrix, block) batches
-    if (plan.dc) chunk = std::min<size_t>(chunk, dc_max_chunk(n));   // (matrix, subproblem, half) GEMM batches
-    // equal chunks: a short last chunk would leave most SMs idle in the one-CTA-per-matrix kernels
-    const size_t nchunks = (batch + chunk - 1) / chunk;
-    chunk = (batch + nchunks - 1) / nchunks;
-    if (per2) {   // equal refinement sub-chunks too
-        nb2 = std::min(nb2, chunk);
-        const size_t nsub = (chunk + nb2 - 1) / nb2;
-        nb2 = (chunk + nsub - 1) / nsub;
+    size_t nb2 = 0, chunk = 0;
+    auto cut = [&]() {
+        // the refinement regions take up to an eighth of the budget (its GEMMs fill the GPU from a
+        // few matrices on); the chunk -- all of whose matrices the one-CTA-per-matrix reduction and
+        // tridiagonal kernels run at once -- takes the rest
+        nb2 = per2 ? std::max<size_t>(1, std::min<size_t>((size_t)batch, budget / 8 / per2)) : 0;
+        chunk = std::max<size_t>(1, std::min<size_t>((budget - nb2 * per2) / per, (size_t)batch));
+        chunk = std::min<size_t>(chunk, 65535);   // grid y / z extent of the per-matrix launches
+        if (!plan.small_bt) chunk = std::min<size_t>(chunk, 65535 / std::max(plan.nblkbt, 1));   // (matrix, block) batches
+        if (plan.dc) chunk = std::min<size_t>(chunk, dc_max_chunk(n));   // (matrix, subproblem, half) GEMM batches
+        // equal chunks: a short last chunk would leave most SMs idle in the one-CTA-per-matrix kernels
+        const size_t nchunks = (batch + chunk - 1) / chunk;
+        chunk = (batch + nchunks - 1) / nchunks;
+        if (per2) {   // equal refinement sub-chunks too
+            nb2 = std::min(nb2, chunk);
+            const size_t nsub = (chunk + nb2 - 1) / nb2;
+            nb2 = (chunk + nsub - 1) / nsub;
+        }
+    };
+    cut();
+    if (!ctx->frozen && chunk * per + nb2 * per2 > ctx->ws_bytes) {
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+            cudaGetLastError();
+            free_b = (size_t)8 << 30;
+        }
+        budget = std::max<size_t>(std::min<size_t>(budget, free_b / 10 * 6 + ctx->ws_bytes), per + per2);
+        cut();
     }
     if (int rc = ensure_workspace(ctx, chunk * per + nb2 * per2)) return rc;
     const size_t nn = (size_t)n * n;

@@ -151,9 +151,10 @@ struct EpRowMajor {
 __global__ void __launch_bounds__(256)
 k_rlm_assemble(const cplx* __restrict__ S, const cplx* __restrict__ cmt, const int* __restrict__ t1s,
                const int* __restrict__ t2s, const __grid_constant__ ThetaList list, int n_phi, int dim, int o,
-               int kpts_per_sample, int kp0, cplx* __restrict__ H) {
+               int kpts_per_sample, int n_theta, int kp0, cplx* __restrict__ H) {
     const int kp = kp0 + blockIdx.y;
-    const int t2 = t2s[kp];
+    // (without lists: the whole mesh, theta_2 fastest)
+    const int mesh = t2s ? 0 : kp % kpts_per_sample, t1 = t2s ? t1s[kp] : mesh / n_theta, t2 = t2s ? t2s[kp] : mesh % n_theta;
     int lo = 0, hi = list.n - 1;   // the slot of t2
     while (lo < hi) {
         const int mid = (lo + hi) / 2;
@@ -165,7 +166,7 @@ k_rlm_assemble(const cplx* __restrict__ S, const cplx* __restrict__ cmt, const i
     if (j >= n_phi) return;
     const int sample = blockIdx.y / kpts_per_sample;
     const cplx* s = S + ((size_t)sample * list.n + lo) * n_phi * dim;
-    const cplx* c1 = cmt + (size_t)t1s[kp] * dim;
+    const cplx* c1 = cmt + (size_t)t1 * dim;
     cplx* h = H + ((size_t)kp * n_phi + j) * n_phi;
     for (int k = threadIdx.x & 31; k < n_phi; k += 32) {
         const int row = min(j, k), delta = max(j, k) - row;
@@ -187,7 +188,8 @@ size_t rlm_assemble_ws_elems(int n_phi, int dim, int nsamples, int n_t2) {
     return std::min(want, rlm_slab_cap(n_phi, dim)) * n_phi * dim;
 }
 
-// k-points kp = 0 .. count-1 (kpts_per_sample consecutive ones per sample, angles d_t1 / d_t2);
+// k-points kp = 0 .. count-1 (kpts_per_sample consecutive ones per sample, angles d_t1 / d_t2, or
+// without these the n_t2 x n_t2 mesh of every sample);
 // uniq_t2: the n_t2 distinct theta_2 indices among them, ascending (host); ws:
 // rlm_assemble_ws_elems(n_phi, dim, samples, n_t2) elements.
 int launch_rlm_assemble(rlmb_context* ctx, const cplx* vmn, const cplx* cmt, const cplx* cjm,
@@ -214,7 +216,7 @@ int launch_rlm_assemble(rlmb_context* ctx, const cplx* vmn, const cplx* cmt, con
             for (int q = 0; q < kps; q += 65535) {
                 prof_begin(ctx, "k_rlm_assemble");
                 k_rlm_assemble<<<dim3((n_phi + 7) / 8, std::min(65535, kps - q)), 256, 0, ctx->stream>>>(
-                    ws, cmt, d_t1, d_t2, list, n_phi, dim, o, kpts_per_sample, kp0 + q, H);
+                    ws, cmt, d_t1, d_t2, list, n_phi, dim, o, kpts_per_sample, n_t2, kp0 + q, H);
                 RLMB_LAUNCHED(ctx);
             }
         }
@@ -535,7 +537,7 @@ int launch_hlm_vtilde(rlmb_context* ctx, const double* pot, int lx, int ly, int 
 template <int QT>
 __global__ void __launch_bounds__(256)
 k_hlm_project(const cplx* __restrict__ hb, const cplx* __restrict__ vt, const int* __restrict__ tlist,
-              int lx, int ly, int Qr, int kpts, cplx* __restrict__ H) {
+              int g, int lx, int ly, int Qr, int kpts, cplx* __restrict__ H) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int Q = QT > 0 ? QT : Qr;
     const int Lxp = lx / Q, N = Lxp * ly, ns = lx * ly;
@@ -543,7 +545,7 @@ k_hlm_project(const cplx* __restrict__ hb, const cplx* __restrict__ vt, const in
     cplx* sv = sh + (size_t)N * Q;                   // [ns]  Vt of this sample
     const int job = blockIdx.y;
     const int sample = job / kpts, k = job % kpts;
-    const int t = tlist[k];
+    const int t = tlist ? tlist[k] : k / g * (g + 1) + k % g;   // (without a list: the mesh, theta_2 < g)
     for (int i = threadIdx.x; i < N * Q; i += blockDim.x) sh[i] = hb[(size_t)t * N * Q + i];
     for (int i = threadIdx.x; i < ns; i += blockDim.x) sv[i] = vt[(size_t)sample * ns + i];
     __syncthreads();
@@ -587,7 +589,7 @@ k_hlm_project(const cplx* __restrict__ hb, const cplx* __restrict__ vt, const in
     }
 }
 
-int launch_hlm_project(rlmb_context* ctx, const cplx* hb, const cplx* vt, const int* d_tlist, int lx,
+int launch_hlm_project(rlmb_context* ctx, const cplx* hb, const cplx* vt, const int* d_tlist, int g, int lx,
                        int ly, int Q, int kpts, int nsamples, cplx* H) {
     const int N = lx * ly / Q;
     const size_t smem = ((size_t)N * Q + (size_t)lx * ly) * sizeof(cplx);
@@ -598,7 +600,7 @@ int launch_hlm_project(rlmb_context* ctx, const cplx* hb, const cplx* vt, const 
     const int bx = std::max(1, std::min(N / 32, 16));   // column slices of >= 32 columns per k-point
     dim3 grid(bx, kpts * nsamples);
     prof_begin(ctx, "k_hlm_project");
-    kern<<<grid, 256, smem, ctx->stream>>>(hb, vt, d_tlist, lx, ly, Q, kpts, H);
+    kern<<<grid, 256, smem, ctx->stream>>>(hb, vt, d_tlist, g, lx, ly, Q, kpts, H);
     RLMB_LAUNCHED(ctx);
     return RLMB_OK;
 }

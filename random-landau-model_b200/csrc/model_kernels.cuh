@@ -27,7 +27,7 @@ int launch_hlm_bloch(rlmb_context* ctx, int lx, int ly, int Q, int band, int g, 
 int launch_hlm_basis_expand(rlmb_context* ctx, const cplx* hb, int lx, int ly, int Q, int g, int t1,
                             int t2, cplx* W);
 int launch_hlm_vtilde(rlmb_context* ctx, const double* pot, int lx, int ly, int Q, int nsamples, cplx* vt);
-int launch_hlm_project(rlmb_context* ctx, const cplx* hb, const cplx* vt, const int* d_tlist, int lx,
+int launch_hlm_project(rlmb_context* ctx, const cplx* hb, const cplx* vt, const int* d_tlist, int g, int lx,
                        int ly, int Q, int kpts, int nsamples, cplx* H);
 int launch_hlm_links(rlmb_context* ctx, const cplx* hb, const cplx* X, int lx, int ly, int Q, int g,
                      int nsamples, cplx* U1, cplx* U2);
