@@ -874,58 +874,63 @@ __device__ __forceinline__ C refl_entry(const C* __restrict__ a, int n, int i, i
     return a[(size_t)(i + 1) * n + r];
 }
 
-// T factors of every block of one matrix (one CTA per matrix):
+// T factor of one block of one matrix, grid (blocks, matrices):
 //   T[k][k] = tau_k,  T[k][q] = -tau_k sum_{l=q}^{k-1} (v_k^H v_l) T[l][q]   (q < k)
 template <class R>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(128)
 k_larft(const typename Cx<R>::T* __restrict__ A, const typename Cx<R>::T* __restrict__ TAU,
         typename Cx<R>::T* __restrict__ Tw, int n) {
     typedef typename Cx<R>::T C;
     __shared__ C G[ORM_NB][ORM_NB];
     __shared__ C T[ORM_NB][ORM_NB];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const size_t mat = blockIdx.x;
+    const size_t mat = blockIdx.y;
     const C* a = A + mat * (size_t)n * n;
     const C* tau = TAU + mat * n;
-    const int nblk = (n - 1 + ORM_NB - 1) / ORM_NB;
-    for (int j = 0; j < nblk; ++j) {
-        const int i0 = j * ORM_NB;
-        // G[k][l] = v_k^H v_l for l < k: rows 0..i0+l overlap
-        for (int pr = warp; pr < ORM_NB * ORM_NB; pr += 8) {
-            const int k = pr / ORM_NB, l = pr % ORM_NB;
-            if (l >= k) continue;
-            const int ik = i0 + k, il = i0 + l;
-            C s = cz<C>();
-            if (ik <= n - 2) {
-                for (int r = lane; r <= il; r += 32) cfmac(s, refl_entry(a, n, ik, r), refl_entry(a, n, il, r));
+    const int i0 = blockIdx.x * ORM_NB;
+    // G[k][l] = v_k^H v_l for l < k: rows 0..i0+l overlap; a warp takes k = warp, warp + 4, ...
+    // with the entries of v_k in registers' reach for all l
+    for (int k = warp; k < ORM_NB; k += 4) {
+        const int ik = i0 + k;
+        if (ik > n - 2) break;
+        for (int l0 = 0; l0 < k; l0 += 4) {
+            C s[4] = {cz<C>(), cz<C>(), cz<C>(), cz<C>()};
+            const int top = i0 + min(l0 + 3, k - 1);
+            for (int r = lane; r <= top; r += 32) {
+                const C vk = refl_entry(a, n, ik, r);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (l0 + u < k) cfmac(s[u], vk, refl_entry(a, n, i0 + l0 + u, r));
             }
-            s = warp_sum(s);
-            if (lane == 0) G[k][l] = s;
-        }
-        __syncthreads();
-        if (warp == 0) {
-            for (int k = 0; k < ORM_NB; ++k) {
-                const int ik = i0 + k;
-                const C tk = ik <= n - 2 ? tau[ik] : cz<C>();
-                if (lane < ORM_NB) {
-                    C val = cz<C>();
-                    if (lane == k) {
-                        val = tk;
-                    } else if (lane < k) {
-                        C s = cz<C>();
-                        for (int l = lane; l < k; ++l) cfma(s, G[k][l], T[l][lane]);
-                        val = cscale(cmul(tk, s), (R)-1);
-                    }
-                    T[k][lane] = val;
-                }
-                __syncwarp();
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const C t = warp_sum(s[u]);
+                if (lane == 0 && l0 + u < k) G[k][l0 + u] = t;
             }
         }
-        __syncthreads();
-        C* out = Tw + (mat * nblk + j) * ORM_NB * ORM_NB;
-        out[threadIdx.x] = T[threadIdx.x / ORM_NB][threadIdx.x % ORM_NB];
-        __syncthreads();
     }
+    __syncthreads();
+    if (warp == 0) {
+        for (int k = 0; k < ORM_NB; ++k) {
+            const int ik = i0 + k;
+            const C tk = ik <= n - 2 ? tau[ik] : cz<C>();
+            if (lane < ORM_NB) {
+                C val = cz<C>();
+                if (lane == k) {
+                    val = tk;
+                } else if (lane < k && ik <= n - 2) {
+                    C s = cz<C>();
+                    for (int l = lane; l < k; ++l) cfma(s, G[k][l], T[l][lane]);
+                    val = cscale(cmul(tk, s), (R)-1);
+                }
+                T[k][lane] = val;
+            }
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    C* out = Tw + (mat * gridDim.x + blockIdx.x) * ORM_NB * ORM_NB;
+    for (int i = threadIdx.x; i < ORM_NB * ORM_NB; i += 128) out[i] = T[i / ORM_NB][i % ORM_NB];
 }
 
 // asynchronous global -> shared copy of one complex element (16 or 8 bytes)
@@ -1080,6 +1085,152 @@ k_ormtr(const typename Cx<R>::T* __restrict__ A, const typename Cx<R>::T* __rest
     }
 }
 
+// The same in double precision on the FP64 tensor path (DMMA, m8n8k4): one CTA keeps CW columns
+// of X in shared memory (X[r][c], rows padded to 8) for the whole transformation, so that X
+// crosses device memory once whatever the number of blocks.  Per block of 16 reflectors, staged
+// as V[r][k]:
+//   W = V^H X     2 x CW/8 tiles of 8 x 8, WH warps per tile (each an equal share of the rows,
+//                 the shares added by the next product's loads)
+//   W <- T W      one tile per warp
+//   X -= V W      a warp takes 8-row tiles, W's fragments in registers
+// Column c of row r of X and V sits at c ^ om_swz(r), so that the 8 lanes of a 16-byte phase hit
+// distinct banks in every fragment: 2 columns x 4 rows (W's operands), 4 even columns x 2 rows
+// (X as the accumulator), 4 columns x 2 rows (V in the last product).
+// 256 threads where two CTAs or more fit an SM, 512 where X and V leave room for one.
+// Bound: the DMMA pipe (8 n^3 flops) and, between the products, barriers and V's staging.
+// (order 256: the pipe is 57 % busy).  k_ormtr took 2.76 ms for 4,624 matrices of order 64 and
+// 0.34 ms for 2,304 of order 32; this kernel 0.65 and 0.07.  Against the GEMM form (X read twice
+// and written once per 64 reflectors), T factors included: order 256, 1,408 matrices 14.5 ->
+// 11.0 ms, order 380, 296 matrices 8.6 -> 7.3 ms.
+static constexpr int OM_TS = ORM_NB + 2;   // row stride of T
+__device__ __forceinline__ int om_swz(int r) { return (r & 1) * 5 + (r & 2); }   // 0, 5, 2, 7 by r mod 4
+template <int CW, int NT>
+struct OrmtrMma {
+    static constexpr int CT = CW / 8, WH = NT / 64 / CT, WS = CW + 2;
+    static __host__ __device__ constexpr size_t smem(int n) {
+        return sizeof(cplx) * ((size_t)((n + 7) / 8 * 8) * (CW + ORM_NB) + WH * ORM_NB * WS + ORM_NB * OM_TS);
+    }
+};
+template <int CW, int NT>
+__global__ void __launch_bounds__(NT, 512 / NT)
+k_ormtr_mma(const cplx* __restrict__ A, const cplx* __restrict__ Tw, const double* __restrict__ Z,
+            cplx* __restrict__ X, int n) {
+    constexpr int CT = OrmtrMma<CW, NT>::CT, WH = OrmtrMma<CW, NT>::WH, WS = OrmtrMma<CW, NT>::WS;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int np = (n + 7) / 8 * 8;
+    cplx* xs = reinterpret_cast<cplx*>(smem_raw);   // [np][CW]
+    cplx* vs = xs + (size_t)np * CW;                // [np][16]
+    cplx* ws = vs + (size_t)np * ORM_NB;            // [WH][16][WS]
+    cplx* ts = ws + WH * ORM_NB * WS;               // [16][OM_TS]
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, g = lane >> 2, q = lane & 3;
+    const int sq = om_swz(q), sg = om_swz(g);       // swizzles of rows 4 k + q and 8 k + g
+    const size_t mat = blockIdx.y;
+    const int col0 = blockIdx.x * CW;
+    const cplx* a = A + mat * (size_t)n * n;
+    const double* z = Z + mat * (size_t)n * n;
+    const int nblk = (n - 1 + ORM_NB - 1) / ORM_NB;
+    const cplx* tw = Tw + mat * (size_t)nblk * ORM_NB * ORM_NB;
+    for (int i = t; i < np * CW; i += NT) {
+        const int r = i / CW, c = i % CW;
+        xs[r * CW + (c ^ om_swz(r))] = mk(r < n && col0 + c < n ? z[(size_t)r * n + col0 + c] : 0.0, 0.0);
+    }
+    const int m = warp & 1, nt = (warp >> 1) % CT, part = warp / (2 * CT);   // the warp's tile of W, its share
+    for (int j = 0; j < nblk; ++j) {
+        const int i0 = j * ORM_NB, i1 = min(i0 + ORM_NB - 1, n - 2);
+        const int rows = (i1 + 1 + 7) / 8 * 8;
+        // stage V (rows 0 .. rows-1, the implicit ones and the zeros included) and T
+        for (int k = warp; k < ORM_NB; k += NT / 32) {
+            const int ir = i0 + k;
+            const cplx* src = a + (size_t)(ir + 1) * n;
+            for (int r = lane; r < rows; r += 32) {
+                cplx* dst = &vs[r * ORM_NB + (k ^ om_swz(r))];
+                if (ir <= n - 2 && r < ir) cp_async_elem(dst, src + r);
+                else *dst = mk(ir <= n - 2 && r == ir ? 1.0 : 0.0, 0.0);
+            }
+        }
+        if (t < ORM_NB * ORM_NB)
+            cp_async_elem(&ts[(t / ORM_NB) * OM_TS + t % ORM_NB], &tw[(size_t)j * ORM_NB * ORM_NB + t]);
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncthreads();
+        {   // W tile (m, nt) = V^H X over this warp's rows
+            double ra[2] = {0, 0}, rb[2] = {0, 0}, ia[2] = {0, 0}, ib[2] = {0, 0};
+            const cplx* vp = vs + q * ORM_NB + ((8 * m + g) ^ sq);
+            const cplx* xp = xs + q * CW + ((8 * nt + g) ^ sq);
+#pragma unroll 4
+            for (int k = 4 * part; k < rows; k += 4 * WH) {
+                const cplx v = vp[k * ORM_NB], x = xp[k * CW];
+                dmma884(ra, v.x, x.x);
+                dmma884(rb, v.y, x.y);
+                dmma884(ia, v.x, x.y);
+                dmma884(ib, -v.y, x.x);
+            }
+            cplx* wp = ws + (part * ORM_NB + 8 * m + g) * WS + 8 * nt + 2 * q;
+            wp[0] = mk(ra[0] + rb[0], ia[0] + ib[0]);
+            wp[1] = mk(ra[1] + rb[1], ia[1] + ib[1]);
+        }
+        __syncthreads();
+        cplx w2[2];
+        if (part == 0) {   // T W tile (m, nt): T is lower triangular, so the upper tile row needs half of it
+            double cr[2] = {0, 0}, ci[2] = {0, 0};
+#pragma unroll
+            for (int k = 0; k < ORM_NB; k += 4) {
+                if (k >= 8 * (m + 1)) break;
+                const cplx v = ts[(8 * m + g) * OM_TS + k + q];
+                cplx x = ws[(k + q) * WS + 8 * nt + g];
+#pragma unroll
+                for (int h = 1; h < WH; ++h) x = cadd(x, ws[(h * ORM_NB + k + q) * WS + 8 * nt + g]);
+                dmma884(cr, v.x, x.x);
+                dmma884(cr, -v.y, x.y);
+                dmma884(ci, v.x, x.y);
+                dmma884(ci, v.y, x.x);
+            }
+            w2[0] = mk(cr[0], ci[0]);
+            w2[1] = mk(cr[1], ci[1]);
+        }
+        __syncthreads();
+        if (part == 0) {
+            cplx* wp = ws + (8 * m + g) * WS + 8 * nt + 2 * q;
+            wp[0] = w2[0];
+            wp[1] = w2[1];
+        }
+        __syncthreads();
+        {   // X -= V W
+            cplx b[4][CT];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int c = 0; c < CT; ++c) b[k][c] = ws[(4 * k + q) * WS + 8 * c + g];
+            for (int r0 = 8 * warp; r0 < rows; r0 += NT / 4) {
+                cplx v[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[k] = vs[(r0 + g) * ORM_NB + ((4 * k + q) ^ sg)];
+#pragma unroll
+                for (int c = 0; c < CT; ++c) {
+                    cplx* xp = xs + (r0 + g) * CW;
+                    const int k0 = (8 * c + 2 * q) ^ sg, k1 = k0 ^ 1;
+                    const cplx x0 = xp[k0], x1 = xp[k1];
+                    double cr[2] = {x0.x, x1.x}, ci[2] = {x0.y, x1.y};
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        dmma884(cr, -v[k].x, b[k][c].x);
+                        dmma884(ci, -v[k].x, b[k][c].y);
+                        dmma884(cr, v[k].y, b[k][c].y);
+                        dmma884(ci, -v[k].y, b[k][c].x);
+                    }
+                    xp[k0] = mk(cr[0], ci[0]);
+                    xp[k1] = mk(cr[1], ci[1]);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (nblk == 0) __syncthreads();
+    cplx* xo = X + mat * (size_t)n * n;
+    for (int c = warp; c < CW; c += NT / 32)
+        for (int r = lane; r < n && col0 + c < n; r += 32) xo[(size_t)(col0 + c) * n + r] = xs[r * CW + (c ^ om_swz(r))];
+}
+
 // ------------------------------------------------ back-transformation for large orders
 // For orders whose 16-reflector blocks do not fit the register/shared-memory scheme of
 // k_ormtr, X = Q Z is applied with blocks of BT_NB = 64 reflectors (or 128, a tuning choice)
@@ -1087,7 +1238,8 @@ k_ormtr(const typename Cx<R>::T* __restrict__ A, const typename Cx<R>::T* __rest
 // X -= V W'.  X lives in global memory (column-major, column = eigenvector) and is read twice
 // and written once per block.
 static constexpr int BT_NB = 64;
-static constexpr int BT_GEMM_MIN = 256;   // order from which the GEMM back-transformation runs
+static constexpr int BT_GEMM_MIN = 256;   // mixed mode: order from which the GEMM back-transformation runs
+static constexpr int BT_MMA_MAX = 408;    // double precision: order up to which k_ormtr_mma runs (the largest that fits)
 // Blocks of 128 reflectors (T from two 64-reflector halves, k_larft128) halve the passes
 // over X, but at order 3000 they were no faster in double precision and 10 % slower in single
 // precision (the block GEMMs are bound by the tensor pipes, not by X's traffic): they are a
@@ -2742,7 +2894,7 @@ struct HeevPlan {
     int band;            // >= 0: every matrix is a cyclic band of this half-bandwidth (rlm), else -1
     size_t smem_tri;
     bool small_bt;       // k_ormtr (register-resident Z chunk) or the blocked GEMM path
-    int ch, dbuf;
+    int ch, dbuf, orm_nt;
     size_t smem_orm;
     int nblk16, bt_nb, nblkbt;   // k_ormtr blocks; GEMM back-transformation block size and count
     int npanels, m_tail;  // blocked reduction: panels of pw columns, then k_hetrd on m_tail
@@ -2783,20 +2935,29 @@ static HeevPlan heev_plan(int n, bool mixed, int refine_steps = 2, int band = -1
     p.nblk16 = (n - 1 + ORM_NB - 1) / ORM_NB;
     p.bt_nb = tune.bt_nb ? tune.bt_nb : n >= BT128_MIN ? 2 * BT_NB : BT_NB;
     p.nblkbt = (n - 1 + p.bt_nb - 1) / p.bt_nb;
-    int ch = 16;
-    while (ch > 1 && (n + 256 / ch - 1) / (256 / ch) > ORM_RPT) ch >>= 1;
-    p.ch = ch;
-    const int onw = 8;   // warps of k_ormtr (256 threads; 512 threads of 8 rows, or 8 columns
-                         // of 8 rows at two CTAs per SM, measured slower)
-    size_t smem = ((size_t)2 * n * ORM_VS + 2 * ORM_NB * ORM_NB + onw * ORM_NB * ch + ORM_NB * ch) * ce;
-    p.dbuf = smem <= 220 * 1024 ? 1 : 0;
-    if (!p.dbuf)
-        smem = ((size_t)std::max(n * ORM_VS, n * ch) + ORM_NB * ORM_NB + onw * ORM_NB * ch + ORM_NB * ch) * ce;
-    p.smem_orm = smem;
-    // register-resident k_ormtr up to order 255 (it beats the GEMM path there), the GEMM path
-    // (double precision on the DMMA engine) from 256 on
-    const bool reg_fits = (n + 256 / ch - 1) / (256 / ch) <= ORM_RPT && smem <= 220 * 1024;
-    p.small_bt = reg_fits && (tune.gemm_bt < 0 ? n < BT_GEMM_MIN : tune.gemm_bt == 0);
+    bool fits;
+    if (mixed) {   // k_ormtr<float>
+        int ch = 16;
+        while (ch > 1 && (n + 256 / ch - 1) / (256 / ch) > ORM_RPT) ch >>= 1;
+        p.ch = ch;
+        const int onw = 8;   // warps of k_ormtr (256 threads; 512 threads of 8 rows, or 8 columns
+                             // of 8 rows at two CTAs per SM, measured slower)
+        size_t smem = ((size_t)2 * n * ORM_VS + 2 * ORM_NB * ORM_NB + onw * ORM_NB * ch + ORM_NB * ch) * ce;
+        p.dbuf = smem <= 220 * 1024 ? 1 : 0;
+        if (!p.dbuf)
+            smem = ((size_t)std::max(n * ORM_VS, n * ch) + ORM_NB * ORM_NB + onw * ORM_NB * ch + ORM_NB * ch) * ce;
+        p.smem_orm = smem;
+        fits = (n + 256 / ch - 1) / (256 / ch) <= ORM_RPT && smem <= 220 * 1024;
+    } else {       // k_ormtr_mma: 32 columns per CTA, 16 where X and V leave no room for more
+        p.ch = OrmtrMma<32, 512>::smem(n) <= 227 * 1024 ? 32 : 16;
+        p.orm_nt = p.ch == 32 && OrmtrMma<32, 256>::smem(n) <= 113 * 1024 ? 256 : 512;
+        p.smem_orm = p.ch == 16 ? OrmtrMma<16, 512>::smem(n)
+                   : p.orm_nt == 256 ? OrmtrMma<32, 256>::smem(n) : OrmtrMma<32, 512>::smem(n);
+        fits = p.smem_orm <= 227 * 1024;
+    }
+    // X resident on the SM where it fits: below order 256 in the mixed mode, up to BT_MMA_MAX in
+    // double precision (it beats the GEMM path there), the GEMM path otherwise
+    p.small_bt = fits && (tune.gemm_bt < 0 ? (mixed ? n < BT_GEMM_MIN : n <= BT_MMA_MAX) : tune.gemm_bt == 0);
     const size_t nn = (size_t)n * n;
     auto r256 = [](size_t v) { return (v + 255) / 256 * 256; };
     size_t off = 0;
@@ -2964,18 +3125,26 @@ static int back_transform(rlmb_context* ctx, cudaStream_t st, const HeevPlan& p,
     const int n = p.n;
     const size_t nn = (size_t)n * n;
     if (p.small_bt) {
-        auto ormtr = p.ch == 16 ? k_ormtr<16, 256, ORM_RPT, R> : p.ch == 8 ? k_ormtr<8, 256, ORM_RPT, R>
-                   : p.ch == 4 ? k_ormtr<4, 256, ORM_RPT, R> : p.ch == 2 ? k_ormtr<2, 256, ORM_RPT, R>
-                   : k_ormtr<1, 256, ORM_RPT, R>;
-        if (cudaFuncSetAttribute(ormtr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem_orm) != cudaSuccess)
-            return RLMB_ERR_CUDA;
         if (n > 1) {
             RLMB_CHUNK_PROF("k_larft");
-            k_larft<R><<<nb, 256, 0, st>>>(Aw, TAUw, Tw, n);
+            k_larft<R><<<dim3(p.nblk16, nb), 128, 0, st>>>(Aw, TAUw, Tw, n);
             RLMB_CHUNK_LAUNCHED();
         }
+        const dim3 grid((n + p.ch - 1) / p.ch, nb);
         RLMB_CHUNK_PROF("k_ormtr");
-        ormtr<<<dim3((n + p.ch - 1) / p.ch, nb), 256, p.smem_orm, st>>>(Aw, Tw, Zw, Xw, n, p.dbuf);
+        if constexpr (std::is_same<R, double>::value) {
+            auto ormtr = p.ch == 16 ? k_ormtr_mma<16, 512> : p.orm_nt == 256 ? k_ormtr_mma<32, 256> : k_ormtr_mma<32, 512>;
+            if (cudaFuncSetAttribute(ormtr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem_orm) != cudaSuccess)
+                return RLMB_ERR_CUDA;
+            ormtr<<<grid, p.orm_nt, p.smem_orm, st>>>(Aw, Tw, Zw, Xw, n);
+        } else {
+            auto ormtr = p.ch == 16 ? k_ormtr<16, 256, ORM_RPT, R> : p.ch == 8 ? k_ormtr<8, 256, ORM_RPT, R>
+                       : p.ch == 4 ? k_ormtr<4, 256, ORM_RPT, R> : p.ch == 2 ? k_ormtr<2, 256, ORM_RPT, R>
+                       : k_ormtr<1, 256, ORM_RPT, R>;
+            if (cudaFuncSetAttribute(ormtr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem_orm) != cudaSuccess)
+                return RLMB_ERR_CUDA;
+            ormtr<<<grid, 256, p.smem_orm, st>>>(Aw, Tw, Zw, Xw, n, p.dbuf);
+        }
         RLMB_CHUNK_LAUNCHED();
         return RLMB_OK;
     }
