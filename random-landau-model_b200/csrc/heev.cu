@@ -6,7 +6,7 @@
 // calls reach is restated from its published algorithms:
 //
 //   reduction      A = Q T Q^H (zhetrd, uplo='U').  From order 256: panels of 16 columns
-//                  (32 from order 1024 in double precision; k_hetrd_panel, zlatrd restated)
+//                  (32 from order 1024 in double precision; k_hetrd_panel_c, zlatrd restated)
 //                  whose rank-32 (rank-64) updates run as batched GEMMs over all SMs
 //                  (launch_zgemm); the last leading
 //                  block (order <= 64, or all of a smaller matrix) by the unblocked,
@@ -231,7 +231,7 @@ __device__ __forceinline__ void reflector(const C alpha, R xnorm2, R& beta, C& t
 // Unblocked reduction A = Q T Q^H (zhetd2, uplo='U') with look-ahead: step i's rank-2
 // update and step i-1's matrix-vector product share one pass over the leading block.
 // a: n*n col-major (upper triangle), real type R (double, or float in the mixed mode); the
-// leading m x m block is reduced (m < n after the blocked panels of k_hetrd_panel, which
+// leading m x m block is reduced (m < n after the blocked panels of k_hetrd_panel_c, which
 // own E and TAU from index m - 1 on).
 // On exit column c (c >= 1) rows 0..c-2 hold the reflector of step c-1 (its entry c-1 is
 // 1 and not stored), D/E the tridiagonal (double) and TAU the reflector scalars.  The
@@ -1525,7 +1525,7 @@ struct EpSub {     // X(r, c) -= acc
 
 // ------------------------------------------------------------- blocked k_hetrd (large n)
 // For large orders the reduction runs in panels of pw (16 or 32) columns (LAPACK zlatrd + zher2k,
-// uplo='U', restated): k_hetrd_panel reduces columns m-1 .. m-pw of the leading m x m
+// uplo='U', restated): k_hetrd_panel_c reduces columns m-1 .. m-pw of the leading m x m
 // block one CTA per matrix, keeping each column's reflector v and its w = tau A' v - ...
 // in the panel buffers V, W instead of updating the leading block: column c is first
 // brought up to date with the panel's earlier pairs, its matrix-vector product reads the
@@ -1740,22 +1740,6 @@ __host__ __device__ constexpr size_t panel_smem(int m) {
     return (2 * (size_t)m + 2 * HP_W_MAX) * sizeof(typename Cx<R>::T) + 2 * (NT / 32) * sizeof(R);
 }
 
-// One CTA per matrix: the panel's pw columns in order.
-template <int NT, class R>
-__global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2)
-k_hetrd_panel(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, double* __restrict__ E,
-              typename Cx<R>::T* __restrict__ TAU, typename Cx<R>::T* __restrict__ PV,
-              typename Cx<R>::T* __restrict__ PW, int n, int m, int pw) {
-    typedef typename Cx<R>::T C;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    C* vn = reinterpret_cast<C*>(smem_raw);
-    C* pn = vn + m;
-    C* coef = pn + m;
-    R* red = reinterpret_cast<R*>(coef + 2 * HP_W_MAX);
-    for (int j = 0; j < pw; ++j)
-        panel_column<NT, R, false>(A, D, E, TAU, PV, PW, n, m, blockIdx.x, j, pw, vn, pn, coef, red);
-}
-
 // The same panel for chunks of more matrices than SMs: one resident CTA of NT threads per SM
 // (grid <= SMs) takes units (matrix, column) from a queue, unit u = claim - base = matrix
 // u % nb, column u / nb, so that every SM keeps NT threads of loads in flight whatever the
@@ -1861,12 +1845,14 @@ __device__ __forceinline__ T* panel_peer(T* p, int rank, int P) {
 // being multiplied while the next three are on their way, whatever the unit they belong to.
 static constexpr int HU_W = 16;
 static constexpr int HU_RING = 4 * 32 * 4;   // entries of a warp's ring: quarters x lanes x columns
+template <class C>
 struct HemvPos {
     int u, g, c0, r0, r1;   // unit counted from segment g on, its strip, block and last row
-    bool ok;
+    bool ok, inside;        // a block; wholly above the diagonal and in the matrix
+    const C* src;           // this lane's first entry of the block
     // the first unit at or after u counted from segment g on
-    __device__ __forceinline__ void unit(int m, int seg) {
-        const int nstrips = (m + HU_W - 1) / HU_W;
+    __device__ __forceinline__ void unit(const C* a, int ld, int m, int seg) {
+        const int lane = threadIdx.x & 31, nstrips = (m + HU_W - 1) / HU_W;
         for (;; ++g) {
             const int s0 = g * seg * (32 / HU_W), cnt = nstrips - s0;
             if (cnt <= 0) {
@@ -1878,18 +1864,35 @@ struct HemvPos {
                 r0 = g * seg * 32;
                 r1 = min(min(c0 + HU_W, m), (g + 1) * seg * 32);   // rows on or above the diagonal
                 ok = true;
+                inside = c0 + HU_W <= m && r0 + 32 <= c0;
+                src = a + (size_t)(c0 + (lane >> 3)) * ld + r0 + (lane & 7);
                 return;
             }
             u -= cnt;
         }
     }
 };
+template <int I>
+__device__ __forceinline__ void hemv_copy(unsigned dst, const cplx* src) {
+    asm volatile("cp.async.cg.shared.global [%0+%2], [%1+%3], 16;\n" ::"r"(dst), "l"(src), "n"(I * 32 * 16), "n"(I * 8 * 16) : "memory");
+}
+template <int I>
+__device__ __forceinline__ void hemv_copy(unsigned dst, const cplxf* src) {
+    asm volatile("cp.async.ca.shared.global [%0+%2], [%1+%3], 8;\n" ::"r"(dst), "l"(src), "n"(I * 32 * 8), "n"(I * 8 * 8) : "memory");
+}
+// Quarter q of block t (src: its entries of this lane) into the lane's ring slots at dst.
 template <class C>
-__device__ __forceinline__ void hemv_fetch(const C* __restrict__ a, int ld, int m, const HemvPos& t, int q, C* ring) {
+__device__ __forceinline__ void hemv_fetch(const C* __restrict__ a, int m, const HemvPos<C>& t, int q, const C* src,
+                                           unsigned dst) {
+    if (t.inside) {
+        hemv_copy<0>(dst, src);
+        hemv_copy<1>(dst, src);
+        hemv_copy<2>(dst, src);
+        hemv_copy<3>(dst, src);
+        return;
+    }
     const int lane = threadIdx.x & 31;
     const int r = t.r0 + (lane & 7), c = t.c0 + 4 * q + (lane >> 3);
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(ring + q * 128 + lane);
-    const C* src = a + (size_t)c * ld + r;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int n = c < m && r + 8 * i <= c ? (int)sizeof(C) : 0;   // outside: zeros
@@ -1902,24 +1905,26 @@ __device__ __forceinline__ void hemv_fetch(const C* __restrict__ a, int ld, int 
 }
 // The first block's four quarters on their way (one group each).
 template <class C>
-__device__ __forceinline__ HemvPos hemv_begin(const C* __restrict__ a, int ld, int m, int gw, int seg, C* ring) {
-    HemvPos t;
+__device__ __forceinline__ HemvPos<C> hemv_begin(const C* __restrict__ a, int ld, int m, int gw, int seg, C* ring) {
+    HemvPos<C> t{};
     t.u = gw;
-    t.g = 0;
-    t.c0 = t.r0 = t.r1 = 0;
-    t.unit(m, seg);
+    t.unit(a, ld, m, seg);
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(ring + (threadIdx.x & 31));
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        if (t.ok) hemv_fetch(a, ld, m, t, q, ring);
+        if (t.ok) hemv_fetch(a, m, t, q, t.src + (size_t)(4 * q) * ld, dst + q * 128 * (int)sizeof(C));
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
     return t;
 }
-// The product from position t (hemv_begin) on; returns this lane's share of v^H A v.
+// The product from position t (hemv_begin) on; returns this lane's share of v^H A v.  v and p
+// are readable up to 32 entries beyond m (entries of A there are 0).
 template <class C, class R>
 __device__ __forceinline__ R hemv_units(const C* __restrict__ a, int ld, int m, const C* __restrict__ v, C* p,
-                                        HemvPos t, int GW, int seg, C* ring) {
+                                        HemvPos<C> t, int GW, int seg, C* ring) {
     const int lane = threadIdx.x & 31, lr = lane & 7, lc = lane >> 3;
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(ring + lane);
+    const size_t qstep = (size_t)4 * ld;
     R quad = 0;
     C es[4], vc[4];
 #pragma unroll
@@ -1927,33 +1932,39 @@ __device__ __forceinline__ R hemv_units(const C* __restrict__ a, int ld, int m, 
     bool first = true;   // block of its unit
 #pragma unroll 1
     while (t.ok) {
-        if (first)
+        if (first) {
+            const C* vp = v + t.c0 + lc;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                vc[j] = v[min(t.c0 + lc + 4 * j, m - 1)];   // (beyond the matrix the entries are 0)
+                vc[j] = vp[4 * j];
                 es[j] = cz<C>();
             }
-        HemvPos nx = t;
+        }
+        HemvPos<C> nx = t;
         nx.r0 += 32;
+        nx.src += 32;
         const bool last = nx.r0 >= t.r1;
         if (last) {
             nx.u += GW;
-            nx.unit(m, seg);
+            nx.unit(a, ld, m, seg);
+        } else {
+            nx.inside = t.inside && nx.r0 + 32 <= t.c0;
         }
-        const bool inside = t.c0 + HU_W <= m && t.r0 + 32 <= t.c0;
         C rs[4], vr[4];
+        const C* vp = v + t.r0 + lr;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             rs[i] = cz<C>();
-            vr[i] = v[min(t.r0 + lr + 8 * i, m - 1)];
+            vr[i] = vp[8 * i];
         }
+        const C* src = nx.src;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             asm volatile("cp.async.wait_group 3;\n" ::: "memory");
             C x[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) x[i] = ring[q * 128 + i * 32 + lane];
-            if (!inside) {
+            if (!t.inside) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
                     if (t.r0 + lr + 8 * i == t.c0 + lc + 4 * q) {   // the diagonal: real, counted once
@@ -1968,9 +1979,12 @@ __device__ __forceinline__ R hemv_units(const C* __restrict__ a, int ld, int m, 
                 cfma(rs[i], x[i], vc[q]);
                 cfmac(es[q], x[i], vr[i]);
             }
-            if (nx.ok) hemv_fetch(a, ld, m, nx, q, ring);
+            if (nx.ok) hemv_fetch(a, m, nx, q, src, dst + q * 128 * (int)sizeof(C));
+            src += qstep;
             asm volatile("cp.async.commit_group;\n" ::: "memory");
         }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) quad += 2 * (vr[i].x * rs[i].x + vr[i].y * rs[i].y);
         {   // row sums over the four lanes of a row: lane ends with row r0 + lane
             const bool u1 = (lane & 16) != 0, u0 = (lane & 8) != 0;
             C y[2];
@@ -1981,12 +1995,7 @@ __device__ __forceinline__ R hemv_units(const C* __restrict__ a, int ld, int m, 
             }
             const C send = u0 ? y[0] : y[1], keep = u0 ? y[1] : y[0];
             const C s = cadd(keep, shfl_xor(send, 8));
-            const int r = t.r0 + lane;
-            if (r < min(t.c0 + HU_W, m)) {
-                const C vl = v[r];
-                quad += 2 * (vl.x * s.x + vl.y * s.y);
-                smem_atomic_add(&p[r], s);
-            }
+            if (t.inside || t.r0 + lane < min(t.c0 + HU_W, m)) smem_atomic_add(&p[t.r0 + lane], s);
         }
         if (last) {   // column sums over the eight lanes of a column: lane ends with column lc + 4 (lr / 2)
             const bool u2 = (lane & 4) != 0, u1 = (lane & 2) != 0;
@@ -2013,7 +2022,7 @@ static constexpr int PC_MAX = 16;   // CTAs per cluster
 template <int NT, class R>
 __host__ __device__ constexpr size_t panel_c_smem(int m, int P) {
     typedef typename Cx<R>::T C;
-    return (2 * (size_t)m + (NT / 32) * HU_RING + (size_t)P * 2 * HP_W_MAX + 4 * HP_W_MAX + 4) * sizeof(C) +
+    return (2 * (size_t)(m + 32) + (NT / 32) * HU_RING + (size_t)P * 2 * HP_W_MAX + 4 * HP_W_MAX + 4) * sizeof(C) +
            2 * (size_t)P * (NT / 32) * sizeof(R);
 }
 
@@ -2027,21 +2036,24 @@ __host__ __device__ constexpr size_t panel_c_smem(int m, int P) {
 //   -- barrier --   sums of the CTAs' parts over distributed shared memory
 // x^H v for w = x - tau/2 (x^H v) v comes from v^H A v and the pairs' products, so that it
 // needs no barrier of its own.
-// Bound: the stream of the leading block (25 matrices of order 2500, clusters of 5: 229 ms for
-// 1.04 TB, 4.5 TB/s; of order 3000 in single precision 224 ms, 4.0 TB/s); 135 ms of the 229
-// remain with the loads taken out.  One CTA per matrix, 25 SMs at work, took 923 and 957 ms.
-template <int NT, class R>
-__global__ void __launch_bounds__(NT, NT > 256 ? 1 : 2)
+// Bound: the stream of the leading block (25 matrices of order 2500, clusters of 5: 215 ms for
+// 1.04 TB, 4.8 TB/s), with the instructions of the product close behind (137 of the 215 ms remain
+// with the loads taken out).  One CTA per matrix, 25 SMs at work, took 923 ms, and 957 at order
+// 3000 in single precision, now 211.
+// ONE: one CTA per matrix, no cluster.
+template <int NT, class R, bool ONE>
+__global__ void __launch_bounds__(NT, NT > 256 ? 1 : 512 / NT)
 k_hetrd_panel_c(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, double* __restrict__ E,
                 typename Cx<R>::T* __restrict__ TAU, typename Cx<R>::T* __restrict__ PV,
-                typename Cx<R>::T* __restrict__ PW, int n, int m, int pw, int P) {
+                typename Cx<R>::T* __restrict__ PW, int n, int m, int pw, int Pr) {
     typedef typename Cx<R>::T C;
     constexpr int NW = NT / 32;
+    const int P = ONE ? 1 : Pr;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* ring = reinterpret_cast<C*>(smem_raw) + (threadIdx.x >> 5) * HU_RING;   // this warp's staging
     C* v = reinterpret_cast<C*>(smem_raw) + NW * HU_RING;   // [m] column / reflector
-    C* pn = v + m;                                // [m] this CTA's part of A v
-    C* coefp = pn + m;                            // [P][2 * HP_W_MAX] the CTAs' parts of w_q^H v, v_q^H v
+    C* pn = v + m + 32;                           // [m] this CTA's part of A v
+    C* coefp = pn + m + 32;                            // [P][2 * HP_W_MAX] the CTAs' parts of w_q^H v, v_q^H v
     C* coef = coefp + (size_t)P * 2 * HP_W_MAX;   // [2 * HP_W_MAX] their sums
     C* rowc = coef + 2 * HP_W_MAX;                // [2 * HP_W_MAX] V_q, W_q at the next column's index
     C* scal_s = rowc + 2 * HP_W_MAX;              // [0..1] alpha by parity, [2] al, [3] w at the next column's index
@@ -2049,7 +2061,7 @@ k_hetrd_panel_c(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, doubl
     R* normp = quadp + (size_t)P * NW;            // [P * NW] parts of the column's norm
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const size_t mat = blockIdx.x / P;
-    const int rank = (int)(blockIdx.x % P);
+    const int rank = ONE ? 0 : (int)(blockIdx.x % P);
     C* a = A + mat * (size_t)n * n;
     double* dd = D + mat * n;
     double* ee = E + mat * n;
@@ -2063,8 +2075,9 @@ k_hetrd_panel_c(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, doubl
     }
     C tau = cz<C>();
     bool act = false;
-    HemvPos pos{};
+    HemvPos<C> pos{};
     int seg = 1;
+    for (int r = m + tid; r < m + 32; r += NT) v[r] = cz<C>();   // (read, times zero, by the product's last blocks)
     for (int j = -1; j < pw; ++j) {
         const int c = m - 1 - j;   // column of step j; the pass below finishes step j and starts step j + 1
         if (j >= 0) {
@@ -2077,11 +2090,12 @@ k_hetrd_panel_c(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, doubl
             C scal;
             reflector(scal_s[j & 1], xn2, beta, tau, scal);
             act = !(tau.x == 0 && tau.y == 0);
+            // (each CTA the whole vector; to memory its own rows)
             for (int r = tid; r < c; r += NT) {
-                C x = r == c - 1 ? cm<C>(1, 0) : act ? cmul(scal, v[r]) : v[r];
+                const C x = r == c - 1 ? cm<C>(1, 0) : act ? cmul(scal, v[r]) : v[r];
                 v[r] = x;
                 pn[r] = cz<C>();
-                if ((r >> 3) % P == rank) {
+                if (ONE) {
                     a[(size_t)c * n + r] = r == c - 1 ? cm<C>(beta, 0) : x;
                     V[(size_t)j * n + r] = x;
                 }
@@ -2097,6 +2111,12 @@ k_hetrd_panel_c(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, doubl
                 wq = __ldcg(W + (size_t)lane * n + c - 1);
             }
             __syncthreads();
+            if (!ONE)
+                for (int r = ((tid >> 3) * P + rank) * 8 + (tid & 7); r < c; r += NT * P) {
+                    const C x = v[r];
+                    a[(size_t)c * n + r] = r == c - 1 ? cm<C>(beta, 0) : x;
+                    V[(size_t)j * n + r] = x;
+                }
             R quad = 0;
             if (act) quad = hemv_units<C, R>(a, n, c, v, pn, pos, P * NW, seg, ring);
             else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -2106,11 +2126,8 @@ k_hetrd_panel_c(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, doubl
             for (int t2 = warp; t2 < 2 * j; t2 += NW) {
                 const C* y = ((t2 & 1) ? V : W) + (size_t)(t2 >> 1) * n;
                 C sd = cz<C>();
-                for (int i = lane;; i += 32) {
-                    const int r = ((i >> 3) * P + rank) * 8 + (i & 7);
-                    if (r >= c) break;
-                    cfmac(sd, y[r], v[r]);
-                }
+#pragma unroll 2
+                for (int r = ((lane >> 3) * P + rank) * 8 + (lane & 7); r < c; r += 32 * P) cfmac(sd, y[r], v[r]);
                 sd = warp_sum(sd);
                 if (lane < P) panel_peer(coefp, lane, P)[rank * 2 * HP_W_MAX + t2] = sd;
             }
@@ -2171,9 +2188,11 @@ k_hetrd_panel_c(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, doubl
                 if (j >= 0) {
                     for (int k = ql; k < P; k += 4) y = cadd(y, panel_peer(pn, k, P)[r]);
                     C s1 = cz<C>();
+                    const C *vq = V + (size_t)ql * n + r, *wq = W + (size_t)ql * n + r;
+                    const size_t step = (size_t)4 * n;
 #pragma unroll 2
-                    for (int q = ql; q < j; q += 4) {
-                        const C vr = V[(size_t)q * n + r], wr = W[(size_t)q * n + r];
+                    for (int q = ql; q < j; q += 4, vq += step, wq += step) {
+                        const C vr = *vq, wr = *wq;
                         cfma(s1, vr, coef[2 * q]);
                         cfma(s1, wr, coef[2 * q + 1]);
                         cfma(s2, vr, cconj(rowc[2 * q + 1]));
@@ -2239,7 +2258,7 @@ static cudaLaunchConfig_t panel_c_config(cudaLaunchAttribute* at, cudaStream_t s
 }
 template <int NT, class R>
 static cudaError_t panel_c_attrs(int m, int P) {
-    auto kern = k_hetrd_panel_c<NT, R>;
+    auto kern = k_hetrd_panel_c<NT, R, false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)panel_c_smem<NT, R>(m, P));
     if (e == cudaSuccess && P > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
@@ -2251,7 +2270,7 @@ static cudaError_t launch_panel_c(cudaStream_t st, typename Cx<R>::T* A, double*
     if (e != cudaSuccess) return e;
     cudaLaunchAttribute at[1];
     const cudaLaunchConfig_t cfg = panel_c_config<NT, R>(at, st, m, nb, P);
-    return cudaLaunchKernelEx(&cfg, k_hetrd_panel_c<NT, R>, A, D, E, TAU, PV, PW, n, m, pw, P);
+    return cudaLaunchKernelEx(&cfg, k_hetrd_panel_c<NT, R, false>, A, D, E, TAU, PV, PW, n, m, pw, P);
 }
 
 // Shape of the cluster panel for a chunk of nb matrices, P = 0 where one CTA per matrix (or the
@@ -2261,7 +2280,7 @@ static cudaError_t launch_panel_c(cudaStream_t st, typename Cx<R>::T* A, double*
 // if that is at least 1.5 (below order 512: 2) times the 512 threads of one CTA per matrix:
 // panels of order 300, double precision, 18 matrices 3.46 -> 2.63 ms, 36 3.47 -> 2.86, but 81
 // 3.49 -> 3.71; of order 512 10.9 -> 5.9, 11.3 -> 6.9, 13.1 -> 10.9; of order 2500, 25 matrices,
-// 923 -> 229.
+// 923 -> 215.
 struct PanelShape {
     int nt, P;
 };
@@ -2274,7 +2293,7 @@ static void panel_shape_try(int m, int nb, PanelShape* best) {
         cudaLaunchAttribute at[1];
         const cudaLaunchConfig_t cfg = panel_c_config<NT, R>(at, 0, m, nb, P);
         if (panel_c_attrs<NT, R>(m, P) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&active, k_hetrd_panel_c<NT, R>, &cfg) != cudaSuccess) {
+            cudaOccupancyMaxActiveClusters(&active, k_hetrd_panel_c<NT, R, false>, &cfg) != cudaSuccess) {
             cudaGetLastError();
             continue;
         }
@@ -2290,6 +2309,57 @@ static PanelShape panel_shape(int m, int nb) {
     panel_shape_try<256, R>(m, nb, &s);
     if (s.nt * s.P < (m >= 512 ? 768 : 1024)) s.P = 0;
     return s;
+}
+
+// One CTA per matrix (k_hetrd_panel_c without a cluster): 512 threads, or 256 or 128 with two
+// or four CTAs per SM, which between them keep the SM busier through each other's chains of
+// small steps.  A wave of 148 k matrices takes about 1, 1.8 and 3.4 units of time for k = 1, 2
+// and 4 (orders 256 to 640), the last one of several counts in part.  Panels in double
+// precision, against a kernel with one row and 8 columns per lane and seven barriers per column:
+// order 256, 592 matrices 9.64 -> 8.00 ms (128 threads), order 512, 592 matrices 51.3 -> 45.2
+// (128), 296 matrices 25.8 -> 23.8 (256), order 1000, 100 matrices 78.4 -> 63.6 (512); in
+// single precision order 256 7.59 -> 5.15, order 512 37.8 -> 28.9.
+// Returns the threads (64 serve the orders whose vectors leave a ring for no more warps), 0 if
+// none fits.  pinned: 512 or 256, or the next smaller that fits; 0: the rule.
+template <class R>
+static int panel_threads(int m, int nb, int pinned) {
+    const size_t smem[4] = {panel_c_smem<512, R>(m, 1), panel_c_smem<256, R>(m, 1), panel_c_smem<128, R>(m, 1),
+                            panel_c_smem<64, R>(m, 1)};
+    const double unit[3] = {1.0, 1.8, 3.4};
+    int best = 0;
+    double best_cost = 0.0;
+    for (int i = 0; i < 3; ++i) {
+        const int nt = 512 >> i, per_sm = (int)std::min<size_t>((size_t)1 << i, (size_t)(228 * 1024) / (smem[i] + 1024));
+        if (per_sm < 1 || smem[i] > 227 * 1024 || (pinned && nt > pinned)) continue;
+        if (pinned) return nt;
+        const double waves = (double)nb / (148.0 * per_sm);
+        const double cost = (per_sm == 1 << i ? unit[i] : unit[i] / (1 << i) * per_sm * 1.3) * (waves <= 1.0 ? 1.0 : waves + 0.35);
+        if (best == 0 || cost < best_cost) {
+            best = nt;
+            best_cost = cost;
+        }
+    }
+    return best ? best : smem[3] <= 227 * 1024 ? 64 : 0;
+}
+// One CTA per matrix rather than the panel queue for more matrices than SMs: where two 256-thread
+// CTAs fit an SM (order 1200 at most, above which the queue is even) and their waves of 296 are
+// at least 80 % full (a single wave always).  Order 600, 592 matrices 101.6 -> 73.5 ms, 200
+// 34.5 -> 31.6; order 1000, 296 matrices 180.2 -> 144.8, 200 122.6 -> 116.5; but order 800, 300
+// matrices 102.5 -> 113.7.
+template <class R>
+static bool panel_waves_full(int m, int nb) {
+    const int waves = (nb + 295) / 296;
+    return m <= 1200 && panel_c_smem<256, R>(m, 1) <= 113 * 1024 && (waves == 1 || nb >= 0.8 * 296 * waves);
+}
+template <int NT, class R>
+static cudaError_t launch_panel_one(cudaStream_t st, typename Cx<R>::T* A, double* D, double* E, typename Cx<R>::T* TAU,
+                                    typename Cx<R>::T* PV, typename Cx<R>::T* PW, int n, int m, int pw, int nb) {
+    auto kern = k_hetrd_panel_c<NT, R, true>;
+    const size_t smem = panel_c_smem<NT, R>(m, 1);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    kern<<<nb, NT, smem, st>>>(A, D, E, TAU, PV, PW, n, m, pw, 1);
+    return cudaGetLastError();
 }
 
 // [V | W] (r, k) and [W | V]^H (k, c) of a panel: the operands of A -= V W^H + W V^H.
@@ -2901,6 +2971,7 @@ struct HeevPlan {
     int pw;               // panel width, 16 or 32
     int panel_nt, xtile;  // tuned launch choices (0: built-in)
     int queue_nt;         // threads of the panel queue's CTAs (512: one per SM, 256: two per SM)
+    bool queue_pinned;    // set by the caller: the queue wherever it applies
     // per: bytes per matrix of the chunk's regions (offsets off_*, times the chunk size);
     // per2: bytes per matrix of the mixed mode's refinement regions (Res, X1), which the
     // refinement uses for one sub-chunk of matrices at a time
@@ -2914,6 +2985,7 @@ static HeevPlan heev_plan(int n, bool mixed, int refine_steps = 2, int band = -1
     p.panel_nt = tune.panel_nt;
     p.xtile = tune.xtile;
     p.queue_nt = tune.queue_nt ? tune.queue_nt : QUEUE_NT_DEFAULT;
+    p.queue_pinned = tune.queue_nt != 0;
     p.n = n;
     p.mixed = mixed;
     p.band = band >= 0 && 32 + 2 * band <= n ? band : -1;   // the band residual needs 32 + 2o <= n
@@ -3025,7 +3097,7 @@ size_t heev_max_chunk(int n) {
         if (ctx) prof_begin(ctx, name); \
     } while (0)
 
-// Householder tridiagonalisation in the working precision R: blocked panels (k_hetrd_panel +
+// Householder tridiagonalisation in the working precision R: blocked panels (k_hetrd_panel_c +
 // rank-2*pw GEMM update) down to order m_tail, then k_hetrd on the leading block.  PV holds
 // the panel pairs of the chunk (V of every matrix, then W of every matrix).
 template <class R>
@@ -3041,31 +3113,26 @@ static int tridiagonalise(rlmb_context* ctx, cudaStream_t st, const HeevPlan& p,
         int dev = 0, sms = 148;
         if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
             return RLMB_ERR_CUDA;
-        // built-in choice above order 512 for chunks of more matrices than SMs: one 512-thread
-        // CTA per SM taking (matrix, column) units from a queue (k_hetrd_panel_q)
+        // above order 512, chunks of more matrices than SMs: one 512-thread CTA per SM taking
+        // (matrix, column) units from a queue (k_hetrd_panel_q), built in where one CTA per matrix
+        // would leave its last wave mostly empty (panel_waves_full)
         const int qnt = p.queue_nt == 256 ? 256 : 512;
         const int qper = qnt == 256 ? 2 : 1;   // resident queue CTAs per SM
-        const bool queue = p.panel_nt == 0 && n > 512 && nb > sms &&
+        const bool queue = p.panel_nt == 0 && n > 512 && nb > sms && (p.queue_pinned || !panel_waves_full<R>(n, nb)) &&
                            (qnt == 512 ? panel_smem<512, R>(n) <= 227 * 1024 : panel_smem<256, R>(n) <= 113 * 1024);
-        // otherwise one CTA per matrix: 256 threads (two CTAs per SM) for orders 385..512,
-        // 512 threads otherwise (measured), unless tuned
-        bool mid = n > 384 && n <= 512;
-        if (p.panel_nt == 256 && panel_smem<256, R>(n) <= 113 * 1024) mid = true;
-        if (p.panel_nt == 512) mid = false;
-        auto panel = mid ? k_hetrd_panel<256, R> : k_hetrd_panel<512, R>;
-        const int pnt = mid ? 256 : 512;
-        const size_t smem = queue ? (qnt == 256 ? panel_smem<256, R>(n) : panel_smem<512, R>(n))
-                                  : mid ? panel_smem<256, R>(n) : panel_smem<512, R>(n);
-        const void* qk = qnt == 256 ? (const void*)k_hetrd_panel_q<256, R> : (const void*)k_hetrd_panel_q<512, R>;
-        if (cudaFuncSetAttribute(queue ? qk : (const void*)panel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem) != cudaSuccess)
-            return RLMB_ERR_CUDA;
-        const int grid = std::min(nb, queue ? qper * sms : sms);
+        if (queue) {
+            const void* qk = qnt == 256 ? (const void*)k_hetrd_panel_q<256, R> : (const void*)k_hetrd_panel_q<512, R>;
+            const size_t smem = qnt == 256 ? panel_smem<256, R>(n) : panel_smem<512, R>(n);
+            if (cudaFuncSetAttribute(qk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+                return RLMB_ERR_CUDA;
+        }
+        const int grid = std::min(nb, qper * sms);
         // the queue's counters, and its abort flag, which k_panel_abort_info reads in every case
         if (cudaMemsetAsync(Q, 0, (8 + (size_t)nb) * sizeof(int), st) != cudaSuccess) return RLMB_ERR_CUDA;
-        // chunks of few matrices: a cluster of CTAs per matrix (k_hetrd_panel_c)
+        // chunks of few matrices: a cluster of CTAs per matrix; otherwise one CTA per matrix,
+        // with the pinned number of threads if there is one
         PanelShape shape{};
-        if (p.panel_nt == 0) shape = panel_shape<R>(n, nb);
+        if (p.panel_nt == 0 && !queue) shape = panel_shape<R>(n, nb);
         for (int k = 0; k < p.npanels; ++k) {
             RLMB_CHUNK_PROF("k_hetrd_panel");
             if (shape.P > 0) {
@@ -3076,16 +3143,18 @@ static int tridiagonalise(rlmb_context* ctx, cudaStream_t st, const HeevPlan& p,
                 const auto launch = shape.nt == 512 ? launch_panel_c<512, R>
                                   : shape.nt == 384 ? launch_panel_c<384, R> : launch_panel_c<256, R>;
                 if (launch(st, A, D, E, TAU, PV, PWb, n, m, pw, nb, shape.P) != cudaSuccess) return RLMB_ERR_CUDA;
-            } else if (queue && qnt == 256)
-                k_hetrd_panel_q<256, R><<<grid, 256, smem, st>>>(A, D, E, TAU, PV, PWb, n, m, pw, nb, Q,
-                                                                 (long long)k * ((long long)nb * pw + grid),
-                                                                 k * pw, info);
-            else if (queue)
-                k_hetrd_panel_q<512, R><<<grid, 512, smem, st>>>(A, D, E, TAU, PV, PWb, n, m, pw, nb, Q,
-                                                                 (long long)k * ((long long)nb * pw + grid),
-                                                                 k * pw, info);
-            else
-                panel<<<nb, pnt, smem, st>>>(A, D, E, TAU, PV, PWb, n, m, pw);
+            } else if (queue && qnt == 256) {
+                k_hetrd_panel_q<256, R><<<grid, 256, panel_smem<256, R>(n), st>>>(
+                    A, D, E, TAU, PV, PWb, n, m, pw, nb, Q, (long long)k * ((long long)nb * pw + grid), k * pw, info);
+            } else if (queue) {
+                k_hetrd_panel_q<512, R><<<grid, 512, panel_smem<512, R>(n), st>>>(
+                    A, D, E, TAU, PV, PWb, n, m, pw, nb, Q, (long long)k * ((long long)nb * pw + grid), k * pw, info);
+            } else {
+                const int nt = panel_threads<R>(m, nb, p.panel_nt);
+                const auto launch = nt == 512 ? launch_panel_one<512, R> : nt == 256 ? launch_panel_one<256, R>
+                                  : nt == 128 ? launch_panel_one<128, R> : launch_panel_one<64, R>;
+                if (nt == 0 || launch(st, A, D, E, TAU, PV, PWb, n, m, pw, nb) != cudaSuccess) return RLMB_ERR_CUDA;
+            }
             RLMB_CHUNK_LAUNCHED();
             m -= pw;
             RLMB_CHUNK_PROF("k_hetrd_her2k");
@@ -3497,7 +3566,7 @@ void rlmb::tune_free(rlmb_context* ctx) {
     ctx->tune = nullptr;
 }
 
-static std::vector<HeevTune> tune_candidates(int n, bool mixed, int nb) {
+static std::vector<HeevTune> tune_candidates(int n, bool mixed) {
     std::vector<HeevTune> out;
     if (n <= JAC_MAX_N) {
         HeevTune t;
@@ -3507,10 +3576,8 @@ static std::vector<HeevTune> tune_candidates(int n, bool mixed, int nb) {
     for (int blocked = 0; blocked <= 1; ++blocked) {
         if (blocked && n < 128) continue;
         for (int gemm = 0; gemm <= 1; ++gemm)
-            for (int nt : {0, 256, 512}) {
+            for (int nt : {0, 512}) {   // panels by the rules, or 512 threads per matrix
                 if (!blocked && nt != 512) continue;   // no panels: one entry
-                // the built-in panels where they are clusters (few matrices)
-                if (nt == 0 && (mixed ? panel_shape<float>(n, nb) : panel_shape<double>(n, nb)).P == 0) continue;
                 for (int xt : {64, 128})
                     for (int bs : {64, 128}) {
                         if ((!gemm || mixed) && xt == 128) continue;
@@ -3542,7 +3609,7 @@ static int autotune(rlmb_context* ctx, int n, bool mixed, int refine_steps, int 
     const size_t nn = (size_t)n * n;
     const size_t cap = std::min<size_t>((size_t)2 * sms, ((size_t)2 << 30) / (nn * sizeof(cplx)));
     const int tb = (int)std::max<size_t>(1, std::min<size_t>((size_t)batch, cap));
-    const std::vector<HeevTune> cands = tune_candidates(n, mixed, tb);
+    const std::vector<HeevTune> cands = tune_candidates(n, mixed);
     size_t per = 0;
     for (const HeevTune& t : cands) {
         const HeevPlan pl = heev_plan(n, mixed, refine_steps, band, t);

@@ -1,7 +1,7 @@
 """The reduction's panels by a cluster of CTAs per matrix (few matrices of order >= 256), against
 LAPACK eigenvalues and the eigenvectors' residual and orthogonality: orders off the 16-column
 strips and 32-row blocks, both panel widths, one matrix (16 CTAs) up to the chunk sizes where the
-cluster shrinks to two CTAs, inactive reflectors."""
+cluster shrinks to two CTAs, inactive reflectors; and by one CTA per matrix in chunks of more."""
 import numpy as np
 import pytest
 
@@ -29,7 +29,10 @@ def _matrices(kind, n, batch, seed):
 @pytest.mark.parametrize("kind,n,batch", [("random", 256, 1), ("random", 257, 18), ("random", 273, 5),
                                           ("random", 300, 36), ("random", 511, 74), ("random", 513, 26),
                                           ("random", 1031, 9), ("random", 1500, 2), ("diagonal", 260, 3),
-                                          ("blocks", 301, 4), ("blocks", 1060, 2)])
+                                          ("blocks", 301, 4), ("blocks", 1060, 2),
+                                          # one CTA per matrix: 512, 256 and 128 threads
+                                          ("random", 258, 100), ("random", 256, 150), ("blocks", 261, 297),
+                                          ("random", 257, 600), ("random", 520, 160)])
 def test_cluster_panels(kind, n, batch, mixed):
     import torch
 
