@@ -363,100 +363,108 @@ k_hetrd(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, double* __res
 }
 
 // ------------------------------------------------------------ k_tridiag
-// Eigen-decomposition of the real symmetric tridiagonal (d, e), one CTA per matrix.
-// Eigenvalues by bisection; eigenvector k by inverse iteration, stored row-major in
-// Z (Z[j*n + k] = component j of eigenvector k) so that the recurrences of the n
-// threads touch consecutive addresses.  Per-thread LU factors live in the interleaved
-// workspace lu (5*n*n doubles per matrix, same layout).
+// Eigen-decomposition of the real symmetric tridiagonal (d, e), scaled by a power of two to unit
+// norm.  A CTA of T threads takes up to T eigenvalues of one matrix at a time (T: the order
+// rounded up to a warp, at most TRI_THREADS); eigenvalues in k_tridiag<1, T>, eigenvectors in
+// k_tridiag<2, T>, stored row-major in Z (Z[j*n + k] = component j of eigenvector k) so that the
+// recurrences of the threads touch consecutive addresses.  Per-thread scratch columns live in
+// the interleaved workspace LU (5 * n * tri_columns(n) doubles per matrix, same layout).
+// Bound: instruction issue in phase 1 (the counts), the latency of the scratch columns in phase
+// 2.  With 256 threads whatever the order, range and sign tests on the FP64 pipe in every step
+// and vectors walked from thread-dependent indices (uncoalesced) the phases took 9.7 and 12.4 ms
+// on 4,224 matrices of order 256, 0.74 and 0.70 on 4,624 of order 64, 1.16 and 0.54 on 18 of
+// order 300; now 5.7 and 5.4, 0.42 and 0.22, 0.34 and 0.18.
 static constexpr int TRI_THREADS = 256;
 static constexpr int INV_MAXITS = 5;
+// scratch columns per matrix: one per eigenvector up to order 384 (a chunk of few matrices then
+// spreads a matrix over two CTAs), else one per thread of one CTA
+__host__ __device__ constexpr int tri_columns(int n) { return n <= 384 ? (n + 31) / 32 * 32 : TRI_THREADS; }
 
-__device__ int sturm_count(const double* __restrict__ d, const double* __restrict__ e2, int n,
-                           double x, double pivmin) {
-    double q = d[0] - x;
-    if (fabs(q) <= pivmin) q = -pivmin;
-    int cnt = q < 0.0;
-    for (int j = 1; j < n; ++j) {
-        q = d[j] - x - e2[j - 1] / q;
-        if (fabs(q) <= pivmin) q = -pivmin;
-        cnt += q < 0.0;
-    }
-    return cnt;
+// Sturm count by the leading principal minors of T - x I,
+//   p_j = (d_j - x) p_{j-1} - e_{j-1}^2 p_{j-2},   p_{-1} = 1:
+// the number of sign changes along p_{-1}, p_0, ..., p_{n-1} is the number of eigenvalues below
+// x (Sturm); a zero minor counts as a change.  The pair (p_j, p_{j-1}) is kept in range by exact
+// powers of two, every fourth step (|T| is about 1, so four steps grow it by less than 2^12);
+// signs, zeros and exponents are looked at as integers, which leaves the FP64 pipe the
+// recurrences.  The derivatives p_j' ride along for the Newton step ratio = p_{n-1}/p_{n-1}'.
+static constexpr int STURM_BIG = (1023 + 400) << 20, STURM_SMALL = (1023 - 400) << 20;
+__device__ __forceinline__ double sturm_nonzero(double pn, double p) {
+    const int hi = __double2hiint(pn), lo = __double2loint(pn);
+    // a zero becomes 2^-700 of the sign opposite to p's
+    return ((hi << 1) | lo) == 0 ? __hiloint2double((~__double2hiint(p) & 0x80000000) | ((1023 - 700) << 20), 0) : pn;
 }
-
-// Division-free Sturm count: the leading principal minors p_j of T - x I obey
-//   p_j = (d_j - x) p_{j-1} - e_{j-1}^2 p_{j-2},   p_{-1} = 1,
-// and the number of sign changes along p_{-1}, p_0, ..., p_{n-1} is the number of
-// eigenvalues below x (Sturm).  The pair (p_j, p_{j-1}) is rescaled by exact powers of two
-// to stay in range; a minor that is tiny relative to its predecessor is replaced by
-// -pivmin * p_{j-1}, the same substitution the pivot form q_j = p_j / p_{j-1} uses
-// (dstebz).  The derivatives p_j' ride along for the Newton step ratio = p_{n-1}/p_{n-1}'.
+__device__ __forceinline__ int sturm_change(double a, double b) {
+    return (int)((unsigned)(__double2hiint(a) ^ __double2hiint(b)) >> 31);
+}
+// 2^-k for the larger of the two, if that is out of range (else 1)
+__device__ __forceinline__ bool sturm_range(double p, double pm, double& sc) {
+    const int m = max(__double2hiint(p) & 0x7fffffff, __double2hiint(pm) & 0x7fffffff);
+    if (m <= STURM_BIG && m >= STURM_SMALL) return false;
+    sc = __hiloint2double((1023 - min((m >> 20) - 1023, 1000)) << 20, 0);
+    return true;
+}
 __device__ __forceinline__ int sturm_poly(const double* __restrict__ d, const double* __restrict__ e2, int n,
-                                          double x, double pivmin, double& ratio) {
-    double pm = 1.0, p = d[0] - x;       // p_{j-1}, p_j
-    double dpm = 0.0, dp = -1.0;          // their derivatives in x
-    if (fabs(p) <= pivmin) p = -pivmin;
-    int cnt = p < 0.0;
-    for (int j = 1; j < n; ++j) {
-        const double a = d[j] - x;
-        double pn = fma(a, p, -e2[j - 1] * pm);
-        double dpn = fma(a, dp, -fma(e2[j - 1], dpm, p));
-        if (fabs(pn) <= pivmin * fabs(p)) pn = -pivmin * p;
-        cnt += (pn < 0.0) != (p < 0.0);
+                                          double x, double& ratio) {
+    double pm = 1.0, p = sturm_nonzero(d[0] - x, 1.0);   // p_{j-1}, p_j
+    double dpm = 0.0, dp = -1.0;                          // their derivatives in x
+    int cnt = sturm_change(p, 1.0);
+    auto step = [&](int j) {
+        const double a = d[j] - x, ee = e2[j - 1];
+        const double pn = sturm_nonzero(fma(a, p, -ee * pm), p);
+        const double dpn = fma(a, dp, -fma(ee, dpm, p));
+        cnt += sturm_change(pn, p);
         pm = p;
         dpm = dp;
         p = pn;
         dp = dpn;
-        const double big = fmax(fabs(p), fabs(pm));
-        if (big > 0x1p+400 || big < 0x1p-400) {
-            int ex;
-            frexp(big, &ex);
-            const double sc = ldexp(1.0, min(max(-ex, -1000), 1000));   // a denormal pair: no overflow
+    };
+    int j = 1;
+    for (; j + 4 <= n; j += 4) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) step(j + u);
+        double sc;
+        if (sturm_range(p, pm, sc)) {
             p *= sc;
             pm *= sc;
             dp *= sc;
             dpm *= sc;
         }
     }
+    for (; j < n; ++j) step(j);
     ratio = p / dp;
     return cnt;
 }
-
-// The counts of sturm_poly at two shifts, the two recurrences interleaved (no derivatives).
+// The counts at two shifts, the two recurrences interleaved (no derivatives).
 __device__ __forceinline__ void sturm_count2(const double* __restrict__ d, const double* __restrict__ e2, int n,
-                                             double xa, double xb, double pivmin, int& ca, int& cb) {
-    double pma = 1.0, pa = d[0] - xa, pmb = 1.0, pb = d[0] - xb;
-    if (fabs(pa) <= pivmin) pa = -pivmin;
-    if (fabs(pb) <= pivmin) pb = -pivmin;
-    int na = pa < 0.0, nb = pb < 0.0;
-    for (int j = 1; j < n; ++j) {
+                                             double xa, double xb, int& ca, int& cb) {
+    double pma = 1.0, pa = sturm_nonzero(d[0] - xa, 1.0), pmb = 1.0, pb = sturm_nonzero(d[0] - xb, 1.0);
+    int na = sturm_change(pa, 1.0), nb = sturm_change(pb, 1.0);
+    auto step = [&](int j) {
         const double ee = e2[j - 1], dj = d[j];
-        double qa = fma(dj - xa, pa, -ee * pma);
-        double qb = fma(dj - xb, pb, -ee * pmb);
-        if (fabs(qa) <= pivmin * fabs(pa)) qa = -pivmin * pa;
-        if (fabs(qb) <= pivmin * fabs(pb)) qb = -pivmin * pb;
-        na += (qa < 0.0) != (pa < 0.0);
-        nb += (qb < 0.0) != (pb < 0.0);
+        const double qa = sturm_nonzero(fma(dj - xa, pa, -ee * pma), pa);
+        const double qb = sturm_nonzero(fma(dj - xb, pb, -ee * pmb), pb);
+        na += sturm_change(qa, pa);
+        nb += sturm_change(qb, pb);
         pma = pa;
         pa = qa;
         pmb = pb;
         pb = qb;
-        const double biga = fmax(fabs(pa), fabs(pma)), bigb = fmax(fabs(pb), fabs(pmb));
-        if (biga > 0x1p+400 || biga < 0x1p-400) {
-            int ex;
-            frexp(biga, &ex);
-            const double sc = ldexp(1.0, min(max(-ex, -1000), 1000));   // a denormal pair: no overflow
+    };
+    int j = 1;
+    for (; j + 4 <= n; j += 4) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) step(j + u);
+        double sc;
+        if (sturm_range(pa, pma, sc)) {
             pa *= sc;
             pma *= sc;
         }
-        if (bigb > 0x1p+400 || bigb < 0x1p-400) {
-            int ex;
-            frexp(bigb, &ex);
-            const double sc = ldexp(1.0, min(max(-ex, -1000), 1000));   // a denormal pair: no overflow
+        if (sturm_range(pb, pmb, sc)) {
             pb *= sc;
             pmb *= sc;
         }
     }
+    for (; j < n; ++j) step(j);
     ca = na;
     cb = nb;
 }
@@ -475,63 +483,122 @@ __device__ __forceinline__ double start_entry(int k, int j) {
 // Eigenvector of an isolated eigenvalue x of (d, e) by the twisted factorisation of
 // T - x I (Parlett & Dhillon): forward pivots D+ (the Sturm recurrence) and backward
 // pivots D-, twist index r minimising |gamma_r| = |D+_r + D-_r - (d_r - x)|, then
-// z_r = 1, z_j = -e_j z_{j+1} / D+_j (j < r), z_j = -e_{j-1} z_{j-1} / D-_j (j > r).
-// D+ and D- go to their own scratch columns so the final recurrences can prefetch them.
-__device__ void twisted_vector(const double* __restrict__ d, const double* __restrict__ e,
-                               const double* __restrict__ e2, int n, double x, double pivmin,
-                               double* __restrict__ z, int k, double* __restrict__ dplus,
-                               double* __restrict__ dminus, int sc) {
-    // D+ (forward, stationary) and D- (backward, progressive) are independent division
-    // chains: one loop advances both, j forward and n-1-j backward
-    double q = d[0] - x;
-    if (fabs(q) <= pivmin) q = -pivmin;
-    dplus[sc] = q;
-    double qb = d[n - 1] - x;
-    if (fabs(qb) <= pivmin) qb = -pivmin;
-    dminus[(size_t)(n - 1) * TRI_THREADS + sc] = qb;
-    for (int j = 1; j < n; ++j) {
-        q = d[j] - x - e2[j - 1] / q;
-        if (fabs(q) <= pivmin) q = -pivmin;
-        dplus[(size_t)j * TRI_THREADS + sc] = q;
-        const int jb = n - 1 - j;
-        double qn = (d[jb] - x) - e2[jb] / qb;
-        if (fabs(qn) <= pivmin) qn = -pivmin;
-        qb = qn;
-        dminus[(size_t)jb * TRI_THREADS + sc] = qb;
+// z_r = 1, z_j = L_j z_{j+1} (j < r), z_j = M_j z_{j-1} (j > r) with the multipliers
+// L_j = -e_j / D+_j and M_j = -e_{j-1} / D-_j.
+// The multipliers, not the pivots, go to the thread's scratch columns lp and lm (stride `ls`), so
+// that only the factorisation divides.  Every loop runs over the same j in all threads -- the
+// parts of z beside the twist start at thread-dependent indices, but are walked from the ends
+// with the value held at 1 until the twist is reached -- so that a warp's accesses stay
+// coalesced, and loads are issued eight steps ahead of their use.
+static constexpr int TW_AHEAD = 8;
+__device__ void twisted_vector(const double* __restrict__ d, const double* __restrict__ e, int n, double x,
+                               double pivmin, double* __restrict__ z, int k, double* __restrict__ lp,
+                               double* __restrict__ lm, int ls) {
+    if (n == 1) {
+        z[k] = 1.0;
+        return;
     }
-    // twist index r = argmin |gamma_j|, gamma_j = D+_j + D-_j - (d_j - x), gamma_{n-1} = D+_{n-1}
-    int r = n - 1;
-    double gbest = fabs(q);
-    for (int j = n - 2; j >= 0; --j) {
-        const double gam = fabs(dplus[(size_t)j * TRI_THREADS + sc] + dminus[(size_t)j * TRI_THREADS + sc] - (d[j] - x));
+    auto pivot = [&](double q) { return fabs(q) <= pivmin ? -pivmin : q; };
+    // D+ (forward, stationary) and D- (backward, progressive) are independent division
+    // chains: one loop advances both, step t forward to t + 1 and backward to n - 2 - t
+    double qf = pivot(d[0] - x), qb = pivot(d[n - 1] - x);
+    auto advance = [&](int t) {
+        const int jb = n - 1 - t;
+        const double l = -e[t] / qf, m = -e[jb - 1] / qb;
+        lp[(size_t)t * ls] = l;
+        lm[(size_t)jb * ls] = m;
+        qf = pivot(fma(e[t], l, d[t + 1] - x));
+        qb = pivot(fma(e[jb - 1], m, d[jb - 1] - x));
+    };
+    int r = 0;
+    double gbest = DBL_MAX;
+    auto twist = [&](int j, double gam) {
+        gam = fabs(gam);
         if (gam < gbest) {
             gbest = gam;
             r = j;
         }
+    };
+    // until the chains have met: after step t0 - 1, D+ is at t0 and D- at n - 1 - t0
+    const int t0 = n / 2;
+    for (int t = 0; t < t0; ++t) advance(t);
+    if (n & 1) twist(t0, qf + qb - (d[t0] - x));
+    else {   // D+ is at n/2, D- at n/2 - 1: their other halves are the last multipliers
+        twist(t0, t0 + 1 < n ? fma(e[t0], lm[(size_t)(t0 + 1) * ls], qf) : qf);
+        twist(t0 - 1, t0 >= 2 ? fma(e[t0 - 2], lp[(size_t)(t0 - 2) * ls], qb) : qb);
     }
-    double zz = 1.0, nrm2 = 1.0, big = 1.0;
-    for (int j = r - 1; j >= 0; --j) {
-        zz = -e[j] * zz / dplus[(size_t)j * TRI_THREADS + sc];
-        z[(size_t)j * n + k] = zz;
-        nrm2 += zz * zz;
-        if (fabs(zz) > fabs(big)) big = zz;
+    // beyond: gamma_j = D+_j + e_j M_{j+1} and D-_j + e_{j-1} L_{j-1}, from multipliers stored
+    // by the other chain
+    for (int t = t0; t < n - 1; t += TW_AHEAD) {
+        double am[TW_AHEAD], ap[TW_AHEAD];
+#pragma unroll
+        for (int u = 0; u < TW_AHEAD; ++u) {
+            const int jf = t + u + 1, jb = n - 2 - t - u;   // D+_jf, D-_jb after step t + u
+            am[u] = jf + 1 < n ? lm[(size_t)(jf + 1) * ls] : 0.0;
+            ap[u] = jb >= 1 ? lp[(size_t)(jb - 1) * ls] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < TW_AHEAD; ++u) {
+            if (t + u >= n - 1) break;
+            advance(t + u);
+            const int jf = t + u + 1, jb = n - 2 - t - u;
+            twist(jf, jf + 1 < n ? fma(e[jf], am[u], qf) : qf);
+            twist(jb, jb >= 1 ? fma(e[jb - 1], ap[u], qb) : qb);
+        }
     }
-    z[(size_t)r * n + k] = 1.0;
-    zz = 1.0;
-    for (int j = r + 1; j < n; ++j) {
-        zz = -e[j - 1] * zz / dminus[(size_t)j * TRI_THREADS + sc];
-        z[(size_t)j * n + k] = zz;
-        nrm2 += zz * zz;
-        if (fabs(zz) > fabs(big)) big = zz;
-    }
-    double rn = 1.0 / sqrt(nrm2);
+    // z from the twist outwards; WRITE: times scale, to memory
+    double nrm2 = 1.0, big = 1.0, rn = 1.0;
+    auto walk = [&](auto write) {
+        double zz = rn;
+        for (int j0 = n - 2; j0 >= 0; j0 -= TW_AHEAD) {   // j = r - 1 .. 0
+            double l[TW_AHEAD];
+#pragma unroll
+            for (int u = 0; u < TW_AHEAD; ++u) l[u] = j0 - u >= 0 ? lp[(size_t)(j0 - u) * ls] : 0.0;
+#pragma unroll
+            for (int u = 0; u < TW_AHEAD; ++u) {
+                const int j = j0 - u;
+                if (j >= 0 && j < r) {
+                    zz *= l[u];
+                    if constexpr (decltype(write)::value) {
+                        z[(size_t)j * n + k] = zz;
+                    } else {
+                        nrm2 = fma(zz, zz, nrm2);
+                        if (fabs(zz) > fabs(big)) big = zz;
+                    }
+                }
+            }
+        }
+        if constexpr (decltype(write)::value) z[(size_t)r * n + k] = rn;
+        zz = rn;
+        for (int j0 = 1; j0 < n; j0 += TW_AHEAD) {   // j = r + 1 .. n - 1
+            double l[TW_AHEAD];
+#pragma unroll
+            for (int u = 0; u < TW_AHEAD; ++u) l[u] = j0 + u < n ? lm[(size_t)(j0 + u) * ls] : 0.0;
+#pragma unroll
+            for (int u = 0; u < TW_AHEAD; ++u) {
+                const int j = j0 + u;
+                if (j < n && j > r) {
+                    zz *= l[u];
+                    if constexpr (decltype(write)::value) {
+                        z[(size_t)j * n + k] = zz;
+                    } else {
+                        nrm2 = fma(zz, zz, nrm2);
+                        if (fabs(zz) > fabs(big)) big = zz;
+                    }
+                }
+            }
+        }
+    };
+    walk(std::false_type{});
+    rn = 1.0 / sqrt(nrm2);
     if (big < 0.0) rn = -rn;
-    for (int j = 0; j < n; ++j) z[(size_t)j * n + k] *= rn;
+    walk(std::true_type{});
 }
 
 // PHASE 1 (k_stebz): eigenvalues into W.  PHASE 2 (k_stein): eigenvectors from W.
-template <int PHASE>
-__global__ void __launch_bounds__(TRI_THREADS, 2)
+// Grid (matrices, CTAs per matrix); CTA y of Y takes the eigenvalues y, y + Y, ...
+template <int PHASE, int T>
+__global__ void __launch_bounds__(T, 512 / T)
 k_tridiag(const double* __restrict__ D, const double* __restrict__ E, double* __restrict__ W,
           double* __restrict__ Z, double* __restrict__ LU, int* __restrict__ info, int n) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -540,53 +607,62 @@ k_tridiag(const double* __restrict__ D, const double* __restrict__ E, double* __
     double* e2 = e + n;                                 // [n]
     double* lam = e2 + n;                               // [n]
     int* leader = reinterpret_cast<int*>(lam + n);      // [n] first index of k's cluster
-    __shared__ double s_gl, s_gu, s_pivmin, s_onenrm;
+    __shared__ double s_red[4][T / 32];
     __shared__ int s_fail;
     const int tid = threadIdx.x;
     const size_t mat = blockIdx.x;
+    const int sub = blockIdx.y, subs = gridDim.y;
     const size_t nn = (size_t)n * n;
     double* z = Z + mat * nn;
-    // per-thread scratch columns (column = thread, stride TRI_THREADS): U diag / super1 /
-    // super2, multipliers and swap flags of the LU of T - x I; the twisted solve uses the
-    // first two as D+ and D-
-    const size_t lus = (size_t)n * TRI_THREADS;
-    double* la = LU + mat * 5 * lus;
+    // per-thread scratch columns (stride ls): U diag / super1 / super2, multipliers and swap
+    // flags of the LU of T - x I; the twisted solve uses the first two for its multipliers
+    const int ls = tri_columns(n);
+    const size_t lus = (size_t)n * ls;
+    double* la = LU + mat * 5 * lus + sub * ((n + subs - 1) / subs) + tid;
     double* lb = la + lus;
     double* lc2 = lb + lus;
     double* lm = lc2 + lus;
     double* lp = lm + lus;
 
-    for (int j = tid; j < n; j += TRI_THREADS) {
-        d[j] = D[mat * n + j];
+    // Gershgorin interval, one-norm (of the rows), largest |e|
+    double gl = DBL_MAX, gu = -DBL_MAX, onenrm = 0.0, emax = 0.0;
+    for (int j = tid; j < n; j += T) {
+        const double dj = D[mat * n + j];
         const double ej = j < n - 1 ? E[mat * n + j] : 0.0;
+        const double ep = j > 0 ? E[mat * n + j - 1] : 0.0;
+        d[j] = dj;
         e[j] = ej;
-        e2[j] = ej * ej;
+        const double off = fabs(ep) + fabs(ej);
+        gl = fmin(gl, dj - off);
+        gu = fmax(gu, dj + off);
+        onenrm = fmax(onenrm, fabs(dj) + off);
+        emax = fmax(emax, fabs(ej));
+    }
+#pragma unroll
+    for (int m = 16; m >= 1; m >>= 1) {
+        gl = fmin(gl, __shfl_xor_sync(0xffffffffu, gl, m));
+        gu = fmax(gu, __shfl_xor_sync(0xffffffffu, gu, m));
+        onenrm = fmax(onenrm, __shfl_xor_sync(0xffffffffu, onenrm, m));
+        emax = fmax(emax, __shfl_xor_sync(0xffffffffu, emax, m));
+    }
+    if ((tid & 31) == 0) {
+        s_red[0][tid >> 5] = gl;
+        s_red[1][tid >> 5] = gu;
+        s_red[2][tid >> 5] = onenrm;
+        s_red[3][tid >> 5] = emax;
     }
     if (tid == 0) s_fail = 0;
     __syncthreads();
-    if (tid == 0) {
-        double gl = d[0], gu = d[0], emax2 = 0.0, onenrm = 0.0;
-        for (int j = 0; j < n; ++j) {
-            const double off = (j > 0 ? fabs(e[j - 1]) : 0.0) + (j < n - 1 ? fabs(e[j]) : 0.0);
-            gl = fmin(gl, d[j] - off);
-            gu = fmax(gu, d[j] + off);
-            onenrm = fmax(onenrm, fabs(d[j]) + off);
-            if (j < n - 1) emax2 = fmax(emax2, e2[j]);
-        }
-        const double pivmin = DBL_MIN * fmax(1.0, emax2);
-        const double tnorm = fmax(fabs(gl), fabs(gu));
-        gl -= 2.1 * tnorm * DBL_EPSILON * n + 4.2 * pivmin;
-        gu += 2.1 * tnorm * DBL_EPSILON * n + 4.2 * pivmin;
-        s_gl = gl;
-        s_gu = gu;
-        s_pivmin = pivmin;
-        s_onenrm = fmax(onenrm, DBL_MIN);
+#pragma unroll
+    for (int w = 0; w < T / 32; ++w) {
+        gl = fmin(gl, s_red[0][w]);
+        gu = fmax(gu, s_red[1][w]);
+        onenrm = fmax(onenrm, s_red[2][w]);
+        emax = fmax(emax, s_red[3][w]);
     }
-    __syncthreads();
-    const double pivmin = s_pivmin, onenrm = s_onenrm;
     if (!(onenrm > 1e3 * DBL_MIN)) {
         // T = 0 to underflow: eigenvalues are the diagonal (sorted), eigenvectors unit vectors
-        if (PHASE == 2) return;
+        if (PHASE == 2 || sub > 0) return;
         if (tid == 0) {
             for (int k = 0; k < n; ++k) leader[k] = k;
             for (int k = 1; k < n; ++k)
@@ -597,42 +673,60 @@ k_tridiag(const double* __restrict__ D, const double* __restrict__ E, double* __
                 }
         }
         __syncthreads();
-        for (int k = tid; k < n; k += TRI_THREADS) {
+        for (int k = tid; k < n; k += T) {
             W[mat * n + k] = d[leader[k]];
             for (int j = 0; j < n; ++j) z[(size_t)j * n + k] = j == leader[k] ? 1.0 : 0.0;
         }
         if (tid == 0 && info) info[mat] = 0;
         return;
     }
+    // scale T to a one-norm in [1, 2) (exactly; the eigenvalues are scaled back)
+    const int ex = min(max(ilogb(onenrm), -1000), 1000);
+    const double scale = ldexp(1.0, -ex), unscale = ldexp(1.0, ex);
+    gl *= scale;
+    gu *= scale;
+    onenrm *= scale;
+    emax *= scale;
+    for (int j = tid; j < n; j += T) {   // (this thread's own entries)
+        d[j] *= scale;
+        e[j] *= scale;
+        e2[j] = e[j] * e[j];
+    }
+    const double pivmin = DBL_MIN * fmax(1.0, emax * emax);
+    {
+        const double tnorm = fmax(fabs(gl), fabs(gu));
+        gl -= 2.1 * tnorm * DBL_EPSILON * n + 4.2 * pivmin;
+        gu += 2.1 * tnorm * DBL_EPSILON * n + 4.2 * pivmin;
+    }
+    __syncthreads();
     // ---- eigenvalue k: bisection on Sturm counts (dstebz bracketing, restated), accelerated
     //      by safeguarded Newton steps on det(T - x I), taken from the current point or from
     //      either end of the bracket, with the step scaled by the number m of eigenvalues in
     //      the bracket (exact for an m-fold root)
     if (PHASE == 1) {
     const double atol = 2.0 * DBL_EPSILON * onenrm;
-    // one collective pass first: Sturm counts at the TRI_THREADS+1 equally spaced points of
+    // one collective pass first: Sturm counts at the T+1 equally spaced points of
     // the Gershgorin interval (count 0 at its left end, n at its right end), so that every
     // eigenvalue starts from the grid cell holding it instead of the whole interval
-    __shared__ double s_gx[TRI_THREADS + 1];
-    __shared__ int s_gc[TRI_THREADS + 1];
+    __shared__ double s_gx[T + 1];
+    __shared__ int s_gc[T + 1];
     {
-        const double gl = s_gl, gu = s_gu;
         const int t = tid;
-        s_gx[t] = t == 0 ? gl : gl + (gu - gl) * ((double)t / TRI_THREADS);
+        s_gx[t] = t == 0 ? gl : gl + (gu - gl) * ((double)t / T);
         if (t == 0) {
             s_gc[0] = 0;
-            s_gx[TRI_THREADS] = gu;
-            s_gc[TRI_THREADS] = n;
+            s_gx[T] = gu;
+            s_gc[T] = n;
         } else {
             double rr;
-            s_gc[t] = sturm_poly(d, e2, n, s_gx[t], pivmin, rr);
+            s_gc[t] = sturm_poly(d, e2, n, s_gx[t], rr);
         }
     }
     __syncthreads();
-    for (int k = tid; k < n; k += TRI_THREADS) {
+    for (int k = tid * subs + sub; k < n; k += T * subs) {
         int cell = 0;   // largest grid point with count <= k
-        for (int step = TRI_THREADS / 2; step >= 1; step >>= 1)
-            if (cell + step < TRI_THREADS && s_gc[cell + step] <= k) cell += step;
+        for (int step = T / 2; step >= 1; step >>= 1)
+            if (cell + step < T && s_gc[cell + step] <= k) cell += step;
         double lo = s_gx[cell], hi = s_gx[cell + 1];
         int clo = s_gc[cell], chi = s_gc[cell + 1];
         // Newton steps p/p' recorded at the bracket ends (valid flags), bracket widths of the
@@ -644,7 +738,7 @@ k_tridiag(const double* __restrict__ D, const double* __restrict__ E, double* __
         double res = x;
         for (int it = 0; it < 200; ++it) {
             double ratio;
-            const int c = sturm_poly(d, e2, n, x, pivmin, ratio);
+            const int c = sturm_poly(d, e2, n, x, ratio);
             const bool rok = isfinite(ratio);
             if (c > k) { hi = x; chi = c; rhi = ratio; vhi = rok; } else { lo = x; clo = c; rlo = ratio; vlo = rok; }
             const double tol = fmax(atol, 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)));
@@ -673,7 +767,7 @@ k_tridiag(const double* __restrict__ D, const double* __restrict__ E, double* __
                     // converged step: accept only if Sturm counts bracket index k at nt +- 2 tol
                     const double a0 = fmax(lo, nt - 2.0 * tol), b0 = fmin(hi, nt + 2.0 * tol);
                     int ca, cb;
-                    sturm_count2(d, e2, n, a0, b0, pivmin, ca, cb);
+                    sturm_count2(d, e2, n, a0, b0, ca, cb);
                     if (ca <= k && cb > k) { res = fmin(fmax(nt, lo), hi); accepted = true; break; }
                     if (ca > k) { hi = a0; chi = ca; vhi = false; } else { lo = b0; clo = cb; vlo = false; }
                     xn = 0.5 * (lo + hi);
@@ -689,20 +783,19 @@ k_tridiag(const double* __restrict__ D, const double* __restrict__ E, double* __
             x = xn;
             res = x;
         }
-        W[mat * n + k] = res;
+        W[mat * n + k] = res * unscale;
     }
+    if (tid == 0 && sub == 0 && info) info[mat] = 0;
     return;
     }
-    for (int k = tid; k < n; k += TRI_THREADS) lam[k] = W[mat * n + k];
+    for (int k = tid; k < n; k += T) lam[k] = W[mat * n + k] * scale;
     __syncthreads();
     // ---- clusters (relative gap 1e-4 of the norm) and eigenvalue output
     const double ortol = 1e-4 * onenrm;
-    if (tid == 0) {
-        int lead = 0;
-        for (int k = 0; k < n; ++k) {
-            if (k > 0 && lam[k] - lam[k - 1] > ortol) lead = k;
-            leader[k] = lead;
-        }
+    for (int k = tid; k < n; k += T) {
+        int lead = k;
+        while (lead > 0 && lam[lead] - lam[lead - 1] <= ortol) --lead;
+        leader[k] = lead;
     }
     __syncthreads();
     // ---- eigenvectors: isolated eigenvalues by one twisted solve; clusters (handled by the
@@ -710,12 +803,12 @@ k_tridiag(const double* __restrict__ D, const double* __restrict__ E, double* __
     //      still separated, else by inverse iteration with modified Gram-Schmidt
     const double eps = DBL_EPSILON;
     const double dtpcrt = sqrt(0.1 / n);
-    for (int k0 = tid; k0 < n; k0 += TRI_THREADS) {
+    for (int k0 = tid * subs + sub; k0 < n; k0 += T * subs) {
         if (leader[k0] != k0) continue;
         int k1 = k0;
         while (k1 + 1 < n && leader[k1 + 1] == k0) ++k1;
         if (k1 == k0) {
-            twisted_vector(d, e, e2, n, lam[k0], pivmin, z, k0, la, lb, tid);
+            twisted_vector(d, e, n, lam[k0], pivmin, z, k0, la, lb, ls);
             continue;
         }
         // a cluster whose members are still 1e-9 * ||T|| apart: each twisted vector is
@@ -725,7 +818,7 @@ k_tridiag(const double* __restrict__ D, const double* __restrict__ E, double* __
         for (int k = k0 + 1; k <= k1; ++k) mingap = fmin(mingap, lam[k] - lam[k - 1]);
         if (mingap > 1e-9 * onenrm) {
             for (int k = k0; k <= k1; ++k) {
-                twisted_vector(d, e, e2, n, lam[k], pivmin, z, k, la, lb, tid);
+                twisted_vector(d, e, n, lam[k], pivmin, z, k, la, lb, ls);
                 for (int q = k0; q < k; ++q) {
                     double dot = 0.0;
                     for (int j = 0; j < n; ++j) dot += z[(size_t)j * n + q] * z[(size_t)j * n + k];
@@ -754,13 +847,13 @@ k_tridiag(const double* __restrict__ D, const double* __restrict__ E, double* __
             // LU with partial pivoting of T - x I (dlagtf).  The active row carries
             // (u0, u1) = its entries in columns j, j+1; the row pivoted into position j is
             // stored as U diag / super1 / super2 (la, lb, lc2), the multiplier in lm and
-            // the swap flag in lp, all at [j*TRI_THREADS + thread] (one column per thread).
+            // the swap flag in lp, all at [j * ls] of this thread's columns.
             double u0 = d[0] - x, u1 = n > 1 ? e[0] : 0.0;
             for (int j = 0; j < n - 1; ++j) {
                 const double cj = e[j];
                 const double anext = d[j + 1] - x;
                 const double bnext = j + 1 < n - 1 ? e[j + 1] : 0.0;
-                const size_t o = (size_t)j * TRI_THREADS + tid;
+                const size_t o = (size_t)j * ls;
                 if (fabs(u0) >= fabs(cj)) {
                     const double mult = u0 != 0.0 ? cj / u0 : 0.0;
                     la[o] = u0;
@@ -781,12 +874,12 @@ k_tridiag(const double* __restrict__ D, const double* __restrict__ E, double* __
                     u1 = -mult * bnext;
                 }
             }
-            la[(size_t)(n - 1) * TRI_THREADS + tid] = u0;
-            lb[(size_t)(n - 1) * TRI_THREADS + tid] = 0.0;
-            lc2[(size_t)(n - 1) * TRI_THREADS + tid] = 0.0;
+            la[(size_t)(n - 1) * ls] = u0;
+            lb[(size_t)(n - 1) * ls] = 0.0;
+            lc2[(size_t)(n - 1) * ls] = 0.0;
             // tiny pivots are perturbed to +-tolp in the solves (dlagts job = -1)
             double umax = 0.0;
-            for (int j = 0; j < n; ++j) umax = fmax(umax, fabs(la[(size_t)j * TRI_THREADS + tid]));
+            for (int j = 0; j < n; ++j) umax = fmax(umax, fabs(la[(size_t)j * ls]));
             const double tolp = fmax(eps * fmax(umax, onenrm), DBL_MIN);
             for (int j = 0; j < n; ++j) z[(size_t)j * n + k] = start_entry(k, j);
             int nrmchk = 0;
@@ -795,13 +888,13 @@ k_tridiag(const double* __restrict__ D, const double* __restrict__ E, double* __
                 // scale the right-hand side to ||b||_1 = n * onenrm * max(eps, |u_nn|)
                 double b1 = 0.0;
                 for (int j = 0; j < n; ++j) b1 += fabs(z[(size_t)j * n + k]);
-                const double unn = fabs(la[(size_t)(n - 1) * TRI_THREADS + tid]);
+                const double unn = fabs(la[(size_t)(n - 1) * ls]);
                 const double sc = n * onenrm * fmax(eps, unn) / fmax(b1, DBL_MIN);
                 // forward: y = L^{-1} P b  (the active right-hand side value is carried)
                 double rc = z[k] * sc;
                 for (int j = 0; j < n - 1; ++j) {
                     const size_t o = (size_t)j * n + k;
-                    const size_t ol = (size_t)j * TRI_THREADS + tid;
+                    const size_t ol = (size_t)j * ls;
                     const double bnext = z[(size_t)(j + 1) * n + k] * sc;
                     const double mult = lm[ol];
                     if (lp[ol] != 0.0) {
@@ -818,7 +911,7 @@ k_tridiag(const double* __restrict__ D, const double* __restrict__ E, double* __
                 double xmax = 0.0;
                 for (int j = n - 1; j >= 0; --j) {
                     const size_t o = (size_t)j * n + k;
-                    const size_t ol = (size_t)j * TRI_THREADS + tid;
+                    const size_t ol = (size_t)j * ls;
                     double u = la[ol];
                     if (fabs(u) < tolp) u = u >= 0.0 ? tolp : -tolp;
                     const double xj = (z[o] - lb[ol] * x1 - lc2[ol] * x2) / u;
@@ -852,7 +945,7 @@ k_tridiag(const double* __restrict__ D, const double* __restrict__ E, double* __
         }
     }
     __syncthreads();
-    if (tid == 0 && info) info[mat] = s_fail;
+    if (tid == 0 && info && s_fail) atomicAdd(&info[mat], s_fail);   // (cleared by phase 1)
 }
 
 // --------------------------------------------------------------- back-transformation
@@ -1543,7 +1636,12 @@ static constexpr int HP_W_MAX = 32;
 static constexpr int HP_W_WIDE_MIN = 1024;
 static constexpr int HT_TAIL = 64;   // order below which the unblocked kernel finishes
 static constexpr int HT_BLOCKED_MIN = 256;   // orders from which the blocked reduction runs
-static constexpr int DC_DEFAULT_MIN = 600;   // orders from which divide and conquer is the built-in tridiagonal solver (measured: even with bisection at 512, 1.4x at 1024, 2.3x at 3000)
+// Orders from which divide and conquer is the built-in tridiagonal solver.  Bisection is the faster
+// one up to order ~2000 (order 640, 289 matrices 5.5 ms against 16.2; order 1200, 148 matrices 14.4
+// against 37.4; order 2000, 25 matrices 25 against 33), but leaves its vectors orthogonal to 1e-13
+// .. 7e-13 at orders 640 to 2000 where divide and conquer's are to 4e-15 .. 8e-15; callers who
+// want the speed pin it (rlmb_set_tridiag_solver).
+static constexpr int DC_DEFAULT_MIN = 600;
 static constexpr int JAC_DEFAULT_MAX = 20;    // orders up to which k_jacobi is the built-in solver (measured: 2.4x the Householder path at 16, 2.1x at 20, 1.2x at 24, even at 28)
 static constexpr int QUEUE_NT_DEFAULT = 512;   // panel queue CTAs: 512 threads, one per SM
 static constexpr int TUNE_MIN_N = 16;         // orders the autotuner tunes: TUNE_MIN_N .. TUNE_MAX_N
@@ -3039,7 +3137,7 @@ static HeevPlan heev_plan(int n, bool mixed, int refine_steps = 2, int band = -1
     p.off_a = off; off += mixed ? r256(nn * ce) : 0;        // single-precision copy of H, then F
     p.dc = n <= DC_MAX_N && (tune.dc < 0 ? n >= DC_DEFAULT_MIN : tune.dc > 0);
     p.off_z = off; off += r256(nn * sizeof(double));
-    p.off_lu = off; off += p.dc ? 0 : r256(5 * (size_t)n * TRI_THREADS * sizeof(double));
+    p.off_lu = off; off += p.dc ? 0 : r256(5 * (size_t)n * tri_columns(n) * sizeof(double));
     p.off_q2 = off; off += p.dc ? r256(nn * sizeof(double)) : 0;
     p.off_u = off; off += p.dc ? r256(nn * sizeof(double)) : 0;
     p.off_rot = off; off += p.dc ? r256((size_t)n * sizeof(DcRot)) : 0;
@@ -3371,6 +3469,17 @@ static int rayleigh_pass(cudaStream_t st, int n, int band, int nb, const cplx* A
     return RLMB_OK;
 }
 
+template <int T>
+static cudaError_t launch_tridiag(int phase, cudaStream_t st, const HeevPlan& p, int nb, const double* D, const double* E,
+                                  double* W, double* Z, double* LU, int* info) {
+    auto kern = phase == 1 ? k_tridiag<1, T> : k_tridiag<2, T>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem_tri);
+    if (e != cudaSuccess) return e;
+    const int subs = nb <= 148 && p.n > T && (phase == 1 || tri_columns(p.n) >= p.n) ? (p.n + T - 1) / T : 1;
+    kern<<<dim3(nb, subs), T, p.smem_tri, st>>>(D, E, W, Z, LU, info, p.n);
+    return cudaGetLastError();
+}
+
 // Eigenvalues W and eigenvectors Z (row-major) of the chunk's tridiagonals (D, E): bisection +
 // inverse iteration (k_tridiag), or divide and conquer level by level (k_dc_*), ending in Zw.
 static int tridiag_solve(rlmb_context* ctx, cudaStream_t st, const HeevPlan& p, int nb, unsigned char* base,
@@ -3379,11 +3488,15 @@ static int tridiag_solve(rlmb_context* ctx, cudaStream_t st, const HeevPlan& p, 
     const int n = p.n;
     const size_t B = (size_t)nb;
     if (!p.dc) {
+        // threads: the order rounded up to a power-of-two number of warps; above 256 chunks of few
+        // matrices take two CTAs per matrix where the scratch has a column per eigenvector
+        const auto go = n <= 32 ? launch_tridiag<32> : n <= 64 ? launch_tridiag<64> : n <= 128 ? launch_tridiag<128>
+                                                                                            : launch_tridiag<TRI_THREADS>;
         RLMB_CHUNK_PROF("k_stebz");
-        k_tridiag<1><<<nb, TRI_THREADS, p.smem_tri, st>>>(Dw, Ew, W, Zw, LUw, info, n);
+        if (go(1, st, p, nb, Dw, Ew, W, Zw, LUw, info) != cudaSuccess) return RLMB_ERR_CUDA;
         RLMB_CHUNK_LAUNCHED();
         RLMB_CHUNK_PROF("k_stein");
-        k_tridiag<2><<<nb, TRI_THREADS, p.smem_tri, st>>>(Dw, Ew, W, Zw, LUw, info, n);
+        if (go(2, st, p, nb, Dw, Ew, W, Zw, LUw, info) != cudaSuccess) return RLMB_ERR_CUDA;
         RLMB_CHUNK_LAUNCHED();
         return RLMB_OK;
     }
@@ -3451,9 +3564,6 @@ static int heev_chunk(rlmb_context* ctx, cudaStream_t st, const HeevPlan& p, cpl
         return RLMB_OK;
     }
     if (p.smem_tri > 227 * 1024) return RLMB_ERR_ARG;
-    if (cudaFuncSetAttribute(k_tridiag<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem_tri) != cudaSuccess ||
-        cudaFuncSetAttribute(k_tridiag<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem_tri) != cudaSuccess)
-        return RLMB_ERR_CUDA;
     if (!p.mixed) {
         cplx* TAUw = reinterpret_cast<cplx*>(base + p.off_tau * B);
         cplx* Xw = reinterpret_cast<cplx*>(base + p.off_x * B);
