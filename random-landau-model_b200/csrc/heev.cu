@@ -17,9 +17,10 @@
 //                  modified Gram-Schmidt (dstein restated).  From order 600 divide and
 //                  conquer (tridiag_dc.cuh: secular equations, Gu-Eisenstat vectors, DMMA
 //                  merges).  Either one may be pinned or autotuned per order.
-//   back-transform X = Q Z (zunmtr): k_larft + k_ormtr (register-resident Z chunks, blocks
-//                  of 16 reflectors) below order 256, else T factors from batched Gram
-//                  GEMMs and three GEMM launches per block of 64 reflectors.
+//   back-transform X = Q Z (zunmtr): with X resident on the SM in blocks of 16 reflectors
+//                  (k_larft, then k_ormtr_mma in double precision up to order 408, k_ormtr in
+//                  single precision below 256), else T factors from batched Gram GEMMs and
+//                  three GEMM launches per block of 64 reflectors.
 //   mixed mode     the reduction and back-transformation in single precision, then double
 //                  refinement of every eigenpair (k_ref_*, Ogita-Aishima restated, with
 //                  cluster Rayleigh-Ritz).

@@ -17,11 +17,20 @@ namespace rlmb {
 // k_vmn_reduce (deterministic).
 static constexpr int VMN_T = 32;       // output tile edge
 static constexpr int VMN_KC = 32;      // impurities staged per step
-static constexpr int VMN_KSPLIT = 2048;  // impurities per CTA
+static constexpr int VMN_KSPLIT = 2048;  // impurities per CTA at most
+// Impurities per CTA: 2048 where the tiles of one sample fill the GPU with that, down to 64 where
+// they are few (a CTA's time is its chain of staged steps: n_phi = 129, 2 samples, 4 tiles each,
+// 200 us with 2048, 17 us now; n_phi = 16, one tile, 29 us, now 11).  It depends on the
+// sample's sizes alone, so that a sample's sums are the same in any batch.
+static int vmn_chunk(int nimp, int dim) {
+    const int nt = (dim + VMN_T - 1) / VMN_T, want = (148 + nt * nt - 1) / (nt * nt);
+    const int chunk = ((nimp + want - 1) / want + VMN_KC - 1) / VMN_KC * VMN_KC;
+    return std::min(std::max(chunk, 64), VMN_KSPLIT);
+}
 
 __global__ void __launch_bounds__(256)
 k_vmn_partial(const double* __restrict__ X, const double* __restrict__ Y,
-              const double* __restrict__ S, int nimp, int dim, int off_head, int nsplit,
+              const double* __restrict__ S, int nimp, int dim, int off_head, int nsplit, int chunk,
               cplx* __restrict__ partial) {
     __shared__ cplx ex[VMN_T][VMN_KC + 1];   // s_i e^{-i 2pi (m-o) x_i}
     __shared__ cplx ey[VMN_T][VMN_KC + 1];   // e^{-i 2pi (n-o) y_i}
@@ -31,7 +40,7 @@ k_vmn_partial(const double* __restrict__ X, const double* __restrict__ Y,
     const double* x = X + (size_t)sample * nimp;
     const double* y = Y + (size_t)sample * nimp;
     const double* s = S + (size_t)sample * nimp;
-    const int i_begin = split * VMN_KSPLIT, i_end = min(nimp, i_begin + VMN_KSPLIT);
+    const int i_begin = split * chunk, i_end = min(nimp, i_begin + chunk);
     // thread owns outputs (m0 + tm + 8*u, n0 + tn) for u = 0..3
     const int tn = tid & 31, tm = tid >> 5;
     cplx acc[4] = {mk(0, 0), mk(0, 0), mk(0, 0), mk(0, 0)};
@@ -80,12 +89,17 @@ __global__ void k_vmn_reduce(const cplx* __restrict__ partial, const cplx* __res
 int launch_rlm_potential(rlmb_context* ctx, const double* x, const double* y, const double* s,
                          int nimp, int nsamples, const cplx* coeff_mn, int dim, int off_head,
                          cplx* partial_ws, cplx* vmn) {
-    const int nsplit = (nimp + VMN_KSPLIT - 1) / VMN_KSPLIT;
+    const int chunk = vmn_chunk(nimp, dim), nsplit = (nimp + chunk - 1) / chunk;
     const int nt = (dim + VMN_T - 1) / VMN_T;
-    dim3 g(nt, nt, nsamples * nsplit);
-    prof_begin(ctx, "k_vmn_partial");
-    k_vmn_partial<<<g, 256, 0, ctx->stream>>>(x, y, s, nimp, dim, off_head, nsplit, partial_ws);
-    RLMB_LAUNCHED(ctx);
+    const int per = std::max(1, 65535 / nsplit);   // samples per launch (grid z extent)
+    for (int s0 = 0; s0 < nsamples; s0 += per) {
+        const dim3 g(nt, nt, std::min(per, nsamples - s0) * nsplit);
+        const size_t o = (size_t)s0 * nimp;
+        prof_begin(ctx, "k_vmn_partial");
+        k_vmn_partial<<<g, 256, 0, ctx->stream>>>(x + o, y + o, s + o, nimp, dim, off_head, nsplit, chunk,
+                                                  partial_ws + (size_t)s0 * nsplit * dim * dim);
+        RLMB_LAUNCHED(ctx);
+    }
     const size_t total = (size_t)dim * dim * nsamples;
     prof_begin(ctx, "k_vmn_reduce");
     k_vmn_reduce<<<(unsigned)((total + 255) / 256), 256, 0, ctx->stream>>>(partial_ws, coeff_mn, dim,
@@ -94,7 +108,7 @@ int launch_rlm_potential(rlmb_context* ctx, const double* x, const double* y, co
     return RLMB_OK;
 }
 size_t rlm_potential_ws_elems(int nimp, int nsamples, int dim) {
-    const int nsplit = (nimp + VMN_KSPLIT - 1) / VMN_KSPLIT;
+    const int chunk = vmn_chunk(nimp, dim), nsplit = (nimp + chunk - 1) / chunk;
     return (size_t)nsamples * nsplit * dim * dim;
 }
 
