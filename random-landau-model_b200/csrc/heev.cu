@@ -134,17 +134,18 @@ __device__ __forceinline__ void hetrd_tile(const S& st, int m, int r0, int c0, c
         es[j] = cz<C>();
         C vc, wc;
         if (UPD) {
-            vc = cconj(v[c]);
-            wc = cconj(w[c]);
+            vc = v[c];
+            wc = w[c];
+            vc.x = -vc.x;   // -conj
+            wc.x = -wc.x;
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int r = r0 + lr + 8 * i;
             const bool in = INSIDE || (c < m && r <= c);
             if (UPD) {
-                C u = cmul(vr[i], wc);
-                cfma(u, wr[i], vc);
-                x[i] = csub(x[i], u);
+                cfma(x[i], vr[i], wc);
+                cfma(x[i], wr[i], vc);
                 if (!INSIDE && r == c) x[i].y = 0;
                 if (in) *st.at(r, c) = x[i];
                 else x[i] = cz<C>();
@@ -204,10 +205,17 @@ __device__ __forceinline__ R hetrd_pass(S st, int m, const C* __restrict__ v, co
 // (A' vn)[r] of the leading m x m block from the tiles' parts.
 template <class C>
 __device__ __forceinline__ C hetrd_sum(const C* __restrict__ part, int m, int r) {
-    const int nb = (m + 15) / 16, b = r >> 4, o = r & 15;
-    C s = cz<C>();
-    for (int cb = b; cb < nb; ++cb) s = cadd(s, part[32 * (cb * (cb + 1) / 2 + b) + o]);
-    for (int rb = 0; rb <= b; ++rb) s = cadd(s, part[32 * (b * (b + 1) / 2 + rb) + 16 + o]);
+    const int nb = (m + 15) / 16, b = r >> 4;
+    const C* q = part + 16 * b * (b + 1) + (r & 15);   // tile (0, b)
+    C s = q[16];
+    for (int rb = 0; rb < b; ++rb) {                   // column sums of tiles (0, b) .. (b, b)
+        q += 32;
+        s = cadd(s, q[16]);
+    }
+    for (int cb = b; cb < nb; ++cb) {                  // row sums of tiles (b, b) .. (b, nb - 1)
+        s = cadd(s, *q);
+        q += 32 * (cb + 1);
+    }
     return s;
 }
 
@@ -223,10 +231,11 @@ __device__ __forceinline__ void reflector(const C alpha, R xnorm2, R& beta, C& t
     }
     const R nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xnorm2);
     beta = alpha.x >= 0 ? -nrm : nrm;
-    tau = cm<C>((beta - alpha.x) / beta, -alpha.y / beta);
+    const R ib = 1 / beta;   // (every warp computes the reflector: two divisions, not four)
+    tau = cm<C>((beta - alpha.x) * ib, -alpha.y * ib);
     const C den = cm<C>(alpha.x - beta, alpha.y);
-    const R dn = cabs2(den);
-    scal = cm<C>(den.x / dn, -den.y / dn);
+    const R id = 1 / cabs2(den);
+    scal = cm<C>(den.x * id, -den.y * id);
 }
 
 // Unblocked reduction A = Q T Q^H (zhetd2, uplo='U') with look-ahead: step i's rank-2
@@ -2221,14 +2230,30 @@ k_hetrd_panel_c(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, doubl
             else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
             quad = warp_sum(quad);
             if (lane < P) panel_peer(quadp, lane, P)[rank * NW + warp] = quad;
-            // this CTA's rows of w_q^H v (even slots) and v_q^H v (odd slots)
-            for (int t2 = warp; t2 < 2 * j; t2 += NW) {
-                const C* y = ((t2 & 1) ? V : W) + (size_t)(t2 >> 1) * n;
-                C sd = cz<C>();
+            // this CTA's rows of w_q^H v (even slots) and v_q^H v (odd slots), two pairs per warp at
+            // a time: their four sums cross the warp together, each ending in eight lanes
+            for (int q0 = 2 * warp; q0 < j; q0 += 2 * NW) {
+                const C *w0 = W + (size_t)q0 * n, *v0 = V + (size_t)q0 * n;
+                const size_t step = q0 + 1 < j ? n : 0;   // (a last pair alone is summed twice)
+                C sd[4] = {cz<C>(), cz<C>(), cz<C>(), cz<C>()};
 #pragma unroll 2
-                for (int r = ((lane >> 3) * P + rank) * 8 + (lane & 7); r < c; r += 32 * P) cfmac(sd, y[r], v[r]);
-                sd = warp_sum(sd);
-                if (lane < P) panel_peer(coefp, lane, P)[rank * 2 * HP_W_MAX + t2] = sd;
+                for (int r = ((lane >> 3) * P + rank) * 8 + (lane & 7); r < c; r += 32 * P) {
+                    const C vr = v[r];
+                    cfmac(sd[0], w0[r], vr);
+                    cfmac(sd[1], v0[r], vr);
+                    cfmac(sd[2], w0[step + r], vr);
+                    cfmac(sd[3], v0[step + r], vr);
+                }
+                const bool u1 = (lane & 16) != 0, u0 = (lane & 8) != 0;
+                C y[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) y[i] = cadd(u1 ? sd[i + 2] : sd[i], shfl_xor(u1 ? sd[i] : sd[i + 2], 16));
+                C s = cadd(u0 ? y[1] : y[0], shfl_xor(u0 ? y[0] : y[1], 8));
+                s = cadd(s, shfl_xor(s, 4));
+                s = cadd(s, shfl_xor(s, 2));
+                s = cadd(s, shfl_xor(s, 1));
+                const int t2 = 2 * q0 + (lane >> 3);   // (an absent second pair's slots are not read)
+                for (int k = lane & 7; k < P; k += 8) panel_peer(coefp, k, P)[rank * 2 * HP_W_MAX + t2] = s;
             }
             panel_sync(P);
             if (warp == 0) {
