@@ -3506,6 +3506,43 @@ static cudaError_t launch_tridiag(int phase, cudaStream_t st, const HeevPlan& p,
     return cudaGetLastError();
 }
 
+static cudaLaunchConfig_t dc_merge_config(cudaLaunchAttribute* at, cudaStream_t st, int nb, int Y, size_t smem) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(nb * Y);
+    cfg.blockDim = dim3(DC_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = Y;
+    at->val.clusterDim.y = 1;
+    at->val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+// CTAs per matrix of k_dc_merge (its shared-memory attribute set): the most, up to 8, with which
+// every cluster of the chunk runs at once.
+static int dc_cluster(int nb, int n, size_t smem) {
+    for (int Y = 8; Y > 1; --Y) {
+        if (nb * Y > 148) continue;
+        int active = 0;
+        cudaLaunchAttribute at[1];
+        const cudaLaunchConfig_t cfg = dc_merge_config(at, 0, nb, Y, smem);
+        if (cudaOccupancyMaxActiveClusters(&active, k_dc_merge, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            continue;
+        }
+        if (active >= nb) return Y;
+    }
+    return 1;
+}
+static cudaError_t launch_dc_merge(cudaStream_t st, int nb, int Y, const double* E, const double* SC, double* W,
+                                   const double* Qo, double* Qn, double* U, DcRot* ROT, int* info, int n, int S) {
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = dc_merge_config(at, st, nb, Y, dc_smem(S, n));
+    return cudaLaunchKernelEx(&cfg, k_dc_merge, E, SC, W, Qo, Qn, U, ROT, info, n, S, Y);
+}
+
 // Eigenvalues W and eigenvectors Z (row-major) of the chunk's tridiagonals (D, E): bisection +
 // inverse iteration (k_tridiag), or divide and conquer level by level (k_dc_*), ending in Zw.
 static int tridiag_solve(rlmb_context* ctx, cudaStream_t st, const HeevPlan& p, int nb, unsigned char* base,
@@ -3541,12 +3578,13 @@ static int tridiag_solve(rlmb_context* ctx, cudaStream_t st, const HeevPlan& p, 
         cudaFuncSetAttribute(k_dc_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DgTiles)) !=
             cudaSuccess)
         return RLMB_ERR_CUDA;
+    const int Y = dc_cluster(nb, n, smem_max);
     RLMB_CHUNK_PROF("k_dc_merge");
     k_dc_init<<<nb, 256, 0, st>>>(Dw, Ew, W, qa, SCw, info, n);
     RLMB_CHUNK_LAUNCHED();
     for (int S = 2; S / 2 < n; S *= 2) {
         RLMB_CHUNK_PROF("k_dc_merge");
-        k_dc_merge<<<nb, DC_THREADS, dc_smem(S, n), st>>>(Ew, SCw, W, qa, qb, Uw, Rw, info, n, S);
+        if (launch_dc_merge(st, nb, Y, Ew, SCw, W, qa, qb, Uw, Rw, info, n, S) != cudaSuccess) return RLMB_ERR_CUDA;
         RLMB_CHUNK_LAUNCHED();
         if (S > DC_SMALL) {
             const int nsub = (n + S - 1) / S;

@@ -30,7 +30,7 @@
 //
 // Q is row-major (Q[j*n + k] = component j of eigenvector k), the layout of k_tridiag's Z that
 // the back-transformation reads.  The tridiagonal is scaled by a power of two (exact) so that
-// its largest entry is ~1.  No kernel waits on another CTA.
+// its largest entry is ~1.  No kernel waits on a CTA outside its cluster.
 #pragma once
 #include <cfloat>
 
@@ -177,14 +177,21 @@ __device__ __forceinline__ void dc_pole_sums(const double* __restrict__ ds, cons
     sw2 = (b0 + b1) + (b2 + b3);
 }
 
-// One level of merges: one CTA of DC_THREADS per matrix, a group of dc_group_threads(S, n)
-// threads per subproblem of size S (children S/2 and the rest).  W holds the children's
+// One level of merges: a cluster of Y CTAs of DC_THREADS per matrix, a group of
+// dc_group_threads(S, n) threads per subproblem of size S (children S/2 and the rest).  Groups
+// smaller than a CTA take subproblems on their own; where a group is a whole CTA the cluster
+// takes each subproblem together: every CTA holds its poles, the roots, z and columns of U are
+// dealt over the CTAs, roots and z being written to all of them (distributed shared memory).
+// A level of a large matrix is bound by the divisions of its secular terms, which one CTA per
+// matrix left to 25 of 148 SMs for 25 matrices: order 2500 41 ms, 20 with clusters of 5 (the
+// rest is the deflation, one thread walking the sorted poles).
+// W holds the children's
 // sorted eigenvalues on entry and the merged ones on return; Qo the children's eigenvectors,
 // Qn the merged ones (for S <= DC_SMALL, else U for k_dc_gemm).
 __global__ void __launch_bounds__(DC_THREADS, 1)
 k_dc_merge(const double* __restrict__ E, const double* __restrict__ SC, double* __restrict__ W,
            const double* __restrict__ Qo, double* __restrict__ Qn, double* __restrict__ U, DcRot* __restrict__ ROT,
-           int* __restrict__ info, int n, int S) {
+           int* __restrict__ info, int n, int S, int Y) {
     extern __shared__ __align__(16) unsigned char dc_sm[];
     const int gs = dc_group_threads(S, n), ng = DC_THREADS / gs;
     const int grp = threadIdx.x / gs, gt = threadIdx.x % gs;
@@ -201,7 +208,30 @@ k_dc_merge(const double* __restrict__ E, const double* __restrict__ SC, double* 
     int* org = src + sm8;
     int* pos = org + sm8;                         // output column -> sorted position (first a flag array)
     int* scal = pos + sm8;                        // K, number of rotations, failure flag
-    const size_t mat = blockIdx.x;
+    const size_t mat = blockIdx.x / Y;
+    const int rank = (int)(blockIdx.x % Y);
+    const bool coop = Y > 1 && gs == DC_THREADS;   // the cluster shares every subproblem
+    // this thread's share of a subproblem's roots, entries of z and columns
+    const int ct = coop ? rank * gs + gt : gt, cs = coop ? Y * gs : gs;
+    auto share = [&](auto* p, int at, auto v) {    // p[at] = v in every CTA that shares the subproblem
+        if (!coop) {
+            p[at] = v;
+            return;
+        }
+        for (int k = 0; k < Y; ++k) {
+            decltype(p) q;
+            asm("mapa.u64 %0, %1, %2;" : "=l"(q) : "l"(p), "r"(k));
+            q[at] = v;
+        }
+    };
+    auto share_sync = [&]() {
+        if (coop) {
+            asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        } else {
+            dc_sync(grp, gs);
+        }
+    };
     const double rs = 1.0 / SC[mat];
     const double* e = E + mat * n;
     double* lam = W + mat * n;
@@ -209,11 +239,11 @@ k_dc_merge(const double* __restrict__ E, const double* __restrict__ SC, double* 
     double* qn = Qn + mat * (size_t)n * n;
     const int nsub = (n + S - 1) / S;
     int fail = 0;
-    for (int s = grp; s < nsub; s += ng) {
+    for (int s = coop ? 0 : rank * ng + grp; s < nsub; s += coop ? 1 : Y * ng) {
         const int o = s * S;
         const int K0 = min(S, n - o), n1 = min(S / 2, K0), n2 = K0 - n1;
         if (n2 <= 0) {   // a single child: its block carries over
-            for (int idx = gt; idx < n1 * n1; idx += gs) {
+            for (int idx = ct; idx < n1 * n1; idx += cs) {
                 const int r = idx / n1, c = idx % n1;
                 qn[(size_t)(o + r) * n + o + c] = qo[(size_t)(o + r) * n + o + c];
             }
@@ -300,7 +330,7 @@ k_dc_merge(const double* __restrict__ E, const double* __restrict__ SC, double* 
         const int K = scal[0], nrot = scal[1];
         const double rrho = 1.0 / fmax(rho, DBL_MIN);
         // secular equation, one thread per root
-        for (int j = gt; j < K; j += gs) {
+        for (int j = ct; j < K; j += cs) {
             int og;
             double lo, hi;
             if (j < K - 1) {
@@ -379,12 +409,12 @@ k_dc_merge(const double* __restrict__ E, const double* __restrict__ SC, double* 
                 t = tn;
             }
             if (!conv) fail = 1;
-            org[j] = og;
-            tau[j] = t;
+            share(org, j, og);
+            share(tau, j, t);
         }
-        dc_sync(grp, gs);
+        share_sync();
         // z from the roots (Gu & Eisenstat): pairs (x_j - d_i) / (d_j - d_i), and (x_i - d_i) / rho
-        for (int i = gt; i < K; i += gs) {
+        for (int i = ct; i < K; i += cs) {
             const double di = ds[i];
             double p0 = 1.0, p1 = 1.0;   // even and odd j: two divisions in flight
             int j = 0;
@@ -394,12 +424,12 @@ k_dc_merge(const double* __restrict__ E, const double* __restrict__ SC, double* 
                 p1 *= x1 / (j + 1 == i ? rho : ds[j + 1] - di);
             }
             if (j < K) p0 *= ((ds[org[j]] - di) + tau[j]) / (j == i ? rho : ds[j] - di);
-            zh[i] = copysign(sqrt(fmax(p0 * p1, 0.0)), zs[i]);
+            share(zh, i, copysign(sqrt(fmax(p0 * p1, 0.0)), zs[i]));
         }
         for (int j = gt; j < K; j += gs) vals[j] = ds[org[j]] + tau[j];
-        dc_sync(grp, gs);
+        share_sync();
         // output order: rank of every merged eigenvalue (ties by column)
-        for (int c = gt; c < K0; c += gs) {
+        for (int c = ct; c < K0; c += cs) {
             const double v = vals[c];
             int rk = 0;
             for (int c2 = 0; c2 < K0; ++c2) {
@@ -407,11 +437,10 @@ k_dc_merge(const double* __restrict__ E, const double* __restrict__ SC, double* 
                 rk += (v2 < v || (v2 == v && c2 < c)) ? 1 : 0;
             }
             pos[c] = rk;   // (the deflation flags in pos are no longer needed)
+            lam[o + rk] = v;
         }
-        dc_sync(grp, gs);
-        for (int c = gt; c < K0; c += gs) lam[o + pos[c]] = vals[c];
         // U: column pos[c] = eigenvector c in the children's basis (rows = child indices)
-        for (int c = gt; c < K0; c += gs) {
+        for (int c = ct; c < K0; c += cs) {   // (this thread's own c)
             const int col = pos[c];
             if (c < K) {
                 const double x0 = ds[org[c]], tc = tau[c];
@@ -439,18 +468,15 @@ k_dc_merge(const double* __restrict__ E, const double* __restrict__ SC, double* 
                 const int row = perm[src[c]];
                 for (int i = 0; i < K0; ++i) us[(size_t)i * K0 + col] = i == row ? 1.0 : 0.0;
             }
+            // U <- G U, the deflation rotations last to first
+            for (int r = nrot - 1; r >= 0; --r) {
+                const DcRot R = rl[r];
+                const double ua = us[(size_t)R.a * K0 + col], ub = us[(size_t)R.b * K0 + col];
+                us[(size_t)R.a * K0 + col] = R.c * ua - R.s * ub;
+                us[(size_t)R.b * K0 + col] = R.s * ua + R.c * ub;
+            }
         }
         dc_sync(grp, gs);
-        if (nrot > 0) {   // U <- G U, the deflation rotations last to first
-            for (int col = gt; col < K0; col += gs)
-                for (int r = nrot - 1; r >= 0; --r) {
-                    const DcRot R = rl[r];
-                    const double ua = us[(size_t)R.a * K0 + col], ub = us[(size_t)R.b * K0 + col];
-                    us[(size_t)R.a * K0 + col] = R.c * ua - R.s * ub;
-                    us[(size_t)R.b * K0 + col] = R.s * ua + R.c * ub;
-                }
-            dc_sync(grp, gs);
-        }
         if (S <= DC_SMALL) {   // Q_new = blockdiag(Q1, Q2) U here
             for (int idx = gt; idx < K0 * K0; idx += gs) {
                 const int r = idx / K0, c = idx % K0;
@@ -460,7 +486,7 @@ k_dc_merge(const double* __restrict__ E, const double* __restrict__ SC, double* 
                 qn[(size_t)(o + r) * n + o + c] = acc;
             }
         }
-        dc_sync(grp, gs);   // the group's shared arrays are rewritten by its next subproblem
+        share_sync();   // the shared arrays are rewritten by the next subproblem, or left
     }
     if (fail && info) atomicMax(info + mat, 1);
 }
