@@ -977,6 +977,14 @@ __device__ __forceinline__ C refl_entry(const C* __restrict__ a, int n, int i, i
     return a[(size_t)(i + 1) * n + r];
 }
 
+// its address, or null with the implicit value in imm
+template <class C>
+__device__ __forceinline__ const C* refl_addr(const C* __restrict__ a, int n, int i, int r, cplx& imm) {
+    if (i <= n - 2 && r < i) return a + (size_t)(i + 1) * n + r;
+    imm.x = i <= n - 2 && r == i ? 1.0 : 0.0;
+    return nullptr;
+}
+
 // T factor of one block of one matrix, grid (blocks, matrices):
 //   T[k][k] = tau_k,  T[k][q] = -tau_k sum_{l=q}^{k-1} (v_k^H v_l) T[l][q]   (q < k)
 template <class R>
@@ -1495,13 +1503,18 @@ struct OpColA {
     __device__ __forceinline__ C elem(size_t mat, int r, int k) const {
         return from_c64<C>(to_c64(p[mat * stride + (size_t)k * ld + r]));
     }
+    static constexpr bool CONJ = false;
+    __device__ __forceinline__ const PT* addr(size_t mat, int r, int k, cplx&) const {
+        return p + mat * stride + (size_t)k * ld + r;
+    }
 };
 
 // A(r, k) = P(k, r), conjugated if CONJ, of a column-major P (entry (k, r) at p[r*ld + k]):
 // the (conjugate) transpose, k contiguous.
-template <class C, class PT, bool CONJ>
+template <class C, class PT, bool CJ>
 struct OpRowA {
     static constexpr bool RFAST = false;
+    static constexpr bool CONJ = CJ;
     const PT* p;
     int ld;
     size_t stride;
@@ -1509,6 +1522,9 @@ struct OpRowA {
         C v = from_c64<C>(to_c64(p[mat * stride + (size_t)r * ld + k]));
         if (CONJ) v.y = -v.y;
         return v;
+    }
+    __device__ __forceinline__ const PT* addr(size_t mat, int r, int k, cplx&) const {
+        return p + mat * stride + (size_t)r * ld + k;
     }
 };
 
@@ -1522,6 +1538,10 @@ struct OpColB {
     __device__ __forceinline__ C elem(size_t mat, int k, int c) const {
         return from_c64<C>(to_c64(p[mat * stride + (size_t)c * ld + k]));
     }
+    static constexpr bool CONJ = false;
+    __device__ __forceinline__ const PT* addr(size_t mat, int k, int c, cplx&) const {
+        return p + mat * stride + (size_t)c * ld + k;
+    }
 };
 
 // Reflectors i0 + q of a reduced matrix as columns of V (V(r, q) = v_{i0+q}[r], with the
@@ -1534,6 +1554,10 @@ struct OpRefl {
     __device__ __forceinline__ C elem(size_t mat, int r, int q) const {
         return refl_entry(a + mat * (size_t)n * n, n, i0 + q, r);
     }
+    static constexpr bool CONJ = false;
+    __device__ __forceinline__ const C* addr(size_t mat, int r, int q, cplx& imm) const {
+        return refl_addr(a + mat * (size_t)n * n, n, i0 + q, r, imm);
+    }
 };
 template <class C>
 struct OpReflH {
@@ -1544,6 +1568,10 @@ struct OpReflH {
         C v = refl_entry(a + mat * (size_t)n * n, n, i0 + q, r);
         v.y = -v.y;
         return v;
+    }
+    static constexpr bool CONJ = true;
+    __device__ __forceinline__ const C* addr(size_t mat, int q, int r, cplx& imm) const {
+        return refl_addr(a + mat * (size_t)n * n, n, i0 + q, r, imm);
     }
 };
 
@@ -1559,6 +1587,10 @@ struct OpBlkReflH {
         v.y = -v.y;
         return v;
     }
+    static constexpr bool CONJ = true;
+    __device__ __forceinline__ const C* addr(size_t z, int q, int r, cplx& imm) const {
+        return refl_addr(a + (z / nblk) * (size_t)n * n, n, (int)(z % nblk) * bs + q, r, imm);
+    }
 };
 template <class C>
 struct OpBlkRefl {
@@ -1567,6 +1599,10 @@ struct OpBlkRefl {
     int n, nblk, bs;
     __device__ __forceinline__ C elem(size_t z, int r, int l) const {
         return refl_entry(a + (z / nblk) * (size_t)n * n, n, (int)(z % nblk) * bs + l, r);
+    }
+    static constexpr bool CONJ = false;
+    __device__ __forceinline__ const C* addr(size_t z, int r, int l, cplx& imm) const {
+        return refl_addr(a + (z / nblk) * (size_t)n * n, n, (int)(z % nblk) * bs + l, r, imm);
     }
 };
 
@@ -2497,6 +2533,10 @@ struct OpPanelA {
         const size_t o = mat * (size_t)w * n;
         return k < w ? pv[o + (size_t)k * n + r] : pw[o + (size_t)(k - w) * n + r];
     }
+    static constexpr bool CONJ = false;
+    __device__ __forceinline__ const C* addr(size_t mat, int r, int k, cplx&) const {
+        return (k < w ? pv + (size_t)k * n : pw + (size_t)(k - w) * n) + mat * (size_t)w * n + r;
+    }
 };
 template <class C, int w>
 struct OpPanelB {
@@ -2507,6 +2547,10 @@ struct OpPanelB {
     __device__ __forceinline__ C elem(size_t mat, int k, int c) const {
         const size_t o = mat * (size_t)w * n;
         return cconj(k < w ? pw[o + (size_t)k * n + c] : pv[o + (size_t)(k - w) * n + c]);
+    }
+    static constexpr bool CONJ = true;
+    __device__ __forceinline__ const C* addr(size_t mat, int k, int c, cplx&) const {
+        return (k < w ? pw + (size_t)k * n : pv + (size_t)(k - w) * n) + mat * (size_t)w * n + c;
     }
 };
 // A(r, c) -= acc on and above the diagonal (real diagonal); tiles below it are skipped.
@@ -2686,6 +2730,14 @@ struct OpBandA {
         k = k < 0 ? k + n : (k >= n ? k - n : k);
         return cconj(p[mat * (size_t)n * n + (size_t)r * n + k]);
     }
+    static constexpr bool CONJ = true;
+    __device__ __forceinline__ const cplx* addr(size_t mat, int r, int kk, cplx&) const {
+        const int r0 = r - r % RB_BM, dist = kk - (r - r0);
+        if (dist < 0 || dist > 2 * o) return nullptr;   // (0)
+        int k = r0 - o + kk;
+        k = k < 0 ? k + n : (k >= n ? k - n : k);
+        return p + mat * (size_t)n * n + (size_t)r * n + k;
+    }
 };
 template <class XT>
 struct OpBandB {
@@ -2696,6 +2748,12 @@ struct OpBandB {
         int k = (int)blockIdx.x * RB_BM - o + kk;   // the tile's r0 (the engine's row tile is RB_BM)
         k = k < 0 ? k + n : (k >= n ? k - n : k);
         return to_c64(p[mat * (size_t)n * n + (size_t)c * n + k]);
+    }
+    static constexpr bool CONJ = false;
+    __device__ __forceinline__ const XT* addr(size_t mat, int kk, int c, cplx&) const {
+        int k = (int)blockIdx.x * RB_BM - o + kk;
+        k = k < 0 ? k + n : (k >= n ? k - n : k);
+        return p + mat * (size_t)n * n + (size_t)c * n + k;
     }
 };
 

@@ -309,12 +309,163 @@ k_zgemm_dmma(LA la, LB lb, EP ep, int M, int N, int K) {
     }
 }
 
+// ---- the same with the operands copied by cp.async
+// Operands that lie in memory as double-complex entries may expose CONJ (the product takes their
+// conjugate) and addr(mat, r, k, imm) / addr(mat, k, c, imm): the entry's address, or null with
+// its value in imm.  Their tiles then go to shared memory by cp.async, ST stages of KC inner
+// entries deep, without passing through registers: one barrier per stage, the copies two or
+// three stages ahead of their use.  In-place epilogues take the room of their prefetched C from
+// the stages (4 entries each instead of 8), so that two CTAs still share an SM.
+// Bound: the DMMA pipe.  With register-staged loads one stage ahead (k_zgemm_dmma) it was 60-67 %
+// busy in the reduction's updates and the back-transformation: rank-64 updates of 25 matrices of
+// order 2500 54.1 -> 49.9 ms and their back-transformation 141 -> 133; rank-32 updates of 4,224
+// matrices of order 256 14.5 -> 13.0, of 578 of order 512 13.7 -> 12.8.
+template <class T, class = void>
+struct zg_async : std::false_type {};
+template <class T>
+struct zg_async<T, std::void_t<decltype(&T::addr)>>
+    : std::is_same<decltype(std::declval<const T&>().addr((size_t)0, 0, 0, std::declval<cplx&>())), const cplx*> {};
+
+template <int BM, class EP>
+struct ZgAsync {
+    static constexpr bool PRE = zg_has_pre<EP>::value;
+    static constexpr int KC = PRE ? 4 : 8, ST = 4;
+    static constexpr size_t stages = sizeof(cplx) * ST * KC * (BM + ZT_PAD + ZG_BN + ZT_PAD);
+    static constexpr size_t smem = stages + (PRE ? (size_t)256 * 4 * (ZG_BN * (BM / 32) / 64) * 2 * sizeof(cplx) : 0);
+};
+
+template <int BM, class LA, class LB, class EP>
+__global__ void __launch_bounds__(256, BM == 64 ? 2 : 1)
+k_zgemm_async(LA la, LB lb, EP ep, int M, int N, int K) {
+    constexpr int KC = ZgAsync<BM, EP>::KC, ST = ZgAsync<BM, EP>::ST;
+    constexpr bool PRE = ZgAsync<BM, EP>::PRE;
+    constexpr int WR = BM / 32, WN = ZG_BN * WR / 8, MI = 4, NJ = WN / 8;
+    constexpr int AS = BM + ZT_PAD, BS = ZG_BN + ZT_PAD;
+    extern __shared__ __align__(16) unsigned char zg_smem[];
+    cplx* sa = reinterpret_cast<cplx*>(zg_smem);     // [ST][KC][AS]
+    cplx* sb = sa + ST * KC * AS;                    // [ST][KC][BS]
+    cplx* pre = reinterpret_cast<cplx*>(zg_smem + ZgAsync<BM, EP>::stages);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int wr = warp % WR, wc = warp / WR, g = lane >> 2, q = lane & 3;
+    const size_t mat = blockIdx.z;
+    const int r0 = blockIdx.x * BM, c0 = blockIdx.y * ZG_BN;
+    if (ep.skip(r0, c0, BM)) return;   // output tile not needed (whole CTA leaves together)
+    auto fetch = [&](int kt) {
+        const int k0 = kt * KC;
+        cplx* da = sa + (kt % ST) * KC * AS;
+        cplx* db = sb + (kt % ST) * KC * BS;
+#pragma unroll
+        for (int e = 0; e < BM * KC / 256; ++e) {
+            const int idx = t + 256 * e;
+            const int kk = LA::RFAST ? idx / BM : idx % KC, rr = LA::RFAST ? idx % BM : idx / KC;
+            cplx imm = mk(0, 0);
+            const cplx* src = r0 + rr < M && k0 + kk < K ? la.addr(mat, r0 + rr, k0 + kk, imm) : nullptr;
+            if (src) zg_cp_async16(da + kk * AS + rr, src);
+            else da[kk * AS + rr] = imm;
+        }
+#pragma unroll
+        for (int e = 0; e < ZG_BN * KC / 256; ++e) {
+            const int idx = t + 256 * e;
+            const int kk = LB::KFAST ? idx % KC : idx / ZG_BN, cc = LB::KFAST ? idx / KC : idx % ZG_BN;
+            cplx imm = mk(0, 0);
+            const cplx* src = c0 + cc < N && k0 + kk < K ? lb.addr(mat, k0 + kk, c0 + cc, imm) : nullptr;
+            if (src) zg_cp_async16(db + kk * BS + cc, src);
+            else db[kk * BS + cc] = imm;
+        }
+    };
+    const int nk = (K + KC - 1) / KC;
+#pragma unroll
+    for (int s = 0; s < ST - 1; ++s) {
+        if (s < nk) fetch(s);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        if (PRE && s == 0) {   // C's entries, after the first operands
+            if constexpr (PRE) {
+#pragma unroll
+                for (int i = 0; i < MI; ++i)
+#pragma unroll
+                    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const int r = r0 + 32 * wr + 8 * i + g, c = c0 + WN * wc + 8 * j + 2 * q + e;
+                            const cplx* src = (r < M && c < N) ? ep.pre_src(mat, r, c) : nullptr;
+                            if (src) zg_cp_async16(pre + ((i * NJ + j) * 2 + e) * 256 + t, src);
+                        }
+            }
+        }
+    }
+    double cr[MI][NJ][2], ci[MI][NJ][2];
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) cr[i][j][0] = cr[i][j][1] = ci[i][j][0] = ci[i][j][1] = 0.0;
+    for (int kt = 0; kt < nk; ++kt) {
+        // stage kt has arrived (this thread's copies; then everyone's), stage kt - 1 is free
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(ST - 2) : "memory");
+        __syncthreads();
+        if (kt + ST - 1 < nk) fetch(kt + ST - 1);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        const cplx* pa = sa + (kt % ST) * KC * AS + q * AS + 32 * wr + g;
+        const cplx* pb = sb + (kt % ST) * KC * BS + q * BS + WN * wc + g;
+#pragma unroll
+        for (int ks = 0; ks < KC / 4; ++ks) {
+            double ar[MI], ai[MI], an[MI], br[NJ], bi[NJ];
+#pragma unroll
+            for (int i = 0; i < MI; ++i) {
+                const cplx x = pa[4 * ks * AS + 8 * i];
+                ar[i] = x.x;
+                ai[i] = LA::CONJ ? -x.y : x.y;
+                an[i] = LA::CONJ ? x.y : -x.y;
+            }
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) {
+                const cplx y = pb[4 * ks * BS + 8 * j];
+                br[j] = y.x;
+                bi[j] = LB::CONJ ? -y.y : y.y;
+            }
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) {
+                    dmma884(cr[i][j], ar[i], br[j]);
+                    dmma884(ci[i][j], ar[i], bi[j]);
+                    dmma884(cr[i][j], an[i], bi[j]);
+                    dmma884(ci[i][j], ai[i], br[j]);
+                }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");   // (this thread's own copies of C)
+#pragma unroll
+    for (int i = 0; i < MI; ++i) {
+        const int r = r0 + 32 * wr + 8 * i + g;
+        if (r >= M) continue;
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int c = c0 + WN * wc + 8 * j + 2 * q + e;
+                if (c >= N) continue;
+                if constexpr (PRE) {
+                    if (ep.pre_src(mat, r, c))
+                        ep.store_pre(mat, r, c, mk(cr[i][j][e], ci[i][j][e]), pre[((i * NJ + j) * 2 + e) * 256 + t]);
+                } else {
+                    ep.store(mat, r, c, mk(cr[i][j][e], ci[i][j][e]));
+                }
+            }
+    }
+}
+
 // Launch on a batch of nb matrices; returns the launch error.  Double precision runs on the
 // DMMA engine, single precision on the FP32 FMA engine.
 template <class C, int BM, class LA, class LB, class EP>
 cudaError_t launch_zgemm(cudaStream_t st, const LA& la, const LB& lb, const EP& ep, int M, int N, int K, int nb) {
     const dim3 grid((M + BM - 1) / BM, (N + ZG_BN - 1) / ZG_BN, nb);
-    if constexpr (std::is_same<C, cplx>::value) {
+    if constexpr (std::is_same<C, cplx>::value && zg_async<LA>::value && zg_async<LB>::value) {
+        auto kern = k_zgemm_async<BM, LA, LB, EP>;
+        const size_t smem = ZgAsync<BM, EP>::smem;
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        kern<<<grid, 256, smem, st>>>(la, lb, ep, M, N, K);
+    } else if constexpr (std::is_same<C, cplx>::value) {
         auto kern = k_zgemm_dmma<BM, LA, LB, EP>;
         const size_t smem = zgemm_dmma_smem<BM, EP>();
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
