@@ -1044,6 +1044,62 @@ k_larft(const typename Cx<R>::T* __restrict__ A, const typename Cx<R>::T* __rest
     for (int i = threadIdx.x; i < ORM_NB * ORM_NB; i += 128) out[i] = T[i / ORM_NB][i % ORM_NB];
 }
 
+// The same in double precision on the FP64 tensor path, one warp per block and LM_WARPS blocks per
+// CTA: G = V^H V as the three 8 x 8 tiles on and below the diagonal (both fragments of a product
+// are the same entries, 4 rows x 8 reflectors of V straight from memory), then lane q forms
+// column q of T in registers.  grid (ceil(blocks / LM_WARPS), matrices).
+// Bound: the latency of V's loads.  As dot products with a warp sum each it took 0.43 ms for
+// 4,624 matrices of order 64 and 0.11 ms for 2,304 of order 32; now 0.10 and 0.03.
+static constexpr int LM_WARPS = 4;
+__global__ void __launch_bounds__(32 * LM_WARPS)
+k_larft_mma(const cplx* __restrict__ A, const cplx* __restrict__ TAU, cplx* __restrict__ Tw, int n, int nblk) {
+    __shared__ cplx Gs[LM_WARPS][ORM_NB][ORM_NB + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+    const int j = blockIdx.x * LM_WARPS + warp;
+    if (j >= nblk) return;
+    const size_t mat = blockIdx.y;
+    const cplx* a = A + mat * (size_t)n * n;
+    const int i0 = j * ORM_NB, rows = min(i0 + ORM_NB, n - 1);
+    const int ia = i0 + g, ib = i0 + 8 + g;   // this lane's reflectors
+    double r0[2] = {0, 0}, m0[2] = {0, 0}, r1[2] = {0, 0}, m1[2] = {0, 0}, r2[2] = {0, 0}, m2[2] = {0, 0};
+    auto product = [&](double (&re)[2], double (&im)[2], cplx x, cplx y) {   // conj(x) y
+        dmma884(re, x.x, y.x);
+        dmma884(im, x.x, y.y);
+        dmma884(re, x.y, y.y);
+        dmma884(im, -x.y, y.x);
+    };
+#pragma unroll 4
+    for (int k = 0; k < rows; k += 4) {
+        const cplx x = refl_entry(a, n, ia, k + q), y = refl_entry(a, n, ib, k + q);
+        product(r0, m0, x, x);
+        product(r1, m1, y, x);
+        product(r2, m2, y, y);
+    }
+    cplx (&G)[ORM_NB][ORM_NB + 1] = Gs[warp];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        G[g][2 * q + e] = mk(r0[e], m0[e]);
+        G[8 + g][2 * q + e] = mk(r1[e], m1[e]);
+        G[8 + g][8 + 2 * q + e] = mk(r2[e], m2[e]);
+    }
+    __syncwarp();
+    // T[k][c] = -tau_k sum_{l < k} G[k][l] T[l][c], T[c][c] = tau_c, zero above the diagonal
+    const int c = lane & 15;
+    cplx t[ORM_NB];
+    const cplx tl = i0 + c <= n - 2 ? TAU[mat * n + i0 + c] : mk(0, 0);
+    cplx* out = Tw + (mat * nblk + j) * ORM_NB * ORM_NB;
+#pragma unroll
+    for (int k = 0; k < ORM_NB; ++k) {
+        const cplx tk = mk(__shfl_sync(0xffffffffu, tl.x, k), __shfl_sync(0xffffffffu, tl.y, k));
+        cplx s0 = mk(0, 0), s1 = mk(0, 0);
+#pragma unroll
+        for (int l = 0; l < k; ++l) cfma(l & 1 ? s1 : s0, G[k][l], t[l]);
+        const cplx s = cadd(s0, s1);
+        t[k] = k == c ? tk : k < c ? mk(0, 0) : cscale(cmul(tk, s), -1.0);
+        if (lane < ORM_NB) out[k * ORM_NB + c] = t[k];
+    }
+}
+
 // asynchronous global -> shared copy of one complex element (16 or 8 bytes)
 __device__ __forceinline__ void cp_async_elem(double2* smem_dst, const double2* gmem_src) {
     const unsigned dst = (unsigned)__cvta_generic_to_shared(smem_dst);
@@ -3378,7 +3434,10 @@ static int back_transform(rlmb_context* ctx, cudaStream_t st, const HeevPlan& p,
     if (p.small_bt) {
         if (n > 1) {
             RLMB_CHUNK_PROF("k_larft");
-            k_larft<R><<<dim3(p.nblk16, nb), 128, 0, st>>>(Aw, TAUw, Tw, n);
+            if constexpr (std::is_same<R, double>::value)
+                k_larft_mma<<<dim3((p.nblk16 + LM_WARPS - 1) / LM_WARPS, nb), 32 * LM_WARPS, 0, st>>>(Aw, TAUw, Tw, n,
+                                                                                                     p.nblk16);
+            else k_larft<R><<<dim3(p.nblk16, nb), 128, 0, st>>>(Aw, TAUw, Tw, n);
             RLMB_CHUNK_LAUNCHED();
         }
         const dim3 grid((n + p.ch - 1) / p.ch, nb);
