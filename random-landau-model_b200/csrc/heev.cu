@@ -253,8 +253,8 @@ __device__ __forceinline__ void reflector(const C alpha, R xnorm2, R& beta, C& t
 // tile, so that it needs neither atomics nor a cleared accumulator.
 // Bound: instruction issue (several CTAs per SM hide the chains of the reflector).  With one
 // row and 16 columns per lane, shared double atomics and eight barriers per column 4,624 matrices
-// of order 64 took 4.03 ms, 2,304 of order 32 0.69 ms and 128 of order 129 0.93 ms; now 1.99,
-// 0.29 and 0.52.
+// of order 64 took 4.03 ms, 2,304 of order 32 0.69 ms and 128 of order 129 0.93 ms; now 1.80,
+// 0.17 and 0.44.
 static constexpr int HT_PARTS_MAX = 144;
 __host__ __device__ constexpr int hetrd_pad(int m) { return (m + 15) / 16 * 16; }
 __host__ __device__ constexpr int hetrd_pn(int m) {   // elements of pn
@@ -3134,9 +3134,12 @@ __global__ void k_to_single(const cplx* __restrict__ A, cplxf* __restrict__ B, s
 }
 
 // Launch shape of k_hetrd: NT threads, as much of the leading triangle resident as fits (all
-// of it up to order ~155 in double precision).  Threads: the tiles of a pass are few (10 at
-// order 64), so 64 threads up to order 48 and 128 up to 100 with several CTAs per SM, 512 above
-// (one CTA per SM); chunks of fewer matrices than SMs take 512 from order 65 on and 256 below.
+// of it up to order ~155 in double precision).  Threads: the tiles of a pass are few (3 at order
+// 32, 10 at 64) and every warp repeats the column's scalar steps, so one warp up to order 40, 64
+// threads up to 48, 128 up to 100 with several CTAs per SM, 256 where one fits or the matrices
+// are fewer than the SMs; 512 where the sums go through atomics.  2,304 matrices of order 32 took
+// 0.26 ms with 64 threads and 0.17 with 32; 128 of order 129 0.46 with 512 and 0.44 with 256;
+// order 64 is even between 64 and 128.
 struct HetrdCfg {
     int nt;
     int tri_cap;
@@ -3145,7 +3148,7 @@ struct HetrdCfg {
 template <class R>
 static HetrdCfg hetrd_config(int m, int nb) {
     const size_t ce = 2 * sizeof(R);   // complex element
-    const int nt = nb <= 148 ? (m > 64 ? 512 : 256) : m <= 48 ? 64 : m <= 100 ? 128 : 512;
+    const int nt = m > HT_PARTS_MAX ? 512 : nb <= 148 || m > 100 ? 256 : m <= 40 ? 32 : m <= 48 ? 64 : 128;
     const size_t vec = (3 * (size_t)hetrd_pad(m) + hetrd_pn(m) + 2) * ce + 2 * (nt / 32) * sizeof(R);
     const size_t budget = 220 * 1024;
     size_t cap = budget > vec ? (budget - vec) / ce : 0;
@@ -3167,8 +3170,8 @@ static cudaError_t launch_hetrd(cudaStream_t st, int nb, typename Cx<R>::T* A, d
     const HetrdCfg c = hetrd_config<R>(m, nb);
     if (c.smem > 227 * 1024) return cudaErrorInvalidValue;
     if (m > HT_PARTS_MAX) return launch_hetrd_t<512, R, false>(c, st, nb, A, D, E, TAU, n, m);
-    const auto launch = c.nt == 64 ? launch_hetrd_t<64, R, true> : c.nt == 128 ? launch_hetrd_t<128, R, true>
-                      : c.nt == 256 ? launch_hetrd_t<256, R, true> : launch_hetrd_t<512, R, true>;
+    const auto launch = c.nt == 32 ? launch_hetrd_t<32, R, true> : c.nt == 64 ? launch_hetrd_t<64, R, true>
+                      : c.nt == 128 ? launch_hetrd_t<128, R, true> : launch_hetrd_t<256, R, true>;
     return launch(c, st, nb, A, D, E, TAU, n, m);
 }
 
