@@ -97,7 +97,8 @@ int rlmb_set_heev_config(rlmb_context* ctx, int n, int precision, int blocked, i
  * reduction / tridiagonal solve / back-transformation path above.  RLMB_SOLVER_JACOBI
  * (n <= 80): two-sided cyclic Jacobi, one CTA per matrix with the matrix and its rotations in
  * shared memory, double precision in either precision mode.  RLMB_SOLVER_AUTO: the built-in
- * choice (Jacobi up to n = 20) or the autotuner's.  rlmb_heev_solver reports the solver that
+ * choice (Jacobi up to n = 20; the mesh solves, whose results do not depend on the phases of the
+ * vectors, take the faster solver of the order, Jacobi up to n = 12) or the autotuner's.  rlmb_heev_solver reports the solver that
  * (n, precision) runs with now.  Jacobi above n = 80 returns RLMB_ERR_ARG. */
 #define RLMB_SOLVER_AUTO 0
 #define RLMB_SOLVER_HOUSEHOLDER 1

@@ -30,7 +30,10 @@ static int grow(rlmb_context* ctx, void** buf, size_t* have, size_t bytes) {
     *have = bytes;
     return RLMB_OK;
 }
-int ensure_workspace(rlmb_context* ctx, size_t bytes) { return grow(ctx, &ctx->ws, &ctx->ws_bytes, bytes); }
+// (at least 32 MB at once: a small mesh call would otherwise grow it from stage to stage)
+int ensure_workspace(rlmb_context* ctx, size_t bytes) {
+    return grow(ctx, &ctx->ws, &ctx->ws_bytes, bytes && bytes < ((size_t)32 << 20) ? (size_t)32 << 20 : bytes);
+}
 int ensure_pipe(rlmb_context* ctx, size_t bytes) { return grow(ctx, &ctx->pipe, &ctx->pipe_bytes, bytes); }
 static int ensure_io(rlmb_context* ctx, size_t bytes) { return grow(ctx, &ctx->io, &ctx->io_bytes, bytes); }
 int ensure_tma_planes(rlmb_context* ctx, size_t bytes) { return grow(ctx, &ctx->tws, &ctx->tws_bytes, bytes); }
@@ -146,14 +149,21 @@ __global__ void k_count_nonzero(const int* __restrict__ info, int count, int* __
     for (int off = 16; off > 0; off >>= 1) c += __shfl_xor_sync(0xffffffffu, c, off);
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(fail, c);
 }
-static int reset_failures(rlmb_context* ctx) {
-    if (!ctx->fail) {
-        if (cudaMalloc(reinterpret_cast<void**>(&ctx->fail), sizeof(int)) != cudaSuccess) {
-            cudaGetLastError();
-            ctx->fail = nullptr;
-            return RLMB_ERR_ALLOC;
-        }
+// The failure counter and the saved disorder stream, in one small allocation.
+int ensure_state(rlmb_context* ctx) {
+    if (ctx->fail) return RLMB_OK;
+    char* p = nullptr;
+    if (cudaMalloc(reinterpret_cast<void**>(&p), 4096) != cudaSuccess) {
+        cudaGetLastError();
+        return RLMB_ERR_ALLOC;
     }
+    ctx->fail = reinterpret_cast<int*>(p);
+    ctx->mt_state = reinterpret_cast<uint32_t*>(p + 1024);   // 626 words
+    ctx->mt_valid = 0;
+    return RLMB_OK;
+}
+static int reset_failures(rlmb_context* ctx) {
+    if (int rc = ensure_state(ctx)) return rc;
     RLMB_CUDA_TRY(cudaMemsetAsync(ctx->fail, 0, sizeof(int), ctx->stream));
     return RLMB_OK;
 }
@@ -239,7 +249,6 @@ int rlmb_destroy(rlmb_context* ctx) {
     if (ctx->io) cudaFree(ctx->io);
     if (ctx->tws) cudaFree(ctx->tws);
     if (ctx->fail) cudaFree(ctx->fail);
-    if (ctx->mt_state) cudaFree(ctx->mt_state);
     if (ctx->hlm_tables) cudaFree(ctx->hlm_tables);
     if (ctx->rlm_tables) cudaFree(ctx->rlm_tables);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
@@ -582,7 +591,7 @@ static int rlm_enqueue(rlmb_context* ctx, const RlmPlan& p, int sample0, const i
         if (int rc = launch_rlm_assemble(ctx, p.d_vmn, p.d_cmt, p.d_cjm, nullptr, nullptr, cnt * kpts,
                                          kpts, n_phi, dim, o, all_t2.data(), g + 1, static_cast<cplx*>(ctx->ws), p.d_H))
             return rc;
-        if (int rc = heevd_batched_band(ctx, reinterpret_cast<double*>(p.d_H), p.d_W, n_phi, cnt * kpts, p.d_info, o))
+        if (int rc = heevd_batched_band(ctx, reinterpret_cast<double*>(p.d_H), p.d_W, n_phi, cnt * kpts, p.d_info, o, true))
             return rc;
         if (int rc = tally_failures(ctx, p.d_info, cnt * kpts)) return rc;
         if (wfs_dir)
@@ -854,7 +863,7 @@ static int hlm_enqueue(rlmb_context* ctx, int lx, int ly, int Q, int band, int n
         const int cnt = std::min(nb, n_samples - s0);
         if (int rc = launch_hlm_vtilde(ctx, d_potentials + (size_t)s0 * ns, lx, ly, Q, cnt, d_vt)) return rc;
         if (int rc = launch_hlm_project(ctx, hb, d_vt, nullptr, g, lx, ly, Q, kpts, cnt, d_H)) return rc;
-        if (int rc = rlmb_heevd_batched(ctx, reinterpret_cast<double*>(d_H), d_W, N, cnt * kpts, d_info))
+        if (int rc = heevd_batched_band(ctx, reinterpret_cast<double*>(d_H), d_W, N, cnt * kpts, d_info, -1, true))
             return rc;
         if (int rc = tally_failures(ctx, d_info, cnt * kpts)) return rc;
         if (int rc = launch_hlm_links(ctx, hb, d_H, lx, ly, Q, g, cnt, d_U1, d_U2)) return rc;

@@ -122,7 +122,8 @@ struct rlmb_context {
     void* io;
     size_t io_bytes;
     int* fail;
-    // the device rlm disorder stream of the last call (state words + block index), for
+    // the device rlm disorder stream of the last call (state words + block index; in the
+    // allocation of `fail`), for
     // continuing it when the next call starts at the next sample
     uint32_t* mt_state;
     // set while a stream capture records this context's work: buffers may not grow then
@@ -169,8 +170,9 @@ namespace rlmb {
 // Per-kernel event timing: prof_begin records a start event on the context stream
 // before a launch, prof_end the stop event after it (no-ops unless profiling is on).
 void prof_begin(rlmb_context* ctx, const char* kernel);
-// rlmb_heevd_batched with a structure hint (band >= 0: cyclic band of that half-bandwidth).
-int heevd_batched_band(rlmb_context* ctx, double* d_a, double* d_w, int n, int batch, int* d_info, int band);
+// rlmb_heevd_batched with a structure hint (band >= 0: cyclic band of that half-bandwidth); mesh:
+// called by a mesh solve.
+int heevd_batched_band(rlmb_context* ctx, double* d_a, double* d_w, int n, int batch, int* d_info, int band, bool mesh);
 void tune_free(rlmb_context* ctx);
 void prof_end(rlmb_context* ctx);
 }  // namespace rlmb
@@ -194,5 +196,6 @@ int ensure_workspace(rlmb_context* ctx, size_t bytes);
 int ensure_tma_planes(rlmb_context* ctx, size_t bytes);
 int ensure_pipe(rlmb_context* ctx, size_t bytes);
 int ensure_pinned(rlmb_context* ctx, size_t bytes);
+int ensure_state(rlmb_context* ctx);   // fail and mt_state
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 }  // namespace rlmb

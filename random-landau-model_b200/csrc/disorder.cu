@@ -183,14 +183,8 @@ extern "C" int rlmb_rlm_disorder_device(rlmb_context* ctx, int impurity_num, dou
         return RLMB_ERR_ARG;
     if (count == 0) return RLMB_OK;
     RLMB_CUDA_TRY(cudaSetDevice(ctx->device));
-    if (!ctx->mt_state) {
-        if (cudaMalloc(reinterpret_cast<void**>(&ctx->mt_state), (MT_N + 2) * sizeof(uint32_t)) != cudaSuccess) {
-            cudaGetLastError();
-            ctx->mt_state = nullptr;
-            return RLMB_ERR_ALLOC;
-        }
-        ctx->mt_valid = 0;
-    }
+    static_assert((MT_N + 2) * sizeof(uint32_t) <= 4096 - 1024, "the context's state allocation holds the stream");
+    if (int rc = ensure_state(ctx)) return rc;
     // continue the context's saved stream when this call starts where the last one ended
     // (same seed and impurity count); otherwise every sample's CTA skips ahead on its own
     const long long first = 3LL * impurity_num * sample0;

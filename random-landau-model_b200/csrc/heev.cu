@@ -1744,7 +1744,13 @@ static constexpr int HT_BLOCKED_MIN = 256;   // orders from which the blocked re
 // .. 7e-13 at orders 640 to 2000 where divide and conquer's are to 4e-15 .. 8e-15; callers who
 // want the speed pin it (rlmb_set_tridiag_solver).
 static constexpr int DC_DEFAULT_MIN = 600;
-static constexpr int JAC_DEFAULT_MAX = 20;    // orders up to which k_jacobi is the built-in solver (measured: 2.4x the Householder path at 16, 2.1x at 20, 1.2x at 24, even at 28)
+// Orders up to which k_jacobi is the built-in solver: of the batched eigensolver (part of its
+// documented behaviour, and of the phases its callers' vectors come with), and of the mesh solves,
+// whose results are gauge invariant and which take the faster one (8,192 matrices: order 10
+// 0.29 ms against the Householder path's 0.40, order 12 0.40 against 0.45, order 13 0.54 against
+// 0.48, order 16, 8,450 matrices, 0.85 against 0.55; 81 matrices of order 12 0.105 against 0.087).
+static constexpr int JAC_DEFAULT_MAX = 20;
+static constexpr int JAC_MESH_MAX = 12;
 static constexpr int QUEUE_NT_DEFAULT = 512;   // panel queue CTAs: 512 threads, one per SM
 static constexpr int TUNE_MIN_N = 16;         // orders the autotuner tunes: TUNE_MIN_N .. TUNE_MAX_N
 static constexpr int TUNE_MAX_N = 1024;
@@ -3967,7 +3973,8 @@ static int heev_steps(const rlmb_context* ctx) { return ctx->refine_steps == 1 &
 // The batched eigensolve of rlmb_heevd_batched with a structure hint: band >= 0 declares every
 // matrix a cyclic band of that half-bandwidth (the rlm Hamiltonian), which the mixed mode's
 // refinement uses for its residual; band < 0 is a dense matrix.
-int rlmb::heevd_batched_band(rlmb_context* ctx, double* d_a, double* d_w, int n, int batch, int* d_info, int band) {
+int rlmb::heevd_batched_band(rlmb_context* ctx, double* d_a, double* d_w, int n, int batch, int* d_info, int band,
+                             bool mesh) {
     if (!ctx || !d_a || !d_w || n <= 0 || batch < 0) return RLMB_ERR_ARG;
     if (batch == 0) return RLMB_OK;
     RLMB_CUDA_TRY(cudaSetDevice(ctx->device));
@@ -3983,6 +3990,8 @@ int rlmb::heevd_batched_band(rlmb_context* ctx, double* d_a, double* d_w, int n,
                 return rc;
         }
     }
+    // (a mesh solve takes the faster solver: its results do not see the vectors' phases)
+    if (mesh && tune.jacobi < 0) tune.jacobi = n <= JAC_MESH_MAX;
     const HeevPlan plan = heev_plan(n, mixed, heev_steps(ctx), band, tune);
     const size_t per = plan.per;
     // workspace: 8 GB, or for large orders enough for two resident matrices per SM (one
@@ -4033,7 +4042,7 @@ int rlmb::heevd_batched_band(rlmb_context* ctx, double* d_a, double* d_w, int n,
 }
 
 extern "C" int rlmb_heevd_batched(rlmb_context* ctx, double* d_a, double* d_w, int n, int batch, int* d_info) {
-    return rlmb::heevd_batched_band(ctx, d_a, d_w, n, batch, d_info, -1);
+    return rlmb::heevd_batched_band(ctx, d_a, d_w, n, batch, d_info, -1, false);
 }
 
 extern "C" int rlmb_set_autotune(rlmb_context* ctx, int on) {
