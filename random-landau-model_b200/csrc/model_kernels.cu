@@ -892,6 +892,128 @@ k_hlm_links_w(const cplx* __restrict__ hb, const cplx* __restrict__ X, int lx, i
     }
 }
 
+// The same links on the FP64 tensor path (DMMA), block sizes 8 and 16: per direction every Bloch
+// block of L partners is a product Y[n][i] = sum_l U'_n[l] S[i][l], K = L, of the states with the
+// block's S, followed by the products with conj(U_n[i]).  One CTA of 16 warps per k-point; a warp
+// owns every sixteenth block and keeps its S fragments in registers for all states, which pass
+// through shared memory eight at a time (U and U', cp.async, the next eight on their way), in
+// the order that makes a block's entries contiguous.  Rows are padded by 4 entries so that the
+// two rows of a fragment's 8-lane phase hit distinct banks.
+// Bound: reading the eigenvectors (three rows of the mesh per k-point and direction) and the
+// barriers between groups of states.  k_hlm_links_w, bound by its shared-memory operands (two per
+// multiply-add), took 10.6 ms for the 4,224 k-points of the 48 x 16 lattice; this one LINKS_NEW.
+static constexpr int LM_T = 512, LM_NS = 8;
+template <int L1, int L2>
+constexpr size_t links_mma_smem() {
+    return sizeof(cplx) * ((size_t)L1 * L2 * (L1 > L2 ? L1 : L2) + 2 * 2 * LM_NS * (L1 * L2 + 4) + 16 * LM_NS);
+}
+template <int L, int NBLK>
+__device__ __forceinline__ void links_mma_dir(const cplx* __restrict__ S, cplx* __restrict__ stage, cplx* __restrict__ red,
+                                              const cplx* __restrict__ Xa, const cplx* __restrict__ Xb, int ly, int dir,
+                                              cplx* __restrict__ U) {
+    constexpr int N = L * NBLK, XS = N + 4, NB = (NBLK + 15) / 16;   // blocks per warp
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+    // S fragments: (l = 4 k + q, i = 8 it + g) of this warp's blocks
+    cplx b[NB][L / 8][L / 4];
+#pragma unroll
+    for (int u = 0; u < NB; ++u) {
+        const int beta = warp + 16 * u;
+#pragma unroll
+        for (int it = 0; it < L / 8; ++it) {
+            const int i = 8 * it + g, a = dir ? beta * ly + i : i * ly + beta;
+#pragma unroll
+            for (int k = 0; k < L / 4; ++k) b[u][it][k] = beta < NBLK ? S[a * L + 4 * k + q] : mk(0, 0);
+        }
+    }
+    auto fetch = [&](int n0, int buf) {   // states n0 .. n0 + 7 of U and U'
+        cplx* d = stage + buf * 2 * LM_NS * XS;
+        for (int i = tid; i < LM_NS * N; i += LM_T) {
+            const int s = i / N, a = i % N;
+            const int at = s * XS + (dir ? a : (a % ly) * L + a / ly);
+            if (n0 + s < N) {
+                const unsigned da = (unsigned)__cvta_generic_to_shared(d + at);
+                const unsigned db = (unsigned)__cvta_generic_to_shared(d + LM_NS * XS + at);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(da), "l"(Xa + (size_t)(n0 + s) * N + a) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(db), "l"(Xb + (size_t)(n0 + s) * N + a) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    fetch(0, 0);
+    for (int n0 = 0, buf = 0; n0 < N; n0 += LM_NS, buf ^= 1) {
+        if (n0 + LM_NS < N) fetch(n0 + LM_NS, buf ^ 1);
+        else asm volatile("cp.async.commit_group;\n" ::: "memory");
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        __syncthreads();
+        const cplx* xa = stage + buf * 2 * LM_NS * XS + g * XS;
+        const cplx* xb = xa + LM_NS * XS;
+        cplx acc = mk(0, 0);
+#pragma unroll
+        for (int u = 0; u < NB; ++u) {
+            const int beta = warp + 16 * u;
+            if (beta >= NBLK) break;
+            double cr[L / 8][2], ci[L / 8][2];
+#pragma unroll
+            for (int it = 0; it < L / 8; ++it) cr[it][0] = cr[it][1] = ci[it][0] = ci[it][1] = 0.0;
+#pragma unroll
+            for (int k = 0; k < L / 4; ++k) {
+                const cplx x = xb[beta * L + 4 * k + q];
+#pragma unroll
+                for (int it = 0; it < L / 8; ++it) {
+                    dmma884(cr[it], x.x, b[u][it][k].x);
+                    dmma884(ci[it], x.x, b[u][it][k].y);
+                    dmma884(cr[it], -x.y, b[u][it][k].y);
+                    dmma884(ci[it], x.y, b[u][it][k].x);
+                }
+            }
+#pragma unroll
+            for (int it = 0; it < L / 8; ++it)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) cfmac(acc, xa[beta * L + 8 * it + 2 * q + e], mk(cr[it][e], ci[it][e]));
+        }
+        acc = cadd(acc, shfl_xor(acc, 1));
+        acc = cadd(acc, shfl_xor(acc, 2));
+        if (q == 0) red[warp * LM_NS + g] = acc;
+        __syncthreads();
+        if (tid < LM_NS && n0 + tid < N) {
+            cplx s = mk(0, 0);
+#pragma unroll
+            for (int w = 0; w < 16; ++w) s = cadd(s, red[w * LM_NS + tid]);
+            U[n0 + tid] = s;
+        }
+        // (red is written again after the next group's first barrier, the buffers after this one)
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+}
+template <int L1, int L2>
+__global__ void __launch_bounds__(LM_T)
+k_hlm_links_mma(const cplx* __restrict__ hb, const cplx* __restrict__ X, int lx, int ly, int Q, int g,
+                cplx* __restrict__ U1, cplx* __restrict__ U2) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int N = L1 * L2;
+    const int kpts = (g + 1) * g;
+    const int job = blockIdx.x, sample = job / kpts, t = job % kpts;
+    const int t1 = t / g, t2 = t % g;
+    cplx* S = reinterpret_cast<cplx*>(smem_raw);   // [N][L]
+    cplx* stage = S + N * (L1 > L2 ? L1 : L2);      // [2][U, U'][8][N + 4]
+    cplx* red = stage + 2 * 2 * LM_NS * (N + 4);    // [16][8]
+    __shared__ cplx Dtab[LINK_MAXL];
+    const int t2n = t2 + 1 == g ? 0 : t2 + 1;       // theta_2 = g is the copy of theta_2 = 0
+    const cplx* ha = hb + ((size_t)t1 * (g + 1) + t2) * N * Q;
+    const size_t nn = (size_t)N * N;
+    const cplx* Xa = X + ((size_t)sample * kpts + t) * nn;
+    const size_t o = ((size_t)sample * kpts + t) * N;
+    if (t1 < g) {
+        build_link_S(S, Dtab, ha, hb + ((size_t)(t1 + 1) * (g + 1) + t2) * N * Q, N, L1, ly, L1, Q, 0, -1.0 / g);
+        __syncthreads();
+        links_mma_dir<L1, L2>(S, stage, red, Xa, X + ((size_t)sample * kpts + (t1 + 1) * g + t2) * nn, ly, 0, U1 + o);
+    }
+    build_link_S(S, Dtab, ha, hb + ((size_t)t1 * (g + 1) + t2n) * N * Q, N, L2, ly, L1, Q, 1, (double)(t2 - t2n) / g);
+    __syncthreads();
+    links_mma_dir<L2, L1>(S, stage, red, Xa, X + ((size_t)sample * kpts + t1 * g + t2n) * nn, ly, 1, U2 + o);
+}
+
 template <int L1, int L2>
 static int launch_links_thread(rlmb_context* ctx, const cplx* hb, const cplx* X, int lx, int ly, int Q, int g,
                                int nsamples, cplx* U1, cplx* U2) {
@@ -912,6 +1034,14 @@ template <int L1, int L2>
 static int launch_links_t(rlmb_context* ctx, const cplx* hb, const cplx* X, int lx, int ly, int Q, int g,
                           int nsamples, cplx* U1, cplx* U2) {
     const int N = lx * ly / Q;
+    if constexpr ((L1 == 8 || L1 == 16) && (L2 == 8 || L2 == 16)) {   // whole DMMA tiles, fragments in registers
+        const size_t smem = links_mma_smem<L1, L2>();
+        RLMB_CUDA_TRY(cudaFuncSetAttribute(k_hlm_links_mma<L1, L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        prof_begin(ctx, "k_hlm_links");
+        k_hlm_links_mma<L1, L2><<<nsamples * (g + 1) * g, LM_T, smem, ctx->stream>>>(hb, X, lx, ly, Q, g, U1, U2);
+        RLMB_LAUNCHED(ctx);
+        return RLMB_OK;
+    }
     const size_t smem_w = ((size_t)N * (L1 + L2) + (size_t)8 * 2 * N) * sizeof(cplx);
     if (smem_w <= 220 * 1024) {
         RLMB_CUDA_TRY(cudaFuncSetAttribute(k_hlm_links_w<L1, L2>, cudaFuncAttributeMaxDynamicSharedMemorySize,

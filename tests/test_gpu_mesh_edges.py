@@ -62,3 +62,15 @@ def test_assemble_theta_groups(n_phi, g):
         ref = orlm.assemble(p, v, cmt, cjm, int(t1[i]), int(t2[i])).reshape(n_phi, n_phi)
         assert np.abs(got[i].cpu().numpy() - ref).max() <= 1e-13 * np.abs(ref).max()
     ctx.close()
+
+
+@pytest.mark.parametrize("lx,ly,g", [(24, 8, 2), (24, 16, 3), (48, 8, 2), (48, 16, 2)])
+def test_hlm_links_block_sizes(lx, ly, g):
+    """Bloch blocks of 8 and 16 in either direction (the tensor-path link kernel)."""
+    import rlmb
+    ctx = rlmb.Context(0)
+    p = ohlm.HlmParams(lx, ly, 3, 0, g, 1, 4)
+    pots = rlmb.hlm_potentials(4, p.n_sites, 1)
+    e, c = ctx.hlm_mesh_solve(lx, ly, 3, 0, g, pots)
+    _close(e[0], c[0], ohlm.run_sample(p, pots[0]))
+    ctx.close()
