@@ -901,7 +901,7 @@ k_hlm_links_w(const cplx* __restrict__ hb, const cplx* __restrict__ X, int lx, i
 // two rows of a fragment's 8-lane phase hit distinct banks.
 // Bound: reading the eigenvectors (three rows of the mesh per k-point and direction) and the
 // barriers between groups of states.  k_hlm_links_w, bound by its shared-memory operands (two per
-// multiply-add), took 10.6 ms for the 4,224 k-points of the 48 x 16 lattice; this one LINKS_NEW.
+// multiply-add), took 10.6 ms for the 4,224 k-points of the 48 x 16 lattice; this one 5.6.
 static constexpr int LM_T = 512, LM_NS = 8;
 template <int L1, int L2>
 constexpr size_t links_mma_smem() {

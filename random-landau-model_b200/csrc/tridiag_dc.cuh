@@ -476,9 +476,9 @@ k_dc_merge(const double* __restrict__ E, const double* __restrict__ SC, double* 
                 us[(size_t)R.b * K0 + col] = R.s * ua + R.c * ub;
             }
         }
-        dc_sync(grp, gs);
         if (S <= DC_SMALL) {   // Q_new = blockdiag(Q1, Q2) U here
-            for (int idx = gt; idx < K0 * K0; idx += gs) {
+            share_sync();      // (U's columns come from every CTA that shares the subproblem)
+            for (int idx = ct; idx < K0 * K0; idx += cs) {
                 const int r = idx / K0, c = idx % K0;
                 const int k0 = r < n1 ? 0 : n1, k1 = r < n1 ? n1 : K0;
                 double acc = 0.0;

@@ -10,7 +10,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,batch,kind", [(513, 1, None), (600, 25, None), (520, 40, None), (300, 150, None),
-                                          (1030, 3, None), (513, 6, "degenerate"), (700, 26, "blocks"),
+                                          (1030, 3, None), (33, 1, None), (64, 2, None),
+                                          (7, 1, "identity"), (513, 6, "degenerate"), (700, 26, "blocks"),
                                           (640, 2, "tridiag_split")])
 def test_dc_cluster(n, batch, kind):
     import torch
