@@ -80,10 +80,11 @@ int rlmb_set_eigenvalue_pass(rlmb_context* ctx, int on);
 /* Eigensolver launch choices (no counterpart in the reference, whose solver is a library
  * call).  With autotuning on, the first eigensolve of each order n in 16..1024 and precision
  * mode on the context times every feasible configuration -- unblocked or blocked reduction,
- * 256- or 512-thread panels, register-resident or GEMM back-transformation, 64- or
- * 128-reflector blocks and 64- or 128-row tiles of the double-precision X update of the
- * latter, and for n <= 80 the batched Jacobi solver -- on copies of up to 2 x SMs of the
- * call's own matrices and keeps the fastest for later calls of that order.  rlmb_heev_config reports the configuration used for
+ * panels by the built-in rules or of 512 threads per matrix, SM-resident or GEMM
+ * back-transformation, 64- or 128-reflector blocks and 64- or 128-row tiles of the
+ * double-precision X update of the latter, either tridiagonal solver, and for n <= 80 the
+ * batched Jacobi solver -- on copies of up to 2 x SMs of the call's own matrices and keeps the
+ * fastest for later calls of that order.  rlmb_heev_config reports the configuration used for
  * (n, precision) (the tuned one, or the built-in one) and returns 1 if it was tuned or set,
  * 0 if built-in; rlmb_set_heev_config pins one (-1 / 0 = built-in choice for that item).
  * panel_threads, x_tile and bt_block 0 mean the built-in choice. */
@@ -98,8 +99,9 @@ int rlmb_set_heev_config(rlmb_context* ctx, int n, int precision, int blocked, i
  * (n <= 80): two-sided cyclic Jacobi, one CTA per matrix with the matrix and its rotations in
  * shared memory, double precision in either precision mode.  RLMB_SOLVER_AUTO: the built-in
  * choice (Jacobi up to n = 20; the mesh solves, whose results do not depend on the phases of the
- * vectors, take the faster solver of the order, Jacobi up to n = 12) or the autotuner's.  rlmb_heev_solver reports the solver that
- * (n, precision) runs with now.  Jacobi above n = 80 returns RLMB_ERR_ARG. */
+ * vectors, take the faster solver of the order, Jacobi up to n = 12) or the autotuner's.
+ * rlmb_heev_solver reports the solver that rlmb_heevd_batched runs (n, precision) with now.
+ * Jacobi above n = 80 returns RLMB_ERR_ARG. */
 #define RLMB_SOLVER_AUTO 0
 #define RLMB_SOLVER_HOUSEHOLDER 1
 #define RLMB_SOLVER_JACOBI 2

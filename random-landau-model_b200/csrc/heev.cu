@@ -1837,17 +1837,16 @@ __device__ __forceinline__ void hemv_upper(const C* __restrict__ a, int ld, int 
     }
 }
 
-// Loads of the panel pairs V, W: through L1 (ld) when one CTA owns the matrix for the whole
-// panel, around it (ld.global.cg) when other CTAs wrote them during the same launch.
-template <bool CG, class C>
+// Loads of the panel pairs V, W: around L1 (ld.global.cg), other CTAs wrote them during the same
+// launch.
+template <class C>
 __device__ __forceinline__ C pv_ld(const C* p) {
-    if constexpr (CG) return __ldcg(p);
-    else return *p;
+    return __ldcg(p);
 }
 
 // Column j of the panel (column c = m - 1 - j of the leading m x m block) of matrix mat, by
 // the NT threads of one CTA; vn, pn, coef, red: the CTA's shared work arrays.
-template <int NT, class R, bool CG>
+template <int NT, class R>
 __device__ __forceinline__ void panel_column(typename Cx<R>::T* __restrict__ A, double* __restrict__ D,
                                              double* __restrict__ E, typename Cx<R>::T* __restrict__ TAU,
                                              typename Cx<R>::T* __restrict__ PV, typename Cx<R>::T* __restrict__ PW,
@@ -1874,8 +1873,8 @@ __device__ __forceinline__ void panel_column(typename Cx<R>::T* __restrict__ A, 
         for (int q = 0; q < j; ++q) {
             const C* vq = V + (size_t)q * n;
             const C* wq = W + (size_t)q * n;
-            C u = cmul(pv_ld<CG>(vq + r), cconj(pv_ld<CG>(wq + c)));
-            cfma(u, pv_ld<CG>(wq + r), cconj(pv_ld<CG>(vq + c)));
+            C u = cmul(pv_ld(vq + r), cconj(pv_ld(wq + c)));
+            cfma(u, pv_ld(wq + r), cconj(pv_ld(vq + c)));
             x = csub(x, u);
         }
         if (r == c) x.y = 0;
@@ -1910,7 +1909,7 @@ __device__ __forceinline__ void panel_column(typename Cx<R>::T* __restrict__ A, 
         const int q = t2 >> 1;
         const C* y = (t2 & 1) ? V + (size_t)q * n : W + (size_t)q * n;
         C sd = cz<C>();
-        for (int r = lane; r < c; r += 32) cfmac(sd, pv_ld<CG>(y + r), vn[r]);
+        for (int r = lane; r < c; r += 32) cfmac(sd, pv_ld(y + r), vn[r]);
         sd = warp_sum(sd);
         if (lane == 0) coef[t2] = sd;
     }
@@ -1920,8 +1919,8 @@ __device__ __forceinline__ void panel_column(typename Cx<R>::T* __restrict__ A, 
     for (int r = tid; r < c; r += NT) {
         C x = pn[r];
         for (int q = 0; q < j; ++q) {
-            C u = cmul(pv_ld<CG>(V + (size_t)q * n + r), coef[2 * q]);
-            cfma(u, pv_ld<CG>(W + (size_t)q * n + r), coef[2 * q + 1]);
+            C u = cmul(pv_ld(V + (size_t)q * n + r), coef[2 * q]);
+            cfma(u, pv_ld(W + (size_t)q * n + r), coef[2 * q + 1]);
             x = csub(x, u);
         }
         x = cmul(tau, x);
@@ -1946,8 +1945,8 @@ __host__ __device__ constexpr size_t panel_smem(int m) {
     return (2 * (size_t)m + 2 * HP_W_MAX) * sizeof(typename Cx<R>::T) + 2 * (NT / 32) * sizeof(R);
 }
 
-// The same panel for chunks of more matrices than SMs: one resident CTA of NT threads per SM
-// (grid <= SMs) takes units (matrix, column) from a queue, unit u = claim - base = matrix
+// The panel for chunks of more matrices than SMs (see panel_waves_full): one resident CTA of NT
+// threads per SM (grid <= SMs) takes units (matrix, column) from a queue, unit u = claim - base = matrix
 // u % nb, column u / nb, so that every SM keeps NT threads of loads in flight whatever the
 // number of matrices (one CTA per matrix would leave SMs with a single CTA when the chunk has
 // between one and two matrices per SM).  Column j of a matrix needs column j - 1 (its panel
@@ -2007,7 +2006,7 @@ k_hetrd_panel_q(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, doubl
         if (u >= units || !go) break;
         __threadfence();
         const int mat = (int)(u % nb), j = (int)(u / nb);
-        panel_column<NT, R, true>(A, D, E, TAU, PV, PW, n, m, mat, j, pw, vn, pn, coef, red);
+        panel_column<NT, R>(A, D, E, TAU, PV, PW, n, m, mat, j, pw, vn, pn, coef, red);
         // every thread's writes of the column, then the release of the column count
         __threadfence();
         __syncthreads();
