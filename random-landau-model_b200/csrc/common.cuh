@@ -49,6 +49,11 @@ __device__ __forceinline__ cplx warp_sum(cplx v) {
     return v;
 }
 
+// Barrier of a thread-block cluster, in its two halves.  A CTA may touch a peer's shared memory
+// only once the peer has started, so a kernel's first such access stands behind a whole barrier.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
+
 // -------------------------------------------- single-precision complex (mixed mode)
 typedef float2 cplxf;
 __host__ __device__ __forceinline__ cplxf cadd(cplxf a, cplxf b) { return make_float2(a.x + b.x, a.y + b.y); }

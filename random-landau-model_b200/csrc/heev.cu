@@ -2024,8 +2024,8 @@ __device__ __forceinline__ void panel_sync(int P) {
     if (P == 1) {
         __syncthreads();
     } else {
-        asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        cluster_arrive();
+        cluster_wait();
     }
 }
 // the address of this CTA's shared variable p in CTA `rank` of the cluster
@@ -2254,6 +2254,7 @@ k_hetrd_panel_c(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, doubl
     typedef typename Cx<R>::T C;
     constexpr int NW = NT / 32;
     const int P = ONE ? 1 : Pr;
+    if (!ONE) cluster_arrive();   // (the wait stands before the first access to a peer's shared memory)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* ring = reinterpret_cast<C*>(smem_raw) + (threadIdx.x >> 5) * HU_RING;   // this warp's staging
     C* v = reinterpret_cast<C*>(smem_raw) + NW * HU_RING;   // [m] column / reflector
@@ -2283,6 +2284,7 @@ k_hetrd_panel_c(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, doubl
     HemvPos<C> pos{};
     int seg = 1;
     for (int r = m + tid; r < m + 32; r += NT) v[r] = cz<C>();   // (read, times zero, by the product's last blocks)
+    if (!ONE) cluster_wait();   // every CTA of the cluster has started: step -1 writes to its peers
     for (int j = -1; j < pw; ++j) {
         const int c = m - 1 - j;   // column of step j; the pass below finishes step j and starts step j + 1
         if (j >= 0) {
