@@ -211,6 +211,7 @@ k_dc_merge(const double* __restrict__ E, const double* __restrict__ SC, double* 
     const size_t mat = blockIdx.x / Y;
     const int rank = (int)(blockIdx.x % Y);
     const bool coop = Y > 1 && gs == DC_THREADS;   // the cluster shares every subproblem
+    if (coop) cluster_arrive();   // (the wait stands before the loop with the shared subproblems)
     // this thread's share of a subproblem's roots, entries of z and columns
     const int ct = coop ? rank * gs + gt : gt, cs = coop ? Y * gs : gs;
     auto share = [&](auto* p, int at, auto v) {    // p[at] = v in every CTA that shares the subproblem
@@ -226,8 +227,8 @@ k_dc_merge(const double* __restrict__ E, const double* __restrict__ SC, double* 
     };
     auto share_sync = [&]() {
         if (coop) {
-            asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-            asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+            cluster_arrive();
+            cluster_wait();
         } else {
             dc_sync(grp, gs);
         }
@@ -239,6 +240,7 @@ k_dc_merge(const double* __restrict__ E, const double* __restrict__ SC, double* 
     double* qn = Qn + mat * (size_t)n * n;
     const int nsub = (n + S - 1) / S;
     int fail = 0;
+    if (coop) cluster_wait();   // every CTA of the cluster has started: the roots go to all of them
     for (int s = coop ? 0 : rank * ng + grp; s < nsub; s += coop ? 1 : Y * ng) {
         const int o = s * S;
         const int K0 = min(S, n - o), n1 = min(S / 2, K0), n2 = K0 - n1;

@@ -24,12 +24,13 @@ def _body(file, kernel):
 
 @pytest.mark.parametrize("file,kernel,loop,remote", [
     ("heev.cu", "k_hetrd_panel_c", "for (int j = -1;", "panel_peer("),
+    ("tridiag_dc.cuh", "k_dc_merge", "for (int s = coop", "share("),
 ])
 def test_cluster_barrier_before_remote_access(file, kernel, loop, remote):
     body = _body(file, kernel)
     ahead = body[:body.index(loop)]
     assert remote in body and remote not in ahead
-    arrive, wait = ahead.find("cluster_arrive();"), ahead.find("cluster_wait();")
+    arrive, wait = ahead.find("cluster_arrive();"), ahead.rfind("cluster_wait();")
     assert 0 <= arrive < wait, "no cluster barrier before the loop with the remote accesses"
     for at in (arrive, wait):   # every CTA of a cluster passes it
         assert ahead[:at].count("{") == ahead[:at].count("}")
