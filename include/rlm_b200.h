@@ -99,7 +99,8 @@ int rlmb_set_heev_config(rlmb_context* ctx, int n, int precision, int blocked, i
  * (n <= 80): two-sided cyclic Jacobi, one CTA per matrix with the matrix and its rotations in
  * shared memory, double precision in either precision mode.  RLMB_SOLVER_AUTO: the built-in
  * choice (Jacobi up to n = 20; the mesh solves, whose results do not depend on the phases of the
- * vectors, take the faster solver of the order, Jacobi up to n = 12) or the autotuner's.
+ * vectors, take the faster solver of the order, Jacobi up to n = 12, and up to n = 20 run in double
+ * precision in either mode) or the autotuner's.
  * rlmb_heev_solver reports the solver that rlmb_heevd_batched runs (n, precision) with now.
  * Jacobi above n = 80 returns RLMB_ERR_ARG. */
 #define RLMB_SOLVER_AUTO 0

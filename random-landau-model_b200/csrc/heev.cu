@@ -1749,6 +1749,9 @@ static constexpr int DC_DEFAULT_MIN = 600;
 // whose results are gauge invariant and which take the faster one (8,192 matrices: order 10
 // 0.29 ms against the Householder path's 0.40, order 12 0.40 against 0.45, order 13 0.54 against
 // 0.48, order 16, 8,450 matrices, 0.85 against 0.55; 81 matrices of order 12 0.105 against 0.087).
+// Up to JAC_DEFAULT_MAX the mixed mode's mesh solves take the double-precision path too: it is the
+// more accurate and the faster one (calls of 81 and 8,450 matrices: order 20, double precision,
+// 0.17 and 1.06 ms; order 21, mixed, 0.38 and 6.5, double precision 0.18 and 1.11).
 static constexpr int JAC_DEFAULT_MAX = 20;
 static constexpr int JAC_MESH_MAX = 12;
 static constexpr int QUEUE_NT_DEFAULT = 512;   // panel queue CTAs: 512 threads, one per SM
@@ -3979,7 +3982,7 @@ int rlmb::heevd_batched_band(rlmb_context* ctx, double* d_a, double* d_w, int n,
     if (!ctx || !d_a || !d_w || n <= 0 || batch < 0) return RLMB_ERR_ARG;
     if (batch == 0) return RLMB_OK;
     RLMB_CUDA_TRY(cudaSetDevice(ctx->device));
-    const bool mixed = ctx->precision == RLMB_PRECISION_MIXED;
+    bool mixed = ctx->precision == RLMB_PRECISION_MIXED;
     HeevTune tune;
     {
         TuneCache& tc = tune_cache(ctx);
@@ -3991,8 +3994,12 @@ int rlmb::heevd_batched_band(rlmb_context* ctx, double* d_a, double* d_w, int n,
                 return rc;
         }
     }
-    // (a mesh solve takes the faster solver: its results do not see the vectors' phases)
-    if (mesh && tune.jacobi < 0) tune.jacobi = n <= JAC_MESH_MAX;
+    // a mesh solve takes the faster solver (its results do not see the vectors' phases) where the
+    // batched eigensolver runs Jacobi, and like Jacobi in double precision in either mode
+    if (mesh && tune.jacobi < 0 && n <= JAC_DEFAULT_MAX) {
+        tune.jacobi = n <= JAC_MESH_MAX;
+        mixed = false;
+    }
     const HeevPlan plan = heev_plan(n, mixed, heev_steps(ctx), band, tune);
     const size_t per = plan.per;
     // workspace: 8 GB, or for large orders enough for two resident matrices per SM (one
