@@ -256,7 +256,8 @@ int rlmb_rlm_mesh_solve_device(rlmb_context* ctx, int n_phi, double quanta_conce
  * reference's write_wfs (diag_wrappers/wfs_file.cpp:2-11; rlm/main_rlm_gpu.cu:187,227 with
  * -DwfsIO): n_phi*n_phi complex doubles, column k = eigenvector k.  The reference keeps only
  * two theta_1 lines (file names use theta_1 % 2); here every line is kept.  Eigenvector
- * phases are those of this solver (any phase is an eigenvector; FHS is gauge invariant). */
+ * phases are those of rlmb_heevd_batched on the same matrices (any phase is an eigenvector; FHS is
+ * gauge invariant). */
 int rlmb_rlm_mesh_export(rlmb_context* ctx, int n_phi, double quanta_concentration,
                          double impurity_concentration, int n_mesh, unsigned long seed, int sample,
                          const char* dir, double* h_energies, double* h_chern);

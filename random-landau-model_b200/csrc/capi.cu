@@ -588,13 +588,26 @@ static int rlm_enqueue(rlmb_context* ctx, const RlmPlan& p, int sample0, const i
         if (int rc = launch_rlm_potential(ctx, dx, dy, ds, nimp, cnt, p.d_cmn, dim, o, static_cast<cplx*>(ctx->ws),
                                           p.d_vmn))
             return rc;
-        if (int rc = launch_rlm_assemble(ctx, p.d_vmn, p.d_cmt, p.d_cjm, nullptr, nullptr, cnt * kpts,
-                                         kpts, n_phi, dim, o, all_t2.data(), g + 1, static_cast<cplx*>(ctx->ws), p.d_H))
-            return rc;
-        if (int rc = heevd_batched_band(ctx, reinterpret_cast<double*>(p.d_H), p.d_W, n_phi, cnt * kpts, p.d_info, o, true))
-            return rc;
-        if (int rc = tally_failures(ctx, p.d_info, cnt * kpts)) return rc;
-        if (wfs_dir)
+        auto assemble = [&]() {
+            return launch_rlm_assemble(ctx, p.d_vmn, p.d_cmt, p.d_cjm, nullptr, nullptr, cnt * kpts, kpts, n_phi, dim, o,
+                                       all_t2.data(), g + 1, static_cast<cplx*>(ctx->ws), p.d_H);
+        };
+        auto solve = [&](bool mesh) {
+            if (int rc = heevd_batched_band(ctx, reinterpret_cast<double*>(p.d_H), p.d_W, n_phi, cnt * kpts, p.d_info, o, mesh))
+                return rc;
+            return tally_failures(ctx, p.d_info, cnt * kpts);
+        };
+        if (int rc = assemble()) return rc;
+        // an export's files hold the batched eigensolver's vectors, phases included; its results are a
+        // mesh solve's, which at some small orders runs another solver
+        const bool apart = wfs_dir && heev_mesh_differs(ctx, n_phi);
+        if (apart) {
+            if (int rc = solve(false)) return rc;
+            if (int rc = export_wfs(ctx, p.d_H, n_phi, g, wfs_dir)) return rc;
+            if (int rc = assemble()) return rc;
+        }
+        if (int rc = solve(true)) return rc;
+        if (wfs_dir && !apart)
             if (int rc = export_wfs(ctx, p.d_H, n_phi, g, wfs_dir)) return rc;   // one sample (cnt == 1)
         cplx* d_U1 = p.d_U;
         cplx* d_U2 = p.d_U + (size_t)n_phi * kpts * nb;

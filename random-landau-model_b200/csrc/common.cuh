@@ -178,6 +178,8 @@ void prof_begin(rlmb_context* ctx, const char* kernel);
 // rlmb_heevd_batched with a structure hint (band >= 0: cyclic band of that half-bandwidth); mesh:
 // called by a mesh solve.
 int heevd_batched_band(rlmb_context* ctx, double* d_a, double* d_w, int n, int batch, int* d_info, int band, bool mesh);
+// Whether a mesh solve of order n may run another solver than the batched eigensolver.
+bool heev_mesh_differs(rlmb_context* ctx, int n);
 void tune_free(rlmb_context* ctx);
 void prof_end(rlmb_context* ctx);
 }  // namespace rlmb

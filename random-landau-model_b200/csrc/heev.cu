@@ -3974,6 +3974,12 @@ static int autotune(rlmb_context* ctx, int n, bool mixed, int refine_steps, int 
 // Refinement steps handed to heev_plan: 1 or 2, or 3 for one step followed by the eigenvalue pass.
 static int heev_steps(const rlmb_context* ctx) { return ctx->refine_steps == 1 && ctx->rq_pass ? 3 : ctx->refine_steps; }
 
+bool rlmb::heev_mesh_differs(rlmb_context* ctx, int n) {
+    const TuneCache& tc = tune_cache(ctx);
+    const auto it = tc.find({n, ctx->precision == RLMB_PRECISION_MIXED ? 1 : 0});
+    return n > JAC_MESH_MAX && n <= JAC_DEFAULT_MAX && (it == tc.end() || it->second.t.jacobi < 0);
+}
+
 // The batched eigensolve of rlmb_heevd_batched with a structure hint: band >= 0 declares every
 // matrix a cyclic band of that half-bandwidth (the rlm Hamiltonian), which the mixed mode's
 // refinement uses for its residual; band < 0 is a dense matrix.
