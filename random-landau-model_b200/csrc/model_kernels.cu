@@ -240,13 +240,14 @@ int launch_rlm_assemble(rlmb_context* ctx, const cplx* vmn, const cplx* cmt, con
 
 // rlm links: U1(t1,t2) = <u_n(t1,t2)|u_n(t1+1,t2)>, U2(t1,t2) = <u_n(t1,t2)|u_n(t1,t2+1)>
 // on the full (g+1)^2 mesh of one sample, eigenvector n of k-point t at X[(t*N + n)*N].
+// blockIdx.x = k-point * chunks + chunk of 8 states (a batch may hold more than 65,535 k-points).
 __global__ void __launch_bounds__(256)
-k_rlm_links(const cplx* __restrict__ X, int n_phi, int g, cplx* __restrict__ U1, cplx* __restrict__ U2) {
-    const int kpt = blockIdx.y;                 // sample * (g+1)^2 + t1*(g+1) + t2
+k_rlm_links(const cplx* __restrict__ X, int n_phi, int g, int chunks, cplx* __restrict__ U1, cplx* __restrict__ U2) {
+    const int kpt = blockIdx.x / chunks;        // sample * (g+1)^2 + t1*(g+1) + t2
     const int per = (g + 1) * (g + 1);
     const int sample = kpt / per, t = kpt % per, t1 = t / (g + 1), t2 = t % (g + 1);
     const int lane = threadIdx.x & 31;
-    const int state = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int state = blockIdx.x % chunks * 8 + (threadIdx.x >> 5);
     if (state >= n_phi) return;
     const size_t nn = (size_t)n_phi * n_phi;
     const cplx* a = X + (size_t)kpt * nn + (size_t)state * n_phi;
@@ -268,9 +269,9 @@ k_rlm_links(const cplx* __restrict__ X, int n_phi, int g, cplx* __restrict__ U1,
 }
 
 int launch_rlm_links(rlmb_context* ctx, const cplx* X, int n_phi, int g, int nsamples, cplx* U1, cplx* U2) {
-    dim3 grid((n_phi + 7) / 8, nsamples * (g + 1) * (g + 1));
+    const int chunks = (n_phi + 7) / 8;
     prof_begin(ctx, "k_rlm_links");
-    k_rlm_links<<<grid, 256, 0, ctx->stream>>>(X, n_phi, g, U1, U2);
+    k_rlm_links<<<(unsigned)chunks * nsamples * (g + 1) * (g + 1), 256, 0, ctx->stream>>>(X, n_phi, g, chunks, U1, U2);
     RLMB_LAUNCHED(ctx);
     return RLMB_OK;
 }
@@ -502,14 +503,15 @@ int launch_hlm_basis_expand(rlmb_context* ctx, const cplx* hb, int lx, int ly, i
     return RLMB_OK;
 }
 
-// Sublattice Fourier transform of the on-site potential (one sample per blockIdx.y):
+// Sublattice Fourier transform of the on-site potential (blockIdx.x = sample * chunks + chunk of 128
+// entries):
 //   Vt[q][dx][dy] = sum_{m'<Lx', j<ly} V[j*lx + Q m' + q] e^{+i 2pi (dx m'/Lx' + dy j/ly)}
 // so that W^H diag(V) W [a][b] = sum_q conj(hhat_a[q]) hhat_b[q] Vt[q][kxa-kxb][kya-kyb]:
 // the twist phases of the two columns cancel in the difference.
-__global__ void k_hlm_vtilde(const double* __restrict__ pot, int lx, int ly, int Q, cplx* __restrict__ vt) {
+__global__ void k_hlm_vtilde(const double* __restrict__ pot, int lx, int ly, int Q, int chunks, cplx* __restrict__ vt) {
     const int Lxp = lx / Q, N = Lxp * ly, ns = lx * ly;
-    const int sample = blockIdx.y;
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    const int sample = blockIdx.x / chunks;
+    const int idx = blockIdx.x % chunks * blockDim.x + threadIdx.x;
     if (idx >= ns) return;
     const int q = idx / N, rest = idx % N, dx = rest / ly, dy = rest % ly;
     const double* V = pot + (size_t)sample * ns;
@@ -531,17 +533,16 @@ __global__ void k_hlm_vtilde(const double* __restrict__ pot, int lx, int ly, int
 }
 
 int launch_hlm_vtilde(rlmb_context* ctx, const double* pot, int lx, int ly, int Q, int nsamples, cplx* vt) {
-    const int ns = lx * ly;
-    dim3 grid((ns + 127) / 128, nsamples);
+    const int chunks = (lx * ly + 127) / 128;
     prof_begin(ctx, "k_hlm_vtilde");
-    k_hlm_vtilde<<<grid, 128, 0, ctx->stream>>>(pot, lx, ly, Q, vt);
+    k_hlm_vtilde<<<(unsigned)chunks * nsamples, 128, 0, ctx->stream>>>(pot, lx, ly, Q, chunks, vt);
     RLMB_LAUNCHED(ctx);
     return RLMB_OK;
 }
 
 // Projected H of k-point (sample, t) into column-major buf[b*N + a] = H[a][b].
-// blockIdx.y = sample * kpts + k, kpts = number of mesh k-points given in tlist.
-// Thread = row a (its Bloch indices and hhat_a held in registers); the CTA's x-slice of the
+// blockIdx.x = (sample * kpts + k) * slices + slice, kpts = number of mesh k-points given in tlist.
+// Thread = row a (its Bloch indices and hhat_a held in registers); the CTA's slice of the
 // columns b is walked in order, so consecutive threads store consecutive entries of a
 // column (coalesced) and every per-b quantity is a warp-uniform shared-memory broadcast.
 // The sublattice offsets (kxa - kxb) mod Lx', (kya - kyb) mod ly advance by wrap-around
@@ -551,13 +552,13 @@ int launch_hlm_vtilde(rlmb_context* ctx, const double* pot, int lx, int ly, int 
 template <int QT>
 __global__ void __launch_bounds__(256)
 k_hlm_project(const cplx* __restrict__ hb, const cplx* __restrict__ vt, const int* __restrict__ tlist,
-              int g, int lx, int ly, int Qr, int kpts, cplx* __restrict__ H) {
+              int g, int lx, int ly, int Qr, int kpts, int slices, cplx* __restrict__ H) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int Q = QT > 0 ? QT : Qr;
     const int Lxp = lx / Q, N = Lxp * ly, ns = lx * ly;
     cplx* sh = reinterpret_cast<cplx*>(smem_raw);   // [N*Q] hhat of this k-point
     cplx* sv = sh + (size_t)N * Q;                   // [ns]  Vt of this sample
-    const int job = blockIdx.y;
+    const int job = blockIdx.x / slices, slice = blockIdx.x % slices;
     const int sample = job / kpts, k = job % kpts;
     const int t = tlist ? tlist[k] : k / g * (g + 1) + k % g;   // (without a list: the mesh, theta_2 < g)
     for (int i = threadIdx.x; i < N * Q; i += blockDim.x) sh[i] = hb[(size_t)t * N * Q + i];
@@ -565,8 +566,8 @@ k_hlm_project(const cplx* __restrict__ hb, const cplx* __restrict__ vt, const in
     __syncthreads();
     cplx* h = H + (size_t)job * N * N;
     // columns of this CTA: [b0, b1)
-    const int per = (N + gridDim.x - 1) / gridDim.x;
-    const int b0 = blockIdx.x * per, b1 = min(N, b0 + per);
+    const int per = (N + slices - 1) / slices;
+    const int b0 = slice * per, b1 = min(N, b0 + per);
     if (b0 >= b1) return;
     for (int a = threadIdx.x; a < N; a += blockDim.x) {
         const int kxa = a / ly, kya = a % ly;
@@ -611,10 +612,9 @@ int launch_hlm_project(rlmb_context* ctx, const cplx* hb, const cplx* vt, const 
     auto kern = Q == 1 ? k_hlm_project<1> : Q == 2 ? k_hlm_project<2> : Q == 3 ? k_hlm_project<3>
               : Q == 4 ? k_hlm_project<4> : k_hlm_project<0>;
     RLMB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int bx = std::max(1, std::min(N / 32, 16));   // column slices of >= 32 columns per k-point
-    dim3 grid(bx, kpts * nsamples);
+    const int slices = std::max(1, std::min(N / 32, 16));   // column slices of >= 32 columns per k-point
     prof_begin(ctx, "k_hlm_project");
-    kern<<<grid, 256, smem, ctx->stream>>>(hb, vt, d_tlist, g, lx, ly, Q, kpts, H);
+    kern<<<(unsigned)slices * kpts * nsamples, 256, smem, ctx->stream>>>(hb, vt, d_tlist, g, lx, ly, Q, kpts, slices, H);
     RLMB_LAUNCHED(ctx);
     return RLMB_OK;
 }
