@@ -220,7 +220,7 @@ __device__ __forceinline__ C hetrd_sum(const C* __restrict__ part, int m, int r)
 }
 
 // Householder reflector of zlarfg for (alpha, x) with ||x||^2 = xnorm2: returns beta, tau
-// and the scale applied to x.
+// and the scale applied to x.  Called by whole warps with the same arguments in every lane.
 template <class C, class R>
 __device__ __forceinline__ void reflector(const C alpha, R xnorm2, R& beta, C& tau, C& scal) {
     if (xnorm2 == 0 && alpha.y == 0) {
@@ -231,11 +231,17 @@ __device__ __forceinline__ void reflector(const C alpha, R xnorm2, R& beta, C& t
     }
     const R nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xnorm2);
     beta = alpha.x >= 0 ? -nrm : nrm;
-    const R ib = 1 / beta;   // (every warp computes the reflector: two divisions, not four)
-    tau = cm<C>((beta - alpha.x) * ib, -alpha.y * ib);
+    // tau = ((beta - alpha.x) / beta, -alpha.y / beta), scal = conj(den) / |den|^2: every warp computes
+    // the reflector, its lanes one of the four quotients each, so that a warp issues one division
+    // (quotients, not products with an inverse: that of a denormal |den|^2 overflows)
     const C den = cm<C>(alpha.x - beta, alpha.y);
-    const R id = 1 / cabs2(den);
-    scal = cm<C>(den.x * id, -den.y * id);
+    const int k = threadIdx.x & 3;
+    const R num = k == 0 ? beta - alpha.x : k == 1 ? -alpha.y : k == 2 ? den.x : -den.y;
+    const R quo = num / (k < 2 ? beta : cabs2(den));
+    tau.x = __shfl_sync(0xffffffffu, quo, 0);
+    tau.y = __shfl_sync(0xffffffffu, quo, 1);
+    scal.x = __shfl_sync(0xffffffffu, quo, 2);
+    scal.y = __shfl_sync(0xffffffffu, quo, 3);
 }
 
 // Unblocked reduction A = Q T Q^H (zhetd2, uplo='U') with look-ahead: step i's rank-2
