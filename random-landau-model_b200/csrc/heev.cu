@@ -399,15 +399,18 @@ __host__ __device__ constexpr int tri_columns(int n) { return n <= 384 ? (n + 31
 // Sturm count by the leading principal minors of T - x I,
 //   p_j = (d_j - x) p_{j-1} - e_{j-1}^2 p_{j-2},   p_{-1} = 1:
 // the number of sign changes along p_{-1}, p_0, ..., p_{n-1} is the number of eigenvalues below
-// x (Sturm); a zero minor counts as a change.  The pair (p_j, p_{j-1}) is kept in range by exact
-// powers of two, every fourth step (|T| is about 1, so four steps grow it by less than 2^12);
-// signs, zeros and exponents are looked at as integers, which leaves the FP64 pipe the
-// recurrences.  The derivatives p_j' ride along for the Newton step ratio = p_{n-1}/p_{n-1}'.
-static constexpr int STURM_BIG = (1023 + 400) << 20, STURM_SMALL = (1023 - 400) << 20;
+// x (Sturm).  A minor below 2^-100 of its predecessor is replaced by -2^-100 of that, a change of T by
+// less than 2^-99 |T| that keeps the recurrence from dying out where couplings or d_j - x vanish
+// (a replacement of fixed size would be a large change of T after smaller minors).  The pair
+// (p_j, p_{j-1}) is kept in range by exact powers of two, every fourth step: |T| is about 1, so
+// four steps grow it by less than 2^12, and p_j, above 2^-500 where the pair is in range, shrinks by
+// 2^400 at most.  Signs, sizes and exponents are looked at as integers, which leaves the FP64 pipe
+// the recurrences.  The derivatives p_j' ride along for the Newton step ratio = p_{n-1}/p_{n-1}'.
+static constexpr int STURM_BIG = (1023 + 400) << 20, STURM_SMALL = (1023 - 400) << 20, STURM_TINY = 100 << 20;
 __device__ __forceinline__ double sturm_nonzero(double pn, double p) {
-    const int hi = __double2hiint(pn), lo = __double2loint(pn);
-    // a zero becomes 2^-700 of the sign opposite to p's
-    return ((hi << 1) | lo) == 0 ? __hiloint2double((~__double2hiint(p) & 0x80000000) | ((1023 - 700) << 20), 0) : pn;
+    const int hp = __double2hiint(p);
+    return (__double2hiint(pn) & 0x7fffffff) < (hp & 0x7fffffff) - STURM_TINY
+               ? __hiloint2double((hp ^ 0x80000000) - STURM_TINY, __double2loint(p)) : pn;
 }
 __device__ __forceinline__ int sturm_change(double a, double b) {
     return (int)((unsigned)(__double2hiint(a) ^ __double2hiint(b)) >> 31);
