@@ -938,12 +938,14 @@ k_tridiag(const double* __restrict__ D, const double* __restrict__ E, double* __
                     x2 = x1;
                     x1 = xj;
                 }
-                // modified Gram-Schmidt against the earlier members of the cluster
-                for (int q = k0; q < k; ++q) {
-                    double dot = 0.0;
-                    for (int j = 0; j < n; ++j) dot += z[(size_t)j * n + q] * z[(size_t)j * n + k];
-                    for (int j = 0; j < n; ++j) z[(size_t)j * n + k] -= dot * z[(size_t)j * n + q];
-                }
+                // modified Gram-Schmidt against the earlier members of the cluster, twice: what is left of an
+                // iterate that is all but one of them is the first pass's rounding
+                for (int pass = 0; pass < 2; ++pass)
+                    for (int q = k0; q < k; ++q) {
+                        double dot = 0.0;
+                        for (int j = 0; j < n; ++j) dot += z[(size_t)j * n + q] * z[(size_t)j * n + k];
+                        for (int j = 0; j < n; ++j) z[(size_t)j * n + k] -= dot * z[(size_t)j * n + q];
+                    }
                 for (int j = 0; j < n; ++j) xmax = fmax(xmax, fabs(z[(size_t)j * n + k]));
                 if (xmax < dtpcrt) continue;   // not yet amplified enough
                 if (++nrmchk < 3) continue;    // two extra iterations after acceptance
