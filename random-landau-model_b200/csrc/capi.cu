@@ -166,28 +166,45 @@ int ensure_state(rlmb_context* ctx) {
     ctx->mt_valid = 0;
     return RLMB_OK;
 }
-static int reset_failures(rlmb_context* ctx) {
-    if (int rc = ensure_state(ctx)) return rc;
-    RLMB_CUDA_TRY(cudaMemsetAsync(ctx->fail, 0, sizeof(int), ctx->stream));
+static int reset_failures(rlmb_context* ctx, int* fail) {
+    RLMB_CUDA_TRY(cudaMemsetAsync(fail, 0, sizeof(int), ctx->stream));
     return RLMB_OK;
 }
-static int tally_failures(rlmb_context* ctx, const int* d_info, int count) {
-    if (count <= 0) return RLMB_OK;
-    k_count_nonzero<<<std::min((count + 255) / 256, 1024), 256, 0, ctx->stream>>>(d_info, count, ctx->fail);
+static int tally_failures(rlmb_context* ctx, const int* d_info, int count, int* fail) {
+    prof_begin(ctx, "k_count_nonzero");
+    k_count_nonzero<<<std::min((count + 255) / 256, 1024), 256, 0, ctx->stream>>>(d_info, count, fail);
     RLMB_LAUNCHED(ctx);
     return RLMB_OK;
 }
-// Small host-bound results travel through the context's pinned buffer (a copy into pageable
-// memory would block on the spot): the failure count in its first 256 bytes, results after it.
-static constexpr size_t PINNED_HEAD = 256;
-static constexpr size_t PINNED_RESULTS_MAX = (size_t)64 << 20;
 // Synchronises the context stream and returns the call's status: the failure count, if any.
 static int finish_call(rlmb_context* ctx) {
-    if (int rc = ensure_pinned(ctx, PINNED_HEAD)) return rc;
-    int* h = static_cast<int*>(ctx->pinned);
-    RLMB_CUDA_TRY(cudaMemcpyAsync(h, ctx->fail, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    int h = 0;
+    RLMB_CUDA_TRY(cudaMemcpyAsync(&h, ctx->fail, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     RLMB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    return *h > 0 ? *h : RLMB_OK;
+    return h > 0 ? h : RLMB_OK;
+}
+// The same for results on their way to the host: d_res holds cnt energies, cnt Chern numbers and
+// the failure count, back to back.  Small ones come in one copy: each copy into pageable memory
+// waits on its own (12 us; pinned memory would save 2 of them and take 1 to 3 ms to allocate).
+static constexpr size_t RESULTS_AT_ONCE = (size_t)256 << 10;
+static constexpr size_t PINNED_RESULTS_MAX = (size_t)64 << 20;   // staging of a call of several batches
+static int finish_results(rlmb_context* ctx, const double* d_res, size_t cnt, double* energies, double* chern) {
+    const size_t bytes = cnt * sizeof(double);
+    int fail = 0;
+    if (2 * bytes <= RESULTS_AT_ONCE) {
+        std::vector<double> h(2 * cnt + 1);
+        RLMB_CUDA_TRY(cudaMemcpyAsync(h.data(), d_res, 2 * bytes + sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        RLMB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+        std::memcpy(energies, h.data(), bytes);
+        std::memcpy(chern, h.data() + cnt, bytes);
+        std::memcpy(&fail, h.data() + 2 * cnt, sizeof(int));
+    } else {
+        RLMB_CUDA_TRY(cudaMemcpyAsync(energies, d_res, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        RLMB_CUDA_TRY(cudaMemcpyAsync(chern, d_res + cnt, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        RLMB_CUDA_TRY(cudaMemcpyAsync(&fail, d_res + 2 * cnt, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        RLMB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    }
+    return fail > 0 ? fail : RLMB_OK;
 }
 
 static bool hlm_args_ok(int lx, int ly, int Q, int band, int g) {
@@ -533,7 +550,7 @@ static int rlm_prepare(rlmb_context* ctx, int n_phi, double qc, double ic, int n
         need<cplx>(bytes, nn * kpts * nb);
         need<double>(bytes, (size_t)n_phi * kpts * nb);
         need<cplx>(bytes, 2 * (size_t)n_phi * kpts * nb);
-        need<double>(bytes, 2 * (size_t)n_phi * nb);
+        need<double>(bytes, 2 * (size_t)n_phi * nb + 1);   // energies, Chern numbers, failure count
         return need<int>(bytes, (size_t)kpts * nb);
     };
     const bool held = n_samples * per_sample <= MESH_BUDGET_MAX && pipe_bytes(n_samples) <= ctx->pipe_bytes;
@@ -557,7 +574,7 @@ static int rlm_prepare(rlmb_context* ctx, int n_phi, double qc, double ic, int n
     p->d_H = cv.take<cplx>(nn * kpts * nb);
     p->d_W = cv.take<double>((size_t)n_phi * kpts * nb);
     p->d_U = cv.take<cplx>(2 * (size_t)n_phi * kpts * nb);
-    p->d_out = cv.take<double>(2 * (size_t)n_phi * nb);
+    p->d_out = cv.take<double>(2 * (size_t)n_phi * nb + 1);
     p->d_info = cv.take<int>((size_t)kpts * nb);
     // (the V_mn partial sums and the assembly's theta_2 slabs, in turn)
     if (int rc = ensure_workspace(ctx, std::max(rlm_potential_ws_elems(nimp, nb, dim),
@@ -571,9 +588,9 @@ static int rlm_prepare(rlmb_context* ctx, int n_phi, double qc, double ic, int n
 // from device memory, for a captured graph), energies / chern n_samples * n_phi values each,
 // in device memory if dev_out, else in host memory: in `staged` (pinned; per batch its energies,
 // then its Chern numbers) if given.  No host round trips: eigensolve failures are tallied on
-// the device.
+// the device, in *fail.
 static int rlm_enqueue(rlmb_context* ctx, const RlmPlan& p, int sample0, const int* d_sample0, double* energies,
-                       double* chern, bool dev_out, const char* wfs_dir, double* staged) {
+                       double* chern, bool dev_out, const char* wfs_dir, double* staged, int* fail) {
     const int n_phi = p.n_phi, nimp = p.nimp, nb = p.nb, kpts = p.kpts, g = p.g, dim = p.dim, o = p.o;
     std::vector<int> all_t2(g + 1);
     for (int t = 0; t <= g; ++t) all_t2[t] = t;
@@ -599,7 +616,7 @@ static int rlm_enqueue(rlmb_context* ctx, const RlmPlan& p, int sample0, const i
         auto solve = [&](bool mesh) {
             if (int rc = heevd_batched_band(ctx, reinterpret_cast<double*>(p.d_H), p.d_W, n_phi, cnt * kpts, p.d_info, o, mesh))
                 return rc;
-            return tally_failures(ctx, p.d_info, cnt * kpts);
+            return tally_failures(ctx, p.d_info, cnt * kpts, fail);
         };
         if (int rc = assemble()) return rc;
         // an export's files hold the batched eigensolver's vectors, phases included; its results are a
@@ -648,14 +665,23 @@ static int rlm_mesh(rlmb_context* ctx, int n_phi, double qc, double ic, int n_me
     RLMB_CUDA_TRY(cudaSetDevice(ctx->device));
     RlmPlan p;
     if (int rc = rlm_prepare(ctx, n_phi, qc, ic, n_mesh, seed, n_samples, &p)) return rc;
-    if (int rc = reset_failures(ctx)) return rc;
+    if (!dev_out && p.nb == n_samples) {   // a single batch's results are read where they lie
+        const size_t cnt = (size_t)n_phi * n_samples;
+        int* fail = reinterpret_cast<int*>(p.d_out + 2 * cnt);
+        if (int rc = reset_failures(ctx, fail)) return rc;
+        if (int rc = rlm_enqueue(ctx, p, sample0, nullptr, p.d_out, p.d_out + cnt, true, wfs_dir, nullptr, fail)) return rc;
+        return finish_results(ctx, p.d_out, cnt, energies, chern);
+    }
+    if (int rc = ensure_state(ctx)) return rc;
+    if (int rc = reset_failures(ctx, ctx->fail)) return rc;
+    // (several batches: through pinned memory, so that no copy holds up the next batch's launches)
     const size_t results = 2 * (size_t)n_phi * n_samples;
     double* staged = nullptr;
-    if (!dev_out && !wfs_dir && results * sizeof(double) <= PINNED_RESULTS_MAX) {   // (an export uses the pinned buffer)
-        if (int rc = ensure_pinned(ctx, PINNED_HEAD + results * sizeof(double))) return rc;
-        staged = reinterpret_cast<double*>(static_cast<char*>(ctx->pinned) + PINNED_HEAD);
+    if (!dev_out && results * sizeof(double) <= PINNED_RESULTS_MAX) {
+        if (int rc = ensure_pinned(ctx, results * sizeof(double))) return rc;
+        staged = static_cast<double*>(ctx->pinned);
     }
-    if (int rc = rlm_enqueue(ctx, p, sample0, nullptr, energies, chern, dev_out, wfs_dir, staged)) return rc;
+    if (int rc = rlm_enqueue(ctx, p, sample0, nullptr, energies, chern, dev_out, wfs_dir, staged, ctx->fail)) return rc;
     const int rc = finish_call(ctx);
     if (rc >= 0 && staged)
         for (int s0 = 0; s0 < n_samples; s0 += p.nb) {
@@ -768,9 +794,9 @@ int rlmb_rlm_fss_graph_create(int device, const int* n_phi, int count, double qc
         if (cudaMalloc(reinterpret_cast<void**>(&o.d_e), 2 * (size_t)n_samples * n_phi[i] * sizeof(double)) != cudaSuccess)
             return fail(RLMB_ERR_ALLOC);
         if ((rc = rlm_prepare(o.ctx, n_phi[i], qc, ic, n_mesh, seed, n_samples, &o.plan))) return fail(rc);
-        if ((rc = reset_failures(o.ctx))) return fail(rc);
+        if ((rc = ensure_state(o.ctx)) || (rc = reset_failures(o.ctx, o.ctx->fail))) return fail(rc);
         if ((rc = rlm_enqueue(o.ctx, o.plan, 0, f->d_sample0, o.d_e, o.d_e + (size_t)n_samples * n_phi[i], true,
-                              nullptr, nullptr)))
+                              nullptr, nullptr, o.ctx->fail)))
             return fail(rc);
         if ((rc = finish_call(o.ctx)) < 0) return fail(rc);
     }
@@ -786,7 +812,8 @@ int rlmb_rlm_fss_graph_create(int device, const int* n_phi, int count, double qc
         o.ctx->frozen = 1;
         if (cudaMemsetAsync(o.ctx->fail, 0, sizeof(int), o.ctx->stream) != cudaSuccess) rc = RLMB_ERR_CUDA;
         if (rc == RLMB_OK)
-            rc = rlm_enqueue(o.ctx, o.plan, 0, f->d_sample0, o.d_e, o.d_e + (size_t)n_samples * n_phi[i], true, nullptr, nullptr);
+            rc = rlm_enqueue(o.ctx, o.plan, 0, f->d_sample0, o.d_e, o.d_e + (size_t)n_samples * n_phi[i], true, nullptr, nullptr,
+                             o.ctx->fail);
         o.ctx->frozen = 0;
         if (rc == RLMB_OK && (cudaEventRecord(o.done, o.ctx->stream) != cudaSuccess ||
                               cudaStreamWaitEvent(f->origin, o.done, 0) != cudaSuccess))
@@ -840,9 +867,10 @@ int rlmb_rlm_fss_graph_destroy(rlmb_fss_graph* f) {
 }
 
 // --------------------------------------------------------------------- hlm pipeline
-// The stream-ordered work of an hlm mesh call (set-up included).
+// The stream-ordered work of an hlm mesh call (set-up included); eigensolve failures are tallied in
+// *fail, or in the context's counter (null).
 static int hlm_enqueue(rlmb_context* ctx, int lx, int ly, int Q, int band, int n_mesh, const double* d_potentials,
-                       int n_samples, double* d_energies, double* d_chern) {
+                       int n_samples, double* d_energies, double* d_chern, int* fail) {
     if (!ctx || !hlm_args_ok(lx, ly, Q, band, n_mesh) || n_samples < 0 ||
         (n_samples > 0 && (!d_potentials || !d_energies || !d_chern)))
         return RLMB_ERR_ARG;
@@ -875,14 +903,18 @@ static int hlm_enqueue(rlmb_context* ctx, int lx, int ly, int Q, int band, int n
     cplx* d_U1 = cv.take<cplx>((size_t)N * kpts * nb);
     cplx* d_U2 = cv.take<cplx>((size_t)N * kpts * nb);
     int* d_info = cv.take<int>((size_t)kpts * nb);
-    if (int rc = reset_failures(ctx)) return rc;
+    if (!fail) {
+        if (int rc = ensure_state(ctx)) return rc;
+        fail = ctx->fail;
+    }
+    if (int rc = reset_failures(ctx, fail)) return rc;
     for (int s0 = 0; s0 < n_samples; s0 += nb) {
         const int cnt = std::min(nb, n_samples - s0);
         if (int rc = launch_hlm_vtilde(ctx, d_potentials + (size_t)s0 * ns, lx, ly, Q, cnt, d_vt)) return rc;
         if (int rc = launch_hlm_project(ctx, hb, d_vt, nullptr, g, lx, ly, Q, kpts, cnt, d_H)) return rc;
         if (int rc = heevd_batched_band(ctx, reinterpret_cast<double*>(d_H), d_W, N, cnt * kpts, d_info, -1, true))
             return rc;
-        if (int rc = tally_failures(ctx, d_info, cnt * kpts)) return rc;
+        if (int rc = tally_failures(ctx, d_info, cnt * kpts, fail)) return rc;
         if (int rc = launch_hlm_links(ctx, hb, d_H, lx, ly, Q, g, cnt, d_U1, d_U2)) return rc;
         if (int rc = launch_plaquettes(ctx, d_U1, d_U2, d_W, N, g, cnt, 1, d_energies + (size_t)s0 * N,
                                        d_chern + (size_t)s0 * N))
@@ -894,7 +926,7 @@ static int hlm_enqueue(rlmb_context* ctx, int lx, int ly, int Q, int band, int n
 int rlmb_hlm_mesh_solve_device(rlmb_context* ctx, int lx, int ly, int Q, int band, int n_mesh,
                                const double* d_potentials, int n_samples, double* d_energies,
                                double* d_chern) {
-    if (int rc = hlm_enqueue(ctx, lx, ly, Q, band, n_mesh, d_potentials, n_samples, d_energies, d_chern)) return rc;
+    if (int rc = hlm_enqueue(ctx, lx, ly, Q, band, n_mesh, d_potentials, n_samples, d_energies, d_chern, nullptr)) return rc;
     return n_samples == 0 ? RLMB_OK : finish_call(ctx);
 }
 
@@ -906,31 +938,16 @@ int rlmb_hlm_mesh_solve(rlmb_context* ctx, int lx, int ly, int Q, int band, int 
     if (n_samples == 0) return RLMB_OK;
     RLMB_CUDA_TRY(cudaSetDevice(ctx->device));
     const int N = lx * ly / Q, ns = lx * ly;
-    const size_t io = ((size_t)ns + 2 * (size_t)N) * n_samples;
+    const size_t cnt = (size_t)N * n_samples, io = (size_t)ns * n_samples + 2 * cnt + 1;
     if (int rc = ensure_io(ctx, io * sizeof(double))) return rc;   // grow-only staging, kept by the context
     double* d_pot = static_cast<double*>(ctx->io);
-    double* d_e = d_pot + (size_t)ns * n_samples;
-    double* d_c = d_e + (size_t)N * n_samples;
+    double* d_res = d_pot + (size_t)ns * n_samples;   // energies, Chern numbers, failure count
     RLMB_CUDA_TRY(cudaMemcpyAsync(d_pot, h_potentials, (size_t)ns * n_samples * sizeof(double), cudaMemcpyHostToDevice,
                                   ctx->stream));
-    if (int rc = hlm_enqueue(ctx, lx, ly, Q, band, n_mesh, d_pot, n_samples, d_e, d_c)) return rc;
-    const size_t cnt = (size_t)N * n_samples, bytes = cnt * sizeof(double);
-    const bool staged = 2 * bytes <= PINNED_RESULTS_MAX;
-    if (staged) {   // energies and Chern numbers lie back to back
-        if (int rc = ensure_pinned(ctx, PINNED_HEAD + 2 * bytes)) return rc;
-        RLMB_CUDA_TRY(cudaMemcpyAsync(static_cast<char*>(ctx->pinned) + PINNED_HEAD, d_e, 2 * bytes,
-                                      cudaMemcpyDeviceToHost, ctx->stream));
-    } else {
-        RLMB_CUDA_TRY(cudaMemcpyAsync(h_energies, d_e, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-        RLMB_CUDA_TRY(cudaMemcpyAsync(h_chern, d_c, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    }
-    const int rc = finish_call(ctx);
-    if (rc >= 0 && staged) {
-        const double* r = reinterpret_cast<const double*>(static_cast<char*>(ctx->pinned) + PINNED_HEAD);
-        std::memcpy(h_energies, r, bytes);
-        std::memcpy(h_chern, r + cnt, bytes);
-    }
-    return rc;
+    if (int rc = hlm_enqueue(ctx, lx, ly, Q, band, n_mesh, d_pot, n_samples, d_res, d_res + cnt,
+                             reinterpret_cast<int*>(d_res + 2 * cnt)))
+        return rc;
+    return finish_results(ctx, d_res, cnt, h_energies, h_chern);
 }
 
 }  // extern "C"
