@@ -3382,7 +3382,19 @@ static int tridiagonalise(rlmb_context* ctx, cudaStream_t st, const HeevPlan& p,
         const int qper = qnt == 256 ? 2 : 1;   // resident queue CTAs per SM
         const bool queue = p.panel_nt == 0 && n > 512 && nb > sms && (p.queue_pinned || !panel_waves_full<R>(n, nb)) &&
                            (qnt == 512 ? panel_smem<512, R>(n) <= 227 * 1024 : panel_smem<256, R>(n) <= 113 * 1024);
-        if (queue) {
+        // chunks of few matrices: a cluster of CTAs per matrix; otherwise one CTA per matrix,
+        // with the pinned number of threads if there is one
+        PanelShape shape{};
+        if (p.panel_nt == 0 && !queue) shape = panel_shape<R>(n, nb);
+        // Where neither runs and the vectors leave the rings of k_hetrd_panel_c no room for 512 threads
+        // (double precision: above order 3000; no cluster fits above 5080), the queue's kernel, whose
+        // loads need no rings, takes the panels until the leading block has shrunk enough.  With the 256 to
+        // 64 threads that fit, eigensolves of 100 matrices of order 4000 took 7.4 s, now 6.4, one of order
+        // 5600 12.7 s, now 3.5, and one of 6300 20.1, now 9.8.
+        auto too_long = [](int order) { return panel_c_smem<512, R>(order, 1) > 227 * 1024; };
+        const bool long_queue = p.panel_nt == 0 && n > 512 && !queue && shape.P == 0 && too_long(n) && qnt == 512 &&
+                                panel_smem<512, R>(n) <= 227 * 1024;
+        if (queue || long_queue) {
             const void* qk = qnt == 256 ? (const void*)k_hetrd_panel_q<256, R> : (const void*)k_hetrd_panel_q<512, R>;
             const size_t smem = qnt == 256 ? panel_smem<256, R>(n) : panel_smem<512, R>(n);
             if (cudaFuncSetAttribute(qk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
@@ -3391,24 +3403,21 @@ static int tridiagonalise(rlmb_context* ctx, cudaStream_t st, const HeevPlan& p,
         const int grid = std::min(nb, qper * sms);
         // the queue's counters, and its abort flag, which k_panel_abort_info reads in every case
         if (cudaMemsetAsync(Q, 0, (8 + (size_t)nb) * sizeof(int), st) != cudaSuccess) return RLMB_ERR_CUDA;
-        // chunks of few matrices: a cluster of CTAs per matrix; otherwise one CTA per matrix,
-        // with the pinned number of threads if there is one
-        PanelShape shape{};
-        if (p.panel_nt == 0 && !queue) shape = panel_shape<R>(n, nb);
         for (int k = 0; k < p.npanels; ++k) {
             RLMB_CHUNK_PROF("k_hetrd_panel");
+            const bool by_queue = queue || (long_queue && too_long(m));
+            if (k > 0 && (shape.P > 0 ? shape.nt < 512 : long_queue && by_queue)) {   // (the vectors have shrunk)
+                const PanelShape wider = panel_shape<R>(m, nb);
+                if (wider.P > 0) shape = wider;
+            }
             if (shape.P > 0) {
-                if (shape.nt < 512 && k > 0) {   // (the vectors have shrunk: a wider CTA may fit by now)
-                    const PanelShape wider = panel_shape<R>(m, nb);
-                    if (wider.P > 0) shape = wider;
-                }
                 const auto launch = shape.nt == 512 ? launch_panel_c<512, R>
                                   : shape.nt == 384 ? launch_panel_c<384, R> : launch_panel_c<256, R>;
                 if (launch(st, A, D, E, TAU, PV, PWb, n, m, pw, nb, shape.P) != cudaSuccess) return RLMB_ERR_CUDA;
-            } else if (queue && qnt == 256) {
+            } else if (by_queue && qnt == 256) {
                 k_hetrd_panel_q<256, R><<<grid, 256, panel_smem<256, R>(n), st>>>(
                     A, D, E, TAU, PV, PWb, n, m, pw, nb, Q, (long long)k * ((long long)nb * pw + grid), k * pw, info);
-            } else if (queue) {
+            } else if (by_queue) {
                 k_hetrd_panel_q<512, R><<<grid, 512, panel_smem<512, R>(n), st>>>(
                     A, D, E, TAU, PV, PWb, n, m, pw, nb, Q, (long long)k * ((long long)nb * pw + grid), k * pw, info);
             } else {
