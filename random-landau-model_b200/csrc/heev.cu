@@ -626,8 +626,10 @@ k_tridiag(const double* __restrict__ D, const double* __restrict__ E, double* __
     double* e2 = e + n;                                 // [n]
     double* lam = e2 + n;                               // [n]
     int* leader = reinterpret_cast<int*>(lam + n);      // [n] first index of k's cluster
-    __shared__ double s_red[4][T / 32];
+    __shared__ double s_gx[T + 1];                      // (first the warps' parts of the norms, then grid points)
     __shared__ int s_fail;
+    static_assert(4 * (T / 32) <= T + 1, "s_gx holds the norms' parts");
+    double (*s_red)[T / 32] = reinterpret_cast<double (*)[T / 32]>(s_gx);
     const int tid = threadIdx.x;
     const size_t mat = blockIdx.x;
     const int sub = blockIdx.y, subs = gridDim.y;
@@ -727,7 +729,6 @@ k_tridiag(const double* __restrict__ D, const double* __restrict__ E, double* __
     // one collective pass first: Sturm counts at the T+1 equally spaced points of
     // the Gershgorin interval (count 0 at its left end, n at its right end), so that every
     // eigenvalue starts from the grid cell holding it instead of the whole interval
-    __shared__ double s_gx[T + 1];
     __shared__ int s_gc[T + 1];
     {
         const int t = tid;
@@ -3778,6 +3779,13 @@ static int heev_chunk(rlmb_context* ctx, cudaStream_t st, const HeevPlan& p, cpl
         return RLMB_OK;
     }
     if (p.smem_tri > 227 * 1024) return RLMB_ERR_ARG;
+    // (the last orders before that do not fit beside k_tridiag's own arrays: refused before any work)
+    if (!p.dc && n > 6000 &&
+        (cudaFuncSetAttribute(k_tridiag<1, TRI_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem_tri) != cudaSuccess ||
+         cudaFuncSetAttribute(k_tridiag<2, TRI_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem_tri) != cudaSuccess)) {
+        cudaGetLastError();
+        return RLMB_ERR_CUDA;
+    }
     if (!p.mixed) {
         cplx* TAUw = reinterpret_cast<cplx*>(base + p.off_tau * B);
         cplx* Xw = reinterpret_cast<cplx*>(base + p.off_x * B);
