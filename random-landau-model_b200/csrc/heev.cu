@@ -262,7 +262,9 @@ __device__ __forceinline__ void reflector(const C alpha, R xnorm2, R& beta, C& t
 // of order 64 took 4.03 ms, 2,304 of order 32 0.69 ms and 128 of order 129 0.93 ms; now 1.80,
 // 0.17 and 0.44.
 static constexpr int HT_PARTS_MAX = 144;
-__host__ __device__ constexpr int hetrd_pad(int m) { return (m + 15) / 16 * 16; }
+// vectors are read up to the next multiple of 16, times zero; with sums by atomics, where shared memory
+// sets the largest order, that may be the next array
+__host__ __device__ constexpr int hetrd_pad(int m) { return m <= HT_PARTS_MAX ? (m + 15) / 16 * 16 : m; }
 __host__ __device__ constexpr int hetrd_pn(int m) {   // elements of pn
     return m <= HT_PARTS_MAX ? 16 * (hetrd_pad(m) / 16) * (hetrd_pad(m) / 16 + 1) : hetrd_pad(m);
 }
@@ -278,10 +280,10 @@ k_hetrd(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, double* __res
     C* vn = v + mp;                           // [mp] the next one / column buffer
     C* w = vn + mp;                           // [mp] w of step i
     C* pn = w + mp;                           // [hetrd_pn(m)] A' v
-    C* alpha = pn + hetrd_pn(m);              // [1]
-    R* normp = reinterpret_cast<R*>(alpha + 1);   // [NW] parts of the column's norm
+    C* alpha = pn + hetrd_pn(m);              // [1] (PARTS; else the entry of pn after the column's)
+    R* normp = reinterpret_cast<R*>(alpha + (PARTS ? 1 : 0));   // [NW] parts of the column's norm
     R* quadp = normp + NW;                    // [NW] parts of v^H A' v
-    C* tri = reinterpret_cast<C*>(smem_raw) + ((3 * mp + hetrd_pn(m) + 1) + (2 * NW * (int)sizeof(R) + (int)sizeof(C) - 1) / (int)sizeof(C));
+    C* tri = reinterpret_cast<C*>(smem_raw) + 3 * mp + hetrd_pn(m) + (PARTS ? 1 : 0) + 2 * NW * sizeof(R) / sizeof(C);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const size_t mat = blockIdx.x;
     GlobalStore<C> gs{A + mat * (size_t)n * n, n};
@@ -309,6 +311,7 @@ k_hetrd(typename Cx<R>::T* __restrict__ A, double* __restrict__ D, double* __res
             __syncthreads();
         }
         // (1) w of step i, and column i brought up to date with it
+        if (!PARTS) alpha = pn + min(i + 1, m - 1);
         R q2 = 0;
 #pragma unroll
         for (int k = 0; k < NW; ++k) q2 += quadp[k];
@@ -3171,7 +3174,7 @@ template <class R>
 static HetrdCfg hetrd_config(int m, int nb) {
     const size_t ce = 2 * sizeof(R);   // complex element
     const int nt = m > HT_PARTS_MAX ? 512 : nb <= 148 || m > 100 ? 256 : m <= 40 ? 32 : m <= 48 ? 64 : 128;
-    const size_t vec = (3 * (size_t)hetrd_pad(m) + hetrd_pn(m) + 2) * ce + 2 * (nt / 32) * sizeof(R);
+    const size_t vec = (3 * (size_t)hetrd_pad(m) + hetrd_pn(m) + (m > HT_PARTS_MAX ? 0 : 2)) * ce + 2 * (nt / 32) * sizeof(R);
     const size_t budget = 220 * 1024;
     size_t cap = budget > vec ? (budget - vec) / ce : 0;
     cap = std::min(cap, (size_t)m * (m + 1) / 2);
@@ -3778,7 +3781,9 @@ static int heev_chunk(rlmb_context* ctx, cudaStream_t st, const HeevPlan& p, cpl
         RLMB_CHUNK_LAUNCHED();
         return RLMB_OK;
     }
-    if (p.smem_tri > 227 * 1024) return RLMB_ERR_ARG;
+    if ((p.mixed ? hetrd_config<float>(p.m_tail, nb) : hetrd_config<double>(p.m_tail, nb)).smem > 227 * 1024 ||
+        p.smem_tri > 227 * 1024)
+        return RLMB_ERR_ARG;
     // (the last orders before that do not fit beside k_tridiag's own arrays: refused before any work)
     if (!p.dc && n > 6000 &&
         (cudaFuncSetAttribute(k_tridiag<1, TRI_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem_tri) != cudaSuccess ||

@@ -42,3 +42,21 @@ def test_orders_beyond_are_refused(n):
     _ok = ctx.heevd(_hermitian(40)[None].contiguous())   # the context works on
     assert bool(torch.isfinite(_ok).all())
     ctx.close()
+
+
+def test_unblocked_limit():
+    """The unblocked reduction pinned: four vectors of 16-byte entries in shared memory, up to order 3628;
+    above, an argument error before any work."""
+    import torch
+
+    import rlmb
+    ctx = rlmb.Context(0)
+    for n in (3628, 3629):
+        ctx.set_heev_config(n, 0, -1, 0, 0, 0)
+    _check(ctx, 3628)
+    a = _hermitian(3629)[None].contiguous()
+    before = a.clone()
+    with pytest.raises(rlmb.RlmbError, match="status -1"):
+        ctx.heevd(a)
+    assert torch.equal(a, before)
+    ctx.close()
