@@ -86,30 +86,36 @@ __global__ void k_vmn_reduce(const cplx* __restrict__ partial, const cplx* __res
     vmn[idx] = cmul(sum, coeff_mn[mn]);
 }
 
+// Samples whose partial sums are held at once: 256 MB of them (a sample of few tiles has up to 37
+// splits), within the grid's z extent, at least one.
+static int vmn_group(int nsplit, int nsamples, int dim) {
+    const size_t sample = (size_t)nsplit * dim * dim * sizeof(cplx);
+    const size_t most = std::min<size_t>(((size_t)256 << 20) / sample, 65535 / nsplit);
+    return (int)std::max<size_t>(1, std::min<size_t>(most, nsamples));
+}
 int launch_rlm_potential(rlmb_context* ctx, const double* x, const double* y, const double* s,
                          int nimp, int nsamples, const cplx* coeff_mn, int dim, int off_head,
                          cplx* partial_ws, cplx* vmn) {
     const int chunk = vmn_chunk(nimp, dim), nsplit = (nimp + chunk - 1) / chunk;
     const int nt = (dim + VMN_T - 1) / VMN_T;
-    const int per = std::max(1, 65535 / nsplit);   // samples per launch (grid z extent)
+    const int per = vmn_group(nsplit, nsamples, dim);
     for (int s0 = 0; s0 < nsamples; s0 += per) {
-        const dim3 g(nt, nt, std::min(per, nsamples - s0) * nsplit);
-        const size_t o = (size_t)s0 * nimp;
+        const int ns = std::min(per, nsamples - s0);
+        const size_t o = (size_t)s0 * nimp, dd = (size_t)dim * dim;
         prof_begin(ctx, "k_vmn_partial");
-        k_vmn_partial<<<g, 256, 0, ctx->stream>>>(x + o, y + o, s + o, nimp, dim, off_head, nsplit, chunk,
-                                                  partial_ws + (size_t)s0 * nsplit * dim * dim);
+        k_vmn_partial<<<dim3(nt, nt, ns * nsplit), 256, 0, ctx->stream>>>(x + o, y + o, s + o, nimp, dim, off_head, nsplit,
+                                                                         chunk, partial_ws);
+        RLMB_LAUNCHED(ctx);
+        prof_begin(ctx, "k_vmn_reduce");
+        k_vmn_reduce<<<(unsigned)((dd * ns + 255) / 256), 256, 0, ctx->stream>>>(partial_ws, coeff_mn, dim, nsplit, ns,
+                                                                                vmn + s0 * dd);
         RLMB_LAUNCHED(ctx);
     }
-    const size_t total = (size_t)dim * dim * nsamples;
-    prof_begin(ctx, "k_vmn_reduce");
-    k_vmn_reduce<<<(unsigned)((total + 255) / 256), 256, 0, ctx->stream>>>(partial_ws, coeff_mn, dim,
-                                                                          nsplit, nsamples, vmn);
-    RLMB_LAUNCHED(ctx);
     return RLMB_OK;
 }
 size_t rlm_potential_ws_elems(int nimp, int nsamples, int dim) {
     const int chunk = vmn_chunk(nimp, dim), nsplit = (nimp + chunk - 1) / chunk;
-    return (size_t)nsamples * nsplit * dim * dim;
+    return (size_t)vmn_group(nsplit, nsamples, dim) * nsplit * dim * dim;
 }
 
 // H(theta_1, theta_2) (rlm/hamiltonian_rlm_cpu.cpp:14-48).  For k >= j:

@@ -98,3 +98,28 @@ def test_results_of_several_batches():
     ctx.rlm_mesh_solve_device(n, 1.0, 16.0, 16, 5, 0, de, dc)
     assert np.array_equal(e, de.cpu().numpy()) and np.array_equal(c, dc.cpu().numpy())
     ctx.close()
+
+
+def test_potential_of_many_samples():
+    """V_mn of 3,000 samples of 2,064 impurities on 47 x 47 coefficients, 33 splits of 35 kB each: its
+    scratch is bounded (3.5 GB at once otherwise), the sums are those of a call of one sample."""
+    import torch
+
+    import rlmb
+    ctx = rlmb.Context(0)
+    samples, nimp, o = 3000, 2064, 23
+    dim = 2 * o + 1
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    x, y, s = (torch.rand((samples, nimp), dtype=torch.float64, device="cuda", generator=gen) for _ in range(3))
+    cmn = torch.randn((dim, dim), dtype=torch.complex128, device="cuda", generator=gen)
+    ctx.rlm_potential(x[:1], y[:1], s[:1], cmn, o)   # (loads the kernels)
+    torch.cuda.empty_cache()
+    out = torch.empty((samples, dim * dim), dtype=torch.complex128, device="cuda")   # as large as the call's own
+    before = _free()
+    del out
+    v = ctx.rlm_potential(x, y, s, cmn, o)
+    assert before - _free() <= 300 << 20
+    for k in (0, 1, 503, 504, samples - 1):
+        one = ctx.rlm_potential(x[k:k + 1].contiguous(), y[k:k + 1].contiguous(), s[k:k + 1].contiguous(), cmn, o)
+        assert torch.equal(v[k].reshape(-1), one.reshape(-1))
+    ctx.close()
