@@ -1034,22 +1034,22 @@ static int launch_links_thread(rlmb_context* ctx, const cplx* hb, const cplx* X,
     return RLMB_OK;
 }
 
-// Warp-per-state links where their shared memory fits (the transposed S blocks and two
-// staged rows per warp), else the thread-per-state kernel.
+// Blocks of 8 and 16 are whole DMMA tiles; else warp-per-state links where their shared memory fits
+// (the transposed S blocks and two staged rows per warp), else the thread-per-state kernel.
 template <int L1, int L2>
 static int launch_links_t(rlmb_context* ctx, const cplx* hb, const cplx* X, int lx, int ly, int Q, int g,
                           int nsamples, cplx* U1, cplx* U2) {
-    const int N = lx * ly / Q;
-    if constexpr ((L1 == 8 || L1 == 16) && (L2 == 8 || L2 == 16)) {   // whole DMMA tiles, fragments in registers
+    if constexpr ((L1 == 8 || L1 == 16) && (L2 == 8 || L2 == 16)) {
         const size_t smem = links_mma_smem<L1, L2>();
         RLMB_CUDA_TRY(cudaFuncSetAttribute(k_hlm_links_mma<L1, L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         prof_begin(ctx, "k_hlm_links");
         k_hlm_links_mma<L1, L2><<<nsamples * (g + 1) * g, LM_T, smem, ctx->stream>>>(hb, X, lx, ly, Q, g, U1, U2);
         RLMB_LAUNCHED(ctx);
         return RLMB_OK;
-    }
-    const size_t smem_w = ((size_t)N * (L1 + L2) + (size_t)8 * 2 * N) * sizeof(cplx);
-    if (smem_w <= 220 * 1024) {
+    } else {
+        const int N = lx * ly / Q;
+        const size_t smem_w = ((size_t)N * (L1 + L2) + (size_t)8 * 2 * N) * sizeof(cplx);
+        if (smem_w > 220 * 1024) return launch_links_thread<L1, L2>(ctx, hb, X, lx, ly, Q, g, nsamples, U1, U2);
         RLMB_CUDA_TRY(cudaFuncSetAttribute(k_hlm_links_w<L1, L2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)smem_w));
         prof_begin(ctx, "k_hlm_links");
@@ -1057,7 +1057,6 @@ static int launch_links_t(rlmb_context* ctx, const cplx* hb, const cplx* X, int 
         RLMB_LAUNCHED(ctx);
         return RLMB_OK;
     }
-    return launch_links_thread<L1, L2>(ctx, hb, X, lx, ly, Q, g, nsamples, U1, U2);
 }
 
 int launch_hlm_links(rlmb_context* ctx, const cplx* hb, const cplx* X, int lx, int ly, int Q, int g,
