@@ -2555,7 +2555,9 @@ static PanelShape panel_shape(int m, int nb) {
 // One CTA per matrix (k_hetrd_panel_c without a cluster): 512 threads, or 256 or 128 with two
 // or four CTAs per SM, which between them keep the SM busier through each other's chains of
 // small steps.  A wave of 148 k matrices takes about 1, 1.8 and 3.4 units of time for k = 1, 2
-// and 4 (orders 256 to 640), the last one of several counts in part.  Panels in double
+// and 4 (orders 256 to 640), the last one of several counts in part, but a second wave of one
+// CTA per SM nearly whole: 149 matrices of order 400 take 21.1 ms with 512 threads and 18.2 with 256
+// (the eigensolve), 200 23.3 and 20.6.  Panels in double
 // precision, against a kernel with one row and 8 columns per lane and seven barriers per column:
 // order 256, 592 matrices 9.64 -> 8.00 ms (128 threads), order 512, 592 matrices 51.3 -> 45.2
 // (128), 296 matrices 25.8 -> 23.8 (256), order 1000, 100 matrices 78.4 -> 63.6 (512); in
@@ -2574,7 +2576,8 @@ static int panel_threads(int m, int nb, int pinned) {
         if (per_sm < 1 || smem[i] > 227 * 1024 || (pinned && nt > pinned)) continue;
         if (pinned) return nt;
         const double waves = (double)nb / (148.0 * per_sm);
-        const double cost = (per_sm == 1 << i ? unit[i] : unit[i] / (1 << i) * per_sm * 1.3) * (waves <= 1.0 ? 1.0 : waves + 0.35);
+        const double cost = (per_sm == 1 << i ? unit[i] : unit[i] / (1 << i) * per_sm * 1.3) *
+                            (waves <= 1.0 ? 1.0 : std::max(waves + 0.35, 1.0 + 0.85 / per_sm));
         if (best == 0 || cost < best_cost) {
             best = nt;
             best_cost = cost;
@@ -2584,13 +2587,14 @@ static int panel_threads(int m, int nb, int pinned) {
 }
 // One CTA per matrix rather than the panel queue for more matrices than SMs: where two 256-thread
 // CTAs fit an SM (order 1200 at most, above which the queue is even) and their waves of 296 are
-// at least 80 % full (a single wave always).  Order 600, 592 matrices 101.6 -> 73.5 ms, 200
-// 34.5 -> 31.6; order 1000, 296 matrices 180.2 -> 144.8, 200 122.6 -> 116.5; but order 800, 300
-// matrices 102.5 -> 113.7.
+// at least 80 % full, a single wave 60 %: eigensolves of 149 matrices of order 520 take 36.6 ms by
+// the queue and 38.4 by 256 threads, 160 38.8 and 39.5, 180 43.0 and 41.8; of order 1100 273 and
+// 290, 292 and 303, 325.5 and 324.5.  Panels of order 600, 592 matrices 101.6 -> 73.5 ms; of order
+// 1000, 296 matrices 180.2 -> 144.8; but order 800, 300 matrices 102.5 -> 113.7.
 template <class R>
 static bool panel_waves_full(int m, int nb) {
     const int waves = (nb + 295) / 296;
-    return m <= 1200 && panel_c_smem<256, R>(m, 1) <= 113 * 1024 && (waves == 1 || nb >= 0.8 * 296 * waves);
+    return m <= 1200 && panel_c_smem<256, R>(m, 1) <= 113 * 1024 && nb >= (waves == 1 ? 0.6 : 0.8) * 296 * waves;
 }
 template <int NT, class R>
 static cudaError_t launch_panel_one(cudaStream_t st, typename Cx<R>::T* A, double* D, double* E, typename Cx<R>::T* TAU,
