@@ -1277,11 +1277,11 @@ k_ormtr(const typename Cx<R>::T* __restrict__ A, const typename Cx<R>::T* __rest
 //   X -= V W      a warp takes 8-row tiles, W's fragments in registers
 // Column c of row r of X and V sits at c ^ om_swz(r), so that the 8 lanes of a 16-byte phase hit
 // distinct banks in every fragment: 2 columns x 4 rows (W's operands), 4 even columns x 2 rows
-// (X as the accumulator), 4 columns x 2 rows (V in the last product).
+// (X in the accumulator's layout), 4 columns x 2 rows (V in the last product).
 // 256 threads where two CTAs or more fit an SM, 512 where X and V leave room for one.
 // Bound: the DMMA pipe (8 n^3 flops) and, between the products, barriers and V's staging.
 // (order 256: the pipe is 57 % busy).  k_ormtr took 2.76 ms for 4,624 matrices of order 64 and
-// 0.34 ms for 2,304 of order 32; this kernel 0.65 and 0.07.  Against the GEMM form (X read twice
+// 0.34 ms for 2,304 of order 32; this kernel 0.66 and 0.07.  Against the GEMM form (X read twice
 // and written once per 64 reflectors), T factors included: order 256, 1,408 matrices 14.5 ->
 // 11.0 ms, order 380, 296 matrices 8.6 -> 7.3 ms.
 static constexpr int OM_TS = ORM_NB + 2;   // row stride of T
@@ -1392,16 +1392,17 @@ k_ormtr_mma(const cplx* __restrict__ A, const cplx* __restrict__ Tw, const doubl
                     cplx* xp = xs + (r0 + g) * CW;
                     const int k0 = (8 * c + 2 * q) ^ sg, k1 = k0 ^ 1;
                     const cplx x0 = xp[k0], x1 = xp[k1];
-                    double cr[2] = {x0.x, x1.x}, ci[2] = {x0.y, x1.y};
+                    // (summed apart: accumulated onto X, every DMMA would round at X's size)
+                    double cr[2] = {0, 0}, ci[2] = {0, 0};
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        dmma884(cr, -v[k].x, b[k][c].x);
-                        dmma884(ci, -v[k].x, b[k][c].y);
-                        dmma884(cr, v[k].y, b[k][c].y);
-                        dmma884(ci, -v[k].y, b[k][c].x);
+                        dmma884(cr, v[k].x, b[k][c].x);
+                        dmma884(ci, v[k].x, b[k][c].y);
+                        dmma884(cr, -v[k].y, b[k][c].y);
+                        dmma884(ci, v[k].y, b[k][c].x);
                     }
-                    xp[k0] = mk(cr[0], ci[0]);
-                    xp[k1] = mk(cr[1], ci[1]);
+                    xp[k0] = mk(x0.x - cr[0], x0.y - ci[0]);
+                    xp[k1] = mk(x1.x - cr[1], x1.y - ci[1]);
                 }
             }
         }

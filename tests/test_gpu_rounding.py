@@ -1,0 +1,31 @@
+"""Rounding of the resident back-transformation and of the unblocked reduction, as means over many
+random matrices (which vary by 1 %), in double precision: as with the kernels that summed on
+the FP64 FMA pipe."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _solve(n, batch, tridiag):
+    import torch
+
+    import rlmb
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    h = torch.randn(batch, n, n, dtype=torch.complex128, device="cuda", generator=gen)
+    h = (h + h.mH) / 2
+    ctx = rlmb.Context(0)
+    ctx.set_tridiag_solver(n, getattr(ctx, tridiag))
+    a = h.transpose(1, 2).contiguous()
+    w = ctx.heevd(a)
+    ctx.close()
+    return h, w, a.transpose(1, 2)
+
+
+# ||X^H X - 1|| with divide and conquer's vectors (orthogonal to 5e-15) in: 2.50e-14 and 2.97e-14 with
+# X in registers, and 6 %.  Accumulated onto X: 2.79e-14 and 3.39e-14.
+@pytest.mark.parametrize("n,most", [(200, 2.65e-14), (255, 3.15e-14)])
+def test_back_transformation_orthogonality(n, most):
+    import torch
+    _, _, x = _solve(n, 150, "TRIDIAG_DC")
+    eye = torch.eye(n, device="cuda")
+    assert torch.linalg.norm(x.mH @ x - eye, dim=(1, 2)).mean().item() <= most
