@@ -134,18 +134,17 @@ __device__ __forceinline__ void hetrd_tile(const S& st, int m, int r0, int c0, c
         es[j] = cz<C>();
         C vc, wc;
         if (UPD) {
-            vc = v[c];
-            wc = w[c];
-            vc.x = -vc.x;   // -conj
-            wc.x = -wc.x;
+            vc = cconj(v[c]);
+            wc = cconj(w[c]);
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int r = r0 + lr + 8 * i;
             const bool in = INSIDE || (c < m && r <= c);
             if (UPD) {
-                cfma(x[i], vr[i], wc);
-                cfma(x[i], wr[i], vc);
+                C u = cmul(vr[i], wc);   // (summed apart: onto x, every term would round at x's size)
+                cfma(u, wr[i], vc);
+                x[i] = csub(x[i], u);
                 if (!INSIDE && r == c) x[i].y = 0;
                 if (in) *st.at(r, c) = x[i];
                 else x[i] = cz<C>();

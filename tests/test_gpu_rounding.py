@@ -29,3 +29,13 @@ def test_back_transformation_orthogonality(n, most):
     _, _, x = _solve(n, 150, "TRIDIAG_DC")
     eye = torch.eye(n, device="cuda")
     assert torch.linalg.norm(x.mH @ x - eye, dim=(1, 2)).mean().item() <= most
+
+
+# ||H X - X W|| / ||H|| with bisection: 1.04e-15, 1.15e-15 and 1.23e-15 where the rank-2 update is summed
+# before it is taken off the matrix, and 8 %.  Accumulated onto the matrix: 1.19e-15 to 1.50e-15.
+@pytest.mark.parametrize("n,most", [(129, 1.12e-15), (200, 1.24e-15), (255, 1.33e-15)])
+def test_reduction_residual(n, most):
+    import torch
+    h, w, x = _solve(n, 150, "TRIDIAG_BISECTION")
+    res = torch.linalg.norm(h @ x - x * w[:, None, :], dim=(1, 2)) / torch.linalg.norm(h, dim=(1, 2))
+    assert res.mean().item() <= most
