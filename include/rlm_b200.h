@@ -116,8 +116,8 @@ int rlmb_heev_solver(rlmb_context* ctx, int n, int precision, int* solver);
  * FP64 tensor-core GEMMs).  RLMB_TRIDIAG_AUTO: the built-in choice (divide and conquer from
  * n = 600) or the autotuned one.  Both run in
  * double precision in either precision mode. */
-/* Panel queue of the blocked reduction (orders above 512, chunks of more matrices than SMs; no
- * counterpart in the reference): CTAs of `threads` = 512 threads, one per SM, or 256 threads,
+/* Panel queue of the blocked reduction (orders above 512, chunks of more matrices than SMs, and the
+ * first panels of orders above 3000 where no cluster of CTAs fits; no counterpart in the reference): CTAs of `threads` = 512 threads, one per SM, or 256 threads,
  * two per SM, take (matrix, column) units; 0 = the built-in choice. */
 int rlmb_set_panel_queue(rlmb_context* ctx, int n, int precision, int threads);
 /* Columns per panel of the blocked reduction: 16 or 32 (rank-32 or rank-64 updates); 0 = the

@@ -24,11 +24,11 @@
 //   mixed mode     the reduction and back-transformation in single precision, then double
 //                  refinement of every eigenpair (k_ref_*, Ogita-Aishima restated, with
 //                  cluster Rayleigh-Ritz).
-//   small orders   up to order 20 (autotuned up to 80) the whole eigensolve is batched
-//                  two-sided Jacobi instead (jacobi.cuh).
+//   small orders   up to order 20 (12 in the mesh solves, autotuned up to 80) the whole eigensolve
+//                  is batched two-sided Jacobi instead (jacobi.cuh).
 //
 // Waits are __syncthreads inside one CTA and the hardware barriers of a cluster
-// (k_hetrd_panel_c), except the panel queue's per-column counts (k_hetrd_panel_q), whose spins
+// (k_hetrd_panel_c, k_dc_merge), except the panel queue's per-column counts (k_hetrd_panel_q), whose spins
 // are bounded in time and abort the chunk when they run out.
 #include "common.cuh"
 #include "jacobi.cuh"
@@ -258,8 +258,8 @@ __device__ __forceinline__ void reflector(const C alpha, R xnorm2, R& beta, C& t
 // tile, so that it needs neither atomics nor a cleared accumulator.
 // Bound: instruction issue (several CTAs per SM hide the chains of the reflector).  With one
 // row and 16 columns per lane, shared double atomics and eight barriers per column 4,624 matrices
-// of order 64 took 4.03 ms, 2,304 of order 32 0.69 ms and 128 of order 129 0.93 ms; now 1.80,
-// 0.17 and 0.44.
+// of order 64 took 4.03 ms, 2,304 of order 32 0.69 ms and 128 of order 129 0.93 ms; now 1.85,
+// 0.17 and 0.46.
 static constexpr int HT_PARTS_MAX = 144;
 // vectors are read up to the next multiple of 16, times zero; with sums by atomics, where shared memory
 // sets the largest order, that may be the next array
@@ -1963,7 +1963,8 @@ __host__ __device__ constexpr size_t panel_smem(int m) {
     return (2 * (size_t)m + 2 * HP_W_MAX) * sizeof(typename Cx<R>::T) + 2 * (NT / 32) * sizeof(R);
 }
 
-// The panel for chunks of more matrices than SMs (see panel_waves_full): one resident CTA of NT
+// The panel for chunks of more matrices than SMs (see panel_waves_full; and for vectors too long for
+// k_hetrd_panel_c's rings, see tridiagonalise): one resident CTA of NT
 // threads per SM (grid <= SMs) takes units (matrix, column) from a queue, unit u = claim - base = matrix
 // u % nb, column u / nb, so that every SM keeps NT threads of loads in flight whatever the
 // number of matrices (one CTA per matrix would leave SMs with a single CTA when the chunk has
@@ -2259,10 +2260,10 @@ __host__ __device__ constexpr size_t panel_c_smem(int m, int P) {
 //   -- barrier --   sums of the CTAs' parts over distributed shared memory
 // x^H v for w = x - tau/2 (x^H v) v comes from v^H A v and the pairs' products, so that it
 // needs no barrier of its own.
-// Bound: the stream of the leading block (25 matrices of order 2500, clusters of 5: 215 ms for
-// 1.04 TB, 4.8 TB/s), with the instructions of the product close behind (137 of the 215 ms remain
-// with the loads taken out).  One CTA per matrix, 25 SMs at work, took 923 ms, and 957 at order
-// 3000 in single precision, now 211.
+// Bound: the stream of the leading block (25 matrices of order 2500, clusters of 5: 198 to 204 ms
+// for 1.04 TB, 5.2 TB/s), with the instructions of the product close behind (two thirds of the time
+// remained with the loads taken out).  One CTA per matrix, 25 SMs at work, took 923 ms, and 957 at
+// order 3000 in single precision, now 208.
 // ONE: one CTA per matrix, no cluster.
 template <int NT, class R, bool ONE>
 __global__ void __launch_bounds__(NT, NT > 256 ? 1 : 512 / NT)
@@ -2521,7 +2522,7 @@ static cudaError_t launch_panel_c(cudaStream_t st, typename Cx<R>::T* A, double*
 // if that is at least 1.5 (below order 512: 2) times the 512 threads of one CTA per matrix:
 // panels of order 300, double precision, 18 matrices 3.46 -> 2.63 ms, 36 3.47 -> 2.86, but 81
 // 3.49 -> 3.71; of order 512 10.9 -> 5.9, 11.3 -> 6.9, 13.1 -> 10.9; of order 2500, 25 matrices,
-// 923 -> 215.
+// 923 -> 198.
 struct PanelShape {
     int nt, P;
 };
@@ -3887,8 +3888,8 @@ using namespace rlmb;
 
 // ----------------------------------------------------------------------- autotuner
 // Per context, per (order, precision): the launch choices of HeevTune picked by timing every
-// feasible candidate -- unblocked or blocked reduction (from order 128), 256- or 512-thread
-// panels, register-resident or GEMM back-transformation, 64- or 128-reflector blocks and 64- or
+// feasible candidate -- unblocked or blocked reduction (from order 128), panels by the built-in
+// rules or of 512 threads, SM-resident or GEMM back-transformation, 64- or 128-reflector blocks and 64- or
 // 128-row X-update tiles (double precision) of the latter, either tridiagonal solver (bisection +
 // inverse iteration, or divide and conquer), and up to order JAC_MAX_N the batched Jacobi solver -- on copies of up to 2 x SMs of the call's own matrices (at most 2 GB of them),
 // each candidate run twice and timed the second time with CUDA events.  Orders
